@@ -51,6 +51,11 @@ cudaError_t launchMeshSdf32(const MeshQueryArgs& a, int warpsPerBlock, int numSm
 // FP64 re-evaluation of the band list (reads band_count on the device).
 cudaError_t launchMeshBand64(const MeshQueryArgs& a, float delta, int numSms, cudaStream_t s);
 
+// The whole query (FP64 results when a.out_d64 is set, else FP32 with the FP64 band pass if band64) with
+// one warp per point, for calls of few points; reads a.mesh, points / points64, n, band, eval and the
+// outputs, and needs no ordering or workspace.
+cudaError_t launchMeshPoint(const MeshQueryArgs& a, float delta, bool band64, int numSms, cudaStream_t s);
+
 // FlatMeshSDF over every triangle (FP64 points and results, DCEL face algorithm); outTri nullable;
 // non-finite points set ST_INPUT in *status and get NaN.
 cudaError_t launchMeshFlat64(const EbgMeshView& m, int64_t numTris, const double* pts, int64_t n, double* out,

@@ -1,0 +1,193 @@
+// Mesh signed distance of few points (sm_100a): one warp per query (mesh_point.cuh).  Compiled with
+// -fmad=false like the other FP64 passes (band64.cuh).
+//
+// One launch does what the packet path needs an ordering, a traversal, a compaction and a band pass
+// for, and takes no workspace.
+#include <cfloat>
+
+#include <math_constants.h>
+
+#include "band64.cuh"
+#include "mesh_kernels.h"
+#include "mesh_point.cuh"
+
+namespace ebg {
+
+namespace {
+
+constexpr int POINT_WARPS = 4;
+
+// The triangle of smallest |d| in FP64 within `bound` of the FP32 point (px, py, pz), which lies
+// `shift` from P (see band64Mesh); its FP32 distance selects the triangles worth an FP64 test.
+template <int EVAL, bool UPPER>
+__device__ int pointSearch64(const EbgMeshView& m, D3 P, float px, float py, float pz, float shift, float delta,
+                             float bound, double& best, int& bt, PointMem& w)
+{
+  const float inf   = __int_as_float(0x7f800000);
+  const float slack = delta + 2.f * shift;
+  best              = DBL_MAX;
+  bt                = -1;
+  return pointSearch<UPPER>(m, px, py, pz, bound, slack, w, [&](bool active, uint32_t tri) {
+    float dd = inf, low = inf;
+    if (active) {
+      const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
+      const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+      float         s, t;
+      int           r;
+      dd  = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
+      low = triLower(h0, h1, h2, px, py, pz, s, t, dd);
+    }
+    const float near = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(dd)));
+    const float rn   = (sqrtf(near) * 1.00001f + slack) * 1.000001f;
+    bound            = fminf(bound, rn * rn);
+    // (not "low <= ...": a point on the triangle has no direction and a NaN bound)
+    const bool cand = active && !(low > sqrtf(bound) * 1.00001f + delta);
+    if (!__any_sync(FULL, cand)) {
+      return;
+    }
+    double d = DBL_MAX;
+    if (cand) {
+      d = EVAL == 0 ? triSd64(m.tri64 + 30 * size_t(tri), P)
+                    : dcelFaceSd(m.tri64 + 30 * size_t(tri), m.dcel_n + 3 * size_t(tri), P);
+    }
+    // the warp's least (|d|, triangle): non-negative doubles order like their words
+    const uint32_t hi = cand ? uint32_t(__double2hiint(fabs(d))) : 0xffffffffu;
+    const uint32_t mh = __reduce_min_sync(FULL, hi);
+    const uint32_t lo = hi == mh ? uint32_t(__double2loint(d)) : 0xffffffffu;
+    const uint32_t ml = __reduce_min_sync(FULL, lo);
+    const uint32_t ti = cand && hi == mh && lo == ml ? tri : 0xffffffffu;
+    const uint32_t mt = __reduce_min_sync(FULL, ti);
+    const unsigned who = __ballot_sync(FULL, ti == mt && cand);
+    if (mt == 0xffffffffu || who == 0u) {
+      return; // only NaN values
+    }
+    const double dm = __shfl_sync(FULL, d, __ffs(int(who)) - 1);
+    if (fabs(dm) < fabs(best) || (fabs(dm) == fabs(best) && int(mt) < bt)) {
+      best           = dm;
+      bt             = int(mt);
+      const float rb = (float(fabs(dm)) + shift) * 1.000001f + 1e-30f;
+      bound          = fminf(bound, rb * rb);
+    }
+  });
+}
+
+// F64: FP64 points and results with evaluator EVAL (0 the Triangle test, 1 the DCEL face).  Else
+// FP32 points and results: the FP32 search, and the FP64 one where |d| is within the band.
+// Bound by the latency of its dependent loads (two per tree level and two per leaf batch), so the
+// FP32 form keeps 32 queries in flight per SM at the cost of a few spills in its rare FP64 part.
+// B200, 20,480 triangles, uniform points, packet path before -> now: 1 point 166 -> 15 us, 32 points
+// 1,281 -> 15 us, 1,000 points 616 -> 27 us, 65,536 points 1.41 -> 0.21 ms; in FP64 1,000 points
+// 1,695 -> 19 us, 65,536 points 3.62 -> 0.27 ms.
+template <bool F64, int EVAL>
+__global__ void __launch_bounds__(32 * POINT_WARPS, F64 ? 5 : 8) kMeshPoint(const MeshQueryArgs a, float delta, int band64)
+{
+  __shared__ PointMem mem[POINT_WARPS];
+  const EbgMeshView&  m    = a.mesh;
+  PointMem&           w    = mem[threadIdx.x >> 5];
+  const int           lane = threadIdx.x & 31;
+  const int64_t       nW   = int64_t(gridDim.x) * POINT_WARPS;
+  const float         inf  = __int_as_float(0x7f800000);
+  for (int64_t id = int64_t(blockIdx.x) * POINT_WARPS + (threadIdx.x >> 5); id < a.n; id += nW) {
+    D3    P;
+    float px, py, pz;
+    if (F64) {
+      P  = {a.points64[3 * id], a.points64[3 * id + 1], a.points64[3 * id + 2]};
+      px = float(P.x), py = float(P.y), pz = float(P.z);
+    }
+    else {
+      px = __ldg(a.points + 3 * id), py = __ldg(a.points + 3 * id + 1), pz = __ldg(a.points + 3 * id + 2);
+      P  = {double(px), double(py), double(pz)};
+    }
+    if (!(isfinite(px) && isfinite(py) && isfinite(pz))) {
+      if (lane == 0) {
+        atomicOr(a.status, ST_INPUT);
+        if (F64) {
+          a.out_d64[id] = double(FLT_MAX);
+        }
+        else {
+          a.out_d[id] = FLT_MAX;
+        }
+        if (a.out_tri) {
+          a.out_tri[id] = -1;
+        }
+      }
+      continue;
+    }
+    const double ex = P.x - double(px), ey = P.y - double(py), ez = P.z - double(pz);
+    const float  shift = F64 ? float(sqrt(ex * ex + ey * ey + ez * ez)) * 1.0001f : 0.f;
+    double       best = DBL_MAX;
+    int          bt   = -1, err;
+    if (F64) {
+      err = pointSearch64<EVAL, true>(m, P, px, py, pz, shift, delta, FLT_MAX, best, bt, w);
+      if (lane == 0) {
+        a.out_d64[id] = bt >= 0 ? best : double(FLT_MAX);
+        if (a.out_tri) {
+          a.out_tri[id] = bt >= 0 ? __ldg(m.tri_id + bt) : -1;
+        }
+      }
+    }
+    else {
+      float bound = FLT_MAX, bd2 = inf;
+      err = pointSearch<true>(m, px, py, pz, bound, delta, w, [&](bool active, uint32_t tri) {
+        float dd = inf;
+        if (active) {
+          const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
+          const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+          float         s, t;
+          int           r;
+          dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
+        }
+        // ties go to the lower leaf position, as in the packet traversal
+        const uint32_t mb = __reduce_min_sync(FULL, __float_as_uint(dd));
+        const uint32_t mt = __reduce_min_sync(FULL, __float_as_uint(dd) == mb ? tri : 0x7fffffffu);
+        const float    md = __uint_as_float(mb);
+        if (md < bd2 || (md == bd2 && int(mt) < bt)) {
+          bd2   = md;
+          bt    = int(mt);
+          bound = fminf(bound, bd2);
+        }
+      });
+      float dist = bt >= 0 ? signedFromWinner(m, uint32_t(bt), px, py, pz) : FLT_MAX;
+      int   tri  = bt;
+      if (band64 && bt >= 0 && fabsf(dist) <= a.band) {
+        const float r = (fabsf(dist) * 1.00001f + delta) * 1.000001f;
+        int         b64;
+        err |= pointSearch64<0, false>(m, P, px, py, pz, 0.f, delta, r * r, best, b64, w);
+        if (b64 >= 0) {
+          dist = float(best);
+          tri  = b64;
+        }
+      }
+      if (lane == 0) {
+        a.out_d[id] = dist;
+        if (a.out_tri) {
+          a.out_tri[id] = tri >= 0 ? __ldg(m.tri_id + tri) : -1;
+        }
+      }
+    }
+    if (err && lane == 0) {
+      atomicOr(a.status, err);
+    }
+  }
+}
+
+} // namespace
+
+cudaError_t launchMeshPoint(const MeshQueryArgs& a, float delta, bool band64, int numSms, cudaStream_t s)
+{
+  const int64_t need = (a.n + POINT_WARPS - 1) / POINT_WARPS;
+  const int64_t most = int64_t(numSms) * 32;
+  const unsigned grid = unsigned(need < most ? need : most);
+  if (a.out_d64 == nullptr) {
+    kMeshPoint<false, 0><<<grid, 32 * POINT_WARPS, 0, s>>>(a, delta, band64 ? 1 : 0);
+  }
+  else if (a.eval == 1) {
+    kMeshPoint<true, 1><<<grid, 32 * POINT_WARPS, 0, s>>>(a, delta, 1);
+  }
+  else {
+    kMeshPoint<true, 0><<<grid, 32 * POINT_WARPS, 0, s>>>(a, delta, 1);
+  }
+  return cudaGetLastError();
+}
+
+} // namespace ebg
