@@ -21,6 +21,7 @@ struct ebg_mesh
   ebg_mesh_info info{};
   // device allocations
   void* dNodes  = nullptr;
+  void* dChildren = nullptr; // the nodes' slots, see EbgChild
   void* dHot    = nullptr;
   void* dSign   = nullptr;
   void* dTri64  = nullptr;

@@ -207,7 +207,9 @@ void setMeshBounds(ebg_mesh* m, const double* lo, const double* hi)
 ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const double* lo, const double* hi,
                       ebg_mesh** out)
 {
-  if (cudaMalloc(reinterpret_cast<void**>(&m->dStatus), sizeof(int)) != cudaSuccess ||
+  const size_t slots = 4 * size_t(std::max<int64_t>(m->info.num_nodes, 1));
+  if (cudaMalloc(&m->dChildren, slots * sizeof(EbgChild)) != cudaSuccess ||
+      cudaMalloc(reinterpret_cast<void**>(&m->dStatus), sizeof(int)) != cudaSuccess ||
       cudaMemset(m->dStatus, 0, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     ebg_mesh_destroy(m);
@@ -215,6 +217,7 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
   }
   EbgMeshView& v = m->view;
   v.nodes        = static_cast<const EbgNode4*>(m->dNodes);
+  v.children     = static_cast<const EbgChild*>(m->dChildren);
   v.hot          = static_cast<const EbgTriHot*>(m->dHot);
   v.sign         = static_cast<const EbgTriSign*>(m->dSign);
   v.tri64        = static_cast<const double*>(m->dTri64);
@@ -228,10 +231,16 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
   inf.num_vertices   = nv;
   inf.leaf_size      = leafSize;
   const size_t N     = size_t(nt);
-  inf.device_bytes = int64_t(size_t(std::max<int64_t>(inf.num_nodes, 1)) * (sizeof(EbgNode4) + sizeof(EbgObb) + 8) +
+  inf.device_bytes = int64_t(size_t(std::max<int64_t>(inf.num_nodes, 1)) * (2 * sizeof(EbgNode4) + sizeof(EbgObb) + 8) +
                              size_t(inf.num_leaves) * (sizeof(EbgObb) + 8) +
                              N * (sizeof(EbgTriHot) + sizeof(EbgTriSign) + 33 * sizeof(double) + 4 + 12));
-  *out             = m;
+  launchNodeChildren(v.nodes, inf.num_nodes, static_cast<EbgChild*>(m->dChildren), nullptr);
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    const std::string e = cudaGetErrorString(cudaGetLastError());
+    ebg_mesh_destroy(m);
+    return setError(EBG_ERR_CUDA, "mesh set-up: " + e);
+  }
+  *out = m;
   return EBG_OK;
 }
 
@@ -499,6 +508,19 @@ bool pointPath(int64_t n, const ebg_query_opts* opts, const unsigned long long* 
          !(opts && (opts->timings || opts->top_nodes > 0 || opts->node_width > 0));
 }
 
+// The FP32 pass by packet boxes (mesh_packet.cu) or by the packet walk (mesh_sdf.cu).  The walk keeps
+//  - what only it has: counters, radius hints, the shared-memory top of the tree, the 8-wide copy;
+//  - meshes of fewer than 4,096 triangles, whose walk is short (4 M points on 1,280 triangles: 0.37
+//    against 0.48 ms near the surface, 0.92 against 0.94 ms everywhere; on 5,120 triangles 1.9 against
+//    1.8 ms everywhere);
+//  - FP32 calls that ask for the closest triangles: of triangles at exactly the same distance the walk
+//    names the one that its order and box rounding leave (2 points of 8 M differed).
+bool packetPath(const ebg_mesh* m, const MeshQueryArgs& a, int width, bool fp32Triangles)
+{
+  return a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && width == 4 && !fp32Triangles &&
+         m->info.num_triangles >= 4096;
+}
+
 } // namespace
 
 ebg_status ebg::meshQuery(const ebg_mesh*       m,
@@ -585,6 +607,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
 
   Workspace ws(s);
   uint32_t* order = nullptr;
+  uint32_t* pointList = nullptr; // points that the packet search puts aside
   if (sort) {
     uint32_t* keysIn  = ws.get<uint32_t>(n);
     uint32_t* keysOut = ws.get<uint32_t>(n);
@@ -604,11 +627,15 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
         cudaSuccess) {
       return setError(EBG_ERR_CUDA, "query sort failed");
     }
+    pointList = idsIn; // free again after the sort
   }
   // The band list: the traversal flags each sorted position, and a compaction of the flags gives
   // the list in position (Morton) order, so that each FP64 packet holds 32 neighbouring queries.
   // (Appending from the traversal lists them in completion order, which interleaves thousands of
   // packets in flight.)
+  if (pointList == nullptr) {
+    pointList = ws.get<uint32_t>(n);
+  }
   unsigned long long* counters = ws.get<unsigned long long>(2); // [0] packets, [1] band count (u32)
   uint32_t*           bandList = band64 ? ws.get<uint32_t>(n) : nullptr;
   uint8_t*            bandFlag = band64 ? ws.get<uint8_t>(n) : nullptr;
@@ -643,6 +670,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   a.band_list  = bandList;
   a.band_count = reinterpret_cast<uint32_t*>(counters + 1);
   a.band_d32   = nullptr;
+  a.point_list = pointList;
   a.band_flag  = bandFlag;
   a.work       = counters;
   a.status     = m->dStatus;
@@ -658,7 +686,16 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     a.node_width = 8;
     a.top_nodes  = 0;
   }
-  if (launchMeshSdf32(a, wpb, m->numSms, s, occ) != cudaSuccess) {
+  const float delta = float(2e-6 * fp32ErrorScale(m)) + 1e-30f;
+  if (packetPath(m, a, width, outTri != nullptr && !fp64all)) {
+    // packets up to three mean leaf sizes wide share one box (the extent of a leaf on a surface of
+    // about the diagonal's square): 6 measured the same on dense points, 2-5 % slower on sparse ones
+    const float leafSize = float(m->info.diagonal / std::sqrt(double(std::max<int64_t>(1, m->info.num_leaves))));
+    if (launchMeshPacket32(a, delta, 3.f * leafSize, m->info.num_leaves, m->numSms, s) != cudaSuccess) {
+      return setError(EBG_ERR_CUDA, std::string("traversal launch failed: ") + cudaGetErrorString(cudaGetLastError()));
+    }
+  }
+  else if (launchMeshSdf32(a, wpb, m->numSms, s, occ) != cudaSuccess) {
     return setError(EBG_ERR_CUDA, std::string("traversal launch failed: ") + cudaGetErrorString(cudaGetLastError()));
   }
   a.mesh       = m->view;
@@ -673,7 +710,6 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     }
     // delta bounds the FP32 distance error: 2e-6 of the mesh's diagonal, or of its coordinates'
     // magnitude for a mesh far from the origin (about 17 FP32 roundings of either)
-    const float delta = float(2e-6 * fp32ErrorScale(m)) + 1e-30f;
     if (launchMeshBand64(a, delta, m->numSms, s) != cudaSuccess) {
       return setError(EBG_ERR_CUDA, "band launch failed");
     }
@@ -771,6 +807,7 @@ ebg_status ebg_mesh_destroy(ebg_mesh* m)
   DeviceGuard guard;
   cudaSetDevice(m->device);
   cudaFree(m->dNodes);
+  cudaFree(m->dChildren);
   cudaFree(m->dHot);
   cudaFree(m->dSign);
   cudaFree(m->dTri64);

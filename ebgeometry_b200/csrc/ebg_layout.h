@@ -55,6 +55,17 @@ struct alignas(128) EbgNode4
   uint32_t count[4];
 };
 
+// One child slot of a node with its words together: the searches that put another child on every
+// lane (mesh_point.cuh, mesh_packet.cu) read a slot as two 16-byte words from the copy `children`,
+// 4 per node in node order, where the structure-of-arrays node costs them eight 4-byte loads.
+struct alignas(32) EbgChild
+{
+  float    lox, loy, loz;
+  uint32_t child;
+  float    hix, hiy, hiz;
+  uint32_t count;
+};
+
 // The optional 8-wide copy of the tree (plain FP32 queries only; mesh_wide.cpp): two 128-byte
 // lines per node, the boxes of eight children as structure-of-arrays (lo.x[8] ... hi.z[8]), then
 // child[8] and count[8] with the 4-wide node's meanings.  Leaves and child boxes are the 4-wide
@@ -97,6 +108,7 @@ struct alignas(16) EbgObb
 };
 
 static_assert(sizeof(EbgNode4) == 128, "node must be one 128-byte line");
+static_assert(sizeof(EbgChild) == 32, "child slot must be two 16-byte words");
 static_assert(sizeof(EbgNode8) == 256, "8-wide node must be two 128-byte lines");
 static_assert(sizeof(EbgObb) == 64, "oriented box must be 64 bytes");
 static_assert(sizeof(EbgTriHot) == 48, "hot triangle record must be 48 bytes");
@@ -106,6 +118,7 @@ static_assert(sizeof(EbgTriSign) == 96, "sign record must be 96 bytes");
 struct EbgMeshView
 {
   const EbgNode4*   nodes;
+  const EbgChild*   children;               // the nodes' slots, 4 per node (the same boxes and words)
   const EbgTriHot*  hot;
   const EbgTriSign* sign;
   const double*     tri64;

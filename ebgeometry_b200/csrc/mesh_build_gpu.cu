@@ -36,6 +36,7 @@
 #include "ebg_device.cuh"
 #include "mesh_build_gpu.h"
 #include "mesh_host.h"
+#include "mesh_kernels.h"
 
 namespace ebg {
 
@@ -1968,6 +1969,7 @@ ebg_status refitMeshOnDevice(ebg_mesh* m, const double* V, bool vOnDevice, int64
   if (numNodes > 0) {
     kSlotBoxes<<<gridFor(4 * int64_t(numNodes), 256), 256, 0, s>>>(leafAabb, nodeAabb, useful, numNodes, numLeaves,
                                                                    static_cast<EbgNode4*>(m->dNodes));
+    launchNodeChildren(m->view.nodes, numNodes, static_cast<EbgChild*>(m->dChildren), s);
   }
   std::vector<double> cdf(N);
   cudaMemcpyAsync(cdf.data(), area, 8 * N, cudaMemcpyDeviceToHost, s);

@@ -26,6 +26,8 @@ struct MeshQueryArgs
   float              band;       // |d| <= band -> FP64 re-evaluation list
   uint32_t*          band_list;  // sorted positions needing FP64 (nullable = no band pass)
   uint32_t*          band_count;
+  uint32_t*          point_list; // sorted positions that the packet search leaves to one warp each; their
+                                 // number is counted in band_count[1] (zeroed before the launch)
   float*             band_d32;   // FP32 distance of each band entry (nullable: read out_d instead)
   uint8_t*           band_flag;  // per sorted position, 1 = needs FP64 (nullable: the traversal
                                  // appends to band_list itself, in completion order)
@@ -45,8 +47,15 @@ struct MeshQueryArgs
 void launchQueryKeys(const float* points, int64_t n, const float* lo, const float* scale, uint32_t* keys,
                      uint32_t* ids, cudaStream_t s);
 
+// children[4 i + k] = slot k of nodes[i].
+void launchNodeChildren(const EbgNode4* nodes, int64_t numNodes, EbgChild* children, cudaStream_t s);
+
 // FP32 packet traversal.  warpsPerBlock in {1,2,4,8}; occupancy 0..3 (see ebg_query_opts).
 cudaError_t launchMeshSdf32(const MeshQueryArgs& a, int warpsPerBlock, int numSms, cudaStream_t s, int occupancy = 0);
+
+// The FP32 search by packet boxes (plain, or with an attached model's cells; no counters, hints, top nodes
+// or 8-wide copy); delta as for launchMeshBand64; packets with a half-extent above split are divided.
+cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, int64_t numLeaves, int numSms, cudaStream_t s);
 
 // FP64 re-evaluation of the band list (reads band_count on the device).
 cudaError_t launchMeshBand64(const MeshQueryArgs& a, float delta, int numSms, cudaStream_t s);

@@ -1,0 +1,749 @@
+// FP32 mesh signed distance of many points (sm_100a): packets of 32 neighbouring queries whose tree
+// search runs once per packet, on the packet's box, with the 32 lanes on 32 different children.
+//
+// A packet's depth-first walk (mesh_sdf.cu) tests every node, oriented box and leaf with all 32
+// points, one after another: about 37,000 warp instructions per packet of the 512^3 grid on 1.3 M
+// triangles, most of them for entries that no lane turns out to need.  Here a lane decides for one
+// entry whether ANY point of the packet can need it:
+//   - `a` is a point of the mesh near the packet, so a query p is at most |p - a| from the mesh;
+//   - e is the entry's point nearest to the packet's centre c, u the unit vector from e to c; the
+//     entry (convex) lies behind the plane through e with normal u, so it is at least u . (p - e)
+//     from p;
+//   - |p - a| - u . (p - e) is convex in p, so over the packet's box it is largest at a corner: where it
+//     is negative at all eight corners, no query of the packet needs the entry.
+// Unlike a bound from two radii, this keeps what lies beside the packet's own patch only as far as
+// the directions to it and to `a` differ.  What is left is a list of leaves, which all lanes test
+// with their own bounds as the walk does (packetLeaf).
+//
+// Packets come off the work counter in groups of up to eight neighbours.  A group's box is taken
+// down the tree once, as far as at most 32 entries reach; its packets start there.  The winners of one
+// packet give the next its `a` and its lanes' first bounds (a query that passes an attached model takes
+// both from the anchors of its cells instead).
+//
+// The list is tested in three steps.  The two leaves nearest to c go through all lanes, which brings
+// the bounds near their final values; then a lane per leaf tests its oriented box against the 32
+// points and bounds, which gives the (lane, leaf) pairs that are left; 32 pairs at a time, a lane per
+// pair, test their triangles, and the results meet in a 64-bit minimum of (d2, triangle) per query.
+//
+// A packet too wide for one box is divided at its widest step.  What stays too wide, holds too few
+// points or reaches too many leaves (points few against the tree's leaves, or near the medial axis) is
+// put on a list, and kMeshListed searches those points eight lanes each.
+//
+// Bound by the L1's data stage (89 % of its wavefronts) and by instruction issue (69 %): per packet of
+// the 512^3 grid 10 rounds of 32 children, 104 listed leaves, 27 of them with a pair, 7 passes over
+// pairs, about 19,000 warp instructions.  B200, 151 M points on 1.3 M triangles, the walk -> here:
+// traversal 172.6 -> 79.5 ms, with a model 92.3 -> 71.2 ms; 1 M uniform points on 20,480 triangles
+// 1.42 -> 0.75 ms; 262,144 on 81,920 triangles 2.11 -> 0.65 ms.
+#include <cfloat>
+
+#include "ebg_device.cuh"
+#include "mesh_kernels.h"
+#include "mesh_point.cuh"
+#include "mesh_traverse.cuh"
+
+namespace ebg {
+
+namespace {
+
+constexpr int PACKET_WARPS = 4;
+constexpr int PACKET_PAIRS = 256; // (lane, leaf) pairs waiting for their triangle tests
+
+__device__ __forceinline__ float warpMin(float x)
+{
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float warpMax(float x)
+{
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The nearest triangle of one point (all lanes on the same point), or with FIRST a near one.
+template <bool FIRST>
+__device__ __noinline__ int pointNearest32(const EbgMeshView& m, float px, float py, float pz, float delta, PointMem& w,
+                                           float& bd2, int& bt)
+{
+  const float inf   = __int_as_float(0x7f800000);
+  float       bound = FLT_MAX, b = inf;
+  int         t = -1;
+  const int   err = pointSearch<true, FIRST>(m, px, py, pz, bound, delta, w, [&](bool active, uint32_t tri) {
+    float dd = inf;
+    if (active) {
+      const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
+      const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+      float         s_, t_;
+      int           r_;
+      dd = triDist2<false>(h0, h1, h2, px, py, pz, s_, t_, r_);
+    }
+    const uint32_t mb = __reduce_min_sync(FULL, __float_as_uint(dd));
+    const uint32_t mt = __reduce_min_sync(FULL, __float_as_uint(dd) == mb ? tri : 0x7fffffffu);
+    const float    md = __uint_as_float(mb);
+    if (md < b || (md == b && int(mt) < t)) {
+      b     = md;
+      t     = int(mt);
+      bound = fminf(bound, b);
+    }
+  });
+  bd2 = b;
+  bt  = t;
+  return err;
+}
+
+// The point of the triangle with weights s, t, moved into the triangle where rounding left it outside.
+__device__ __forceinline__ void triPoint(const float4 h0, const float4 h1, const float4 h2, float s, float t, float& x,
+                                         float& y, float& z)
+{
+  s             = fmaxf(s, 0.f);
+  t             = fmaxf(t, 0.f);
+  const float k = __fdividef(1.f, fmaxf(1.f, s + t));
+  s *= k;
+  t *= k;
+  x = h0.x + fmaf(s, h1.x, t * h2.x);
+  y = h0.y + fmaf(s, h1.y, t * h2.y);
+  z = h0.z + fmaf(s, h1.z, t * h2.z);
+}
+
+// Whether some corner of the packet's box (half-extents hx, hy, hz about c) reaches the entry whose
+// nearest point to c lies at c - (wx, wy, wz); A0, A1 the corners' bounds, signs (+++, ---, ++-, --+) and
+// (+-+, -+-, +--, -++).  An entry that contains c (no direction, NaN) is kept.
+__device__ __forceinline__ bool cornersReach(const float4 A0, const float4 A1, float hx, float hy, float hz, float wx,
+                                             float wy, float wz, float& d2)
+{
+  d2              = fmaf(wx, wx, fmaf(wy, wy, wz * wz));
+  const float inv = rsqrtf(d2), d = d2 * inv;
+  const float tx = wx * hx * inv, ty = wy * hy * inv, tz = wz * hz * inv;
+  const float p = tx + ty, q = tx - ty;
+  const float k0 = p + tz, k1 = p - tz, k2 = q + tz, k3 = q - tz;
+  const float m0 = fmaxf(fmaxf(A0.x - k0, A0.y + k0), fmaxf(A0.z - k1, A0.w + k1));
+  const float m1 = fmaxf(fmaxf(A1.x - k2, A1.y + k2), fmaxf(A1.z - k3, A1.w + k3));
+  return !(fmaxf(m0, m1) < d);
+}
+
+__device__ __forceinline__ bool cornersReachObb(const float4 A0, const float4 A1, float hx, float hy, float hz,
+                                                const float4* __restrict__ ob, float cx, float cy, float cz, float& d2)
+{
+  const float4 o0 = __ldg(ob), o1 = __ldg(ob + 1), o2 = __ldg(ob + 2), o3 = __ldg(ob + 3);
+  const float  a = fmaf(o0.x, cx, fmaf(o0.y, cy, fmaf(o0.z, cz, -o0.w)));
+  const float  b = fmaf(o1.x, cx, fmaf(o1.y, cy, fmaf(o1.z, cz, -o1.w)));
+  const float  e = fmaf(o2.x, cx, fmaf(o2.y, cy, fmaf(o2.z, cz, -o2.w)));
+  const float  wa = copysignf(fmaxf(fabsf(a) - o3.x, 0.f), a);
+  const float  wb = copysignf(fmaxf(fabsf(b) - o3.y, 0.f), b);
+  const float  we = copysignf(fmaxf(fabsf(e) - o3.z, 0.f), e);
+  return cornersReach(A0, A1, hx, hy, hz, fmaf(wa, o0.x, fmaf(wb, o1.x, we * o2.x)),
+                      fmaf(wa, o0.y, fmaf(wb, o1.y, we * o2.y)), fmaf(wa, o0.z, fmaf(wb, o1.z, we * o2.z)), d2);
+}
+
+constexpr int PACKET_FRONT = 32; // entries of a group's frontier
+
+struct PacketMem
+{
+  float4             query[32]; // the lanes' points and bounds
+  unsigned long long key[32];   // the lanes' best (d2, triangle)
+  float4             corner[2]; // the corners' bounds
+  float4             last;      // centre and half-extent of the box before
+  uint32_t           front[PACKET_FRONT], frontCount[PACKET_FRONT]; // child and count words
+  uint32_t           pairTri[PACKET_PAIRS];                         // (lane, leaf) pairs: first triangle,
+  uint16_t           pairLane[PACKET_PAIRS];                        // triangle count and lane
+  PointMem           w;
+};
+
+// The packet's (or group's) box and the mesh point that bounds its distances.
+struct Reach
+{
+  float cx, cy, cz, hx, hy, hz;
+};
+
+// The corners' bounds |corner - a| by the lanes 0..7 in cornersReach's order (bit i of each mask: the
+// sign of corner i on that axis, 1 = plus).
+__device__ __forceinline__ void setCorners(PacketMem& pm, const Reach& r, float ax, float ay, float az, float delta)
+{
+  const int   lane = threadIdx.x & 31;
+  const bool  sx = (0x55u >> (lane & 7)) & 1u, sy = (0xa5u >> (lane & 7)) & 1u, sz = (0x99u >> (lane & 7)) & 1u;
+  const float ex = (sx ? r.cx + r.hx : r.cx - r.hx) - ax, ey = (sy ? r.cy + r.hy : r.cy - r.hy) - ay,
+              ez = (sz ? r.cz + r.hz : r.cz - r.hz) - az;
+  const float A  = sqrtf(fmaf(ex, ex, fmaf(ey, ey, ez * ez))) * 1.000004f + delta;
+  __syncwarp(); // the box before has been read
+  if (lane < 8) {
+    reinterpret_cast<float*>(pm.corner)[lane] = A;
+  }
+  __syncwarp();
+}
+
+// Whether the packet reaches the child of slot k of node `node`; child and cw are its words, d2 the squared
+// distance from the box's centre to it.
+__device__ __forceinline__ bool childReach(const EbgMeshView& m, const PacketMem& pm, const Reach& r, uint32_t node, int k,
+                                           uint32_t& child, uint32_t& cw, float& d2)
+{
+  const float4  A0 = pm.corner[0], A1 = pm.corner[1];
+  const float4* sl = reinterpret_cast<const float4*>(m.children + 4 * size_t(node) + k);
+  const float4  lo = __ldg(sl), hi = __ldg(sl + 1);
+  child = __float_as_uint(lo.w);
+  cw    = __float_as_uint(hi.w);
+  if ((child | cw) == 0u) { // an empty slot
+    return false;
+  }
+  if (!cornersReach(A0, A1, r.hx, r.hy, r.hz, r.cx - fminf(fmaxf(r.cx, lo.x), hi.x),
+                    r.cy - fminf(fmaxf(r.cy, lo.y), hi.y), r.cz - fminf(fmaxf(r.cz, lo.z), hi.z), d2)) {
+    return false;
+  }
+  const bool leaf = (child & EBG_LEAF_BIT) != 0u;
+  if (!leaf && !(cw & EBG_NODE_HAS_OBB)) {
+    return true;
+  }
+  return cornersReachObb(A0, A1, r.hx, r.hy, r.hz,
+                         reinterpret_cast<const float4*>(leaf ? m.obb + (cw >> EBG_COUNT_BITS) : m.node_obb + child), r.cx,
+                         r.cy, r.cz, d2);
+}
+
+// The lanes (bits) whose bound reaches this lane's leaf box: lanes [b, e), points and bounds in q.
+__device__ __forceinline__ unsigned lanesReach(const float4* __restrict__ ob, const float4* q, int b, int e)
+{
+  const float4 o0 = __ldg(ob), o1 = __ldg(ob + 1), o2 = __ldg(ob + 2), o3 = __ldg(ob + 3);
+  unsigned     mask = 0u;
+#pragma unroll 1
+  for (int j = b & ~3; j < e; j += 4) {
+    unsigned four = 0u;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const float4 p = q[j + i];
+      if (obbDist2(o0, o1, o2, o3, p.x, p.y, p.z) <= p.w) {
+        four |= 1u << i;
+      }
+    }
+    mask |= four << j;
+  }
+  return mask;
+}
+
+// A query's results from its winning triangle (-1: none).
+__device__ __forceinline__ void store(const MeshQueryArgs& a, const EbgMeshView& m, int tri, float px, float py, float pz,
+                                      uint32_t id, int64_t pos)
+{
+  const float dist = tri >= 0 ? signedFromWinner(m, uint32_t(tri), px, py, pz) : FLT_MAX;
+  a.out_d[id]      = dist;
+  if (a.out_tri) {
+    a.out_tri[id] = tri >= 0 ? (a.tri_leaf ? tri : __ldg(m.tri_id + tri)) : -1;
+  }
+  if (a.band_flag) {
+    // one flag per sorted position; the list is compacted from them in position order
+    a.band_flag[pos] = uint8_t(tri >= 0 && fabsf(dist) <= a.band);
+  }
+}
+
+// The points that kMeshPacket32 put aside, eight lanes each.
+__global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshListed(const __grid_constant__ MeshQueryArgs a, float delta)
+{
+  __shared__ GroupMem mem[4 * PACKET_WARPS];
+  const EbgMeshView&  m   = a.mesh;
+  const uint32_t      n   = a.band_count[1];
+  const uint32_t      nG  = gridDim.x * (4 * PACKET_WARPS);
+  const uint32_t      grp = threadIdx.x >> 3;
+  for (uint32_t i0 = blockIdx.x * (4 * PACKET_WARPS) + (grp & ~3u); i0 < n; i0 += nG) {
+    const uint32_t i   = i0 + (grp & 3u);
+    const bool     on  = i < n;
+    const uint32_t pos = __ldg(a.point_list + (on ? i : i0));
+    const uint32_t id  = a.order ? __ldg(a.order + pos) : pos;
+    const float    px = __ldg(a.points + 3 * size_t(id)), py = __ldg(a.points + 3 * size_t(id) + 1),
+                pz = __ldg(a.points + 3 * size_t(id) + 2);
+    float     bd2;
+    int       bt;
+    const int err = groupNearest(m, on, px, py, pz, delta, mem[grp], bd2, bt);
+    if (on && (threadIdx.x & 7) == 0) {
+      if (err) {
+        atomicOr(a.status, err);
+      }
+      store(a, m, bt, px, py, pz, id, pos);
+    }
+    __syncwarp();
+  }
+}
+
+// 32 waiting pairs (or the last ones): a lane per pair tests its leaf's triangles.
+__device__ __forceinline__ void testPairs(const EbgMeshView& m, PacketMem& pm, int first, int count)
+{
+  const int      lane = threadIdx.x & 31;
+  const bool     on   = lane < count;
+  uint32_t       tt = on ? pm.pairTri[first + lane] : 0u;
+  const uint32_t v  = on ? pm.pairLane[first + lane] : 0u;
+  const uint32_t te = tt + (v >> 5), ql = v & 31u;
+  const float4   q  = pm.query[ql];
+  float          d  = __int_as_float(0x7f800000);
+  uint32_t       di = 0u;
+#pragma unroll 1
+  for (; tt < te; tt++) {
+    const float4* h  = reinterpret_cast<const float4*>(m.hot + tt);
+    const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+    float         s, t;
+    int           r;
+    const float   dd = triDist2<false>(h0, h1, h2, q.x, q.y, q.z, s, t, r);
+    if (dd < d) { // the lower position on ties
+      d  = dd;
+      di = tt;
+    }
+  }
+  if (on && d <= q.w) {
+    atomicMin(pm.key + ql, (unsigned long long)__float_as_uint(d) << 32 | di);
+  }
+}
+
+// The anchor of the cell that holds a point (nearest cell outside the grid): the triangle nearest to
+// the cell's centre, or -1.
+__device__ __forceinline__ int cellAnchor(const SeedCellsView& cv, float px, float py, float pz)
+{
+  if (cv.anchor == nullptr) {
+    return -1;
+  }
+  const float gm = float(cv.g - 1);
+  const int   ix = int(fminf(fmaxf((px - cv.lo[0]) * cv.inv[0], 0.f), gm));
+  const int   iy = int(fminf(fmaxf((py - cv.lo[1]) * cv.inv[1], 0.f), gm));
+  const int   iz = int(fminf(fmaxf((pz - cv.lo[2]) * cv.inv[2], 0.f), gm));
+  return __ldg(cv.anchor + (int64_t(iz) * cv.g + iy) * cv.g + ix);
+}
+
+// CELLS: the query passes an attached model, and its cells' anchors give the lanes' first bounds and
+// the mesh points `a`.
+template <bool CELLS>
+__global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __grid_constant__ MeshQueryArgs a, float delta,
+                                                                     float split, bool sparse)
+{
+  __shared__ PacketMem mem[PACKET_WARPS];
+  const EbgMeshView&   m    = a.mesh;
+  PacketMem&           pm   = mem[threadIdx.x >> 5];
+  PointMem&            w    = pm.w;
+  const int            lane = threadIdx.x & 31;
+  const unsigned       lt   = (1u << lane) - 1u;
+  const float          inf  = __int_as_float(0x7f800000);
+  const uint64_t       numPackets = (uint64_t(a.n) + 31) / 32;
+  unsigned long long   pk = 0, pkEnd = 0;
+  int                  besttri = -1, frontN = 0;
+  int                  limit = 0; // leaves per point that a range may reach
+  while (true) {
+    if (pk == pkEnd) {
+      // fewer at a time towards the end (a stale count only shifts that)
+      unsigned long long take = 0;
+      if (lane == 0) {
+        const unsigned long long done = *reinterpret_cast<volatile unsigned long long*>(a.work);
+        take = done < numPackets ? (numPackets - done) / (gridDim.x * (2ull * PACKET_WARPS)) : 0ull;
+        take = take < 1ull ? 1ull : (take > (unsigned long long)a.chunk ? (unsigned long long)a.chunk : take);
+        pk   = atomicAdd(a.work, take);
+      }
+      pk    = __shfl_sync(FULL, pk, 0);
+      pkEnd = pk + __shfl_sync(FULL, take, 0);
+      if (pk >= numPackets) {
+        break;
+      }
+      // the group of packets: its box, a mesh point near it, and the frontier of the tree that it
+      // reaches -- at most PACKET_FRONT entries -- where its packets start
+      // (found from one of the points: the centre of a wide group may be equally far from everything)
+      float lx = inf, ly = inf, lz = inf, ux = -inf, uy = -inf, uz = -inf, qx = 0.f, qy = 0.f, qz = 0.f;
+      bool  got = false;
+      for (unsigned long long i = pk; i < pkEnd && i < numPackets; i++) {
+        const int64_t  pos = int64_t(i) * 32 + lane;
+        const uint32_t id  = pos < a.n ? (a.order ? __ldg(a.order + pos) : uint32_t(pos)) : 0u;
+        const float    px = __ldg(a.points + 3 * size_t(id)), py = __ldg(a.points + 3 * size_t(id) + 1),
+                    pz = __ldg(a.points + 3 * size_t(id) + 2);
+        const bool     ok  = pos < a.n && fabsf(px) + fabsf(py) + fabsf(pz) < 1e12f;
+        const unsigned mk  = __ballot_sync(FULL, ok);
+        if (!got && mk != 0u) {
+          const int j = (mk >> 16) & 1u ? 16 : __ffs(int(mk)) - 1;
+          qx          = __shfl_sync(FULL, px, j);
+          qy          = __shfl_sync(FULL, py, j);
+          qz          = __shfl_sync(FULL, pz, j);
+          got         = true;
+        }
+        if (ok) {
+          lx = fminf(lx, px), ly = fminf(ly, py), lz = fminf(lz, pz);
+          ux = fmaxf(ux, px), uy = fmaxf(uy, py), uz = fmaxf(uz, pz);
+        }
+      }
+      lx = warpMin(lx), ly = warpMin(ly), lz = warpMin(lz), ux = warpMax(ux), uy = warpMax(uy), uz = warpMax(uz);
+      Reach r;
+      r.cx = 0.5f * lx + 0.5f * ux, r.cy = 0.5f * ly + 0.5f * uy, r.cz = 0.5f * lz + 0.5f * uz;
+      r.hx = fmaxf(ux - r.cx, r.cx - lx), r.hy = fmaxf(uy - r.cy, r.cy - ly), r.hz = fmaxf(uz - r.cz, r.cz - lz);
+      besttri = -1;
+      frontN  = 1;
+      __syncwarp();
+      if (lane == 0) {
+        pm.last          = make_float4(qx, qy, qz, fmaxf(split, 0.f)); // (the first packet's anchor is found below)
+        pm.front[0]      = m.root_ref;
+        pm.frontCount[0] = m.root_count;
+      }
+      __syncwarp();
+      limit = numPackets - pk > gridDim.x * (8ull * PACKET_WARPS) ? 32 : 12;
+      if (got) {
+        float bd2;
+        int   err = 0;
+        if (CELLS) {
+          besttri = cellAnchor(a.cells, qx, qy, qz);
+        }
+        if (besttri < 0) {
+          err = pointNearest32<true>(m, qx, qy, qz, delta, w, bd2, besttri);
+        }
+        if (err && lane == 0) {
+          atomicOr(a.status, err);
+        }
+        if (besttri >= 0 && pkEnd - pk > 1 && !(m.root_ref & EBG_LEAF_BIT)) {
+          const float4* h  = reinterpret_cast<const float4*>(m.hot + besttri);
+          const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+          float         s, t, ax, ay, az;
+          int           reg;
+          triDist2<false>(h0, h1, h2, qx, qy, qz, s, t, reg);
+          triPoint(h0, h1, h2, s, t, ax, ay, az);
+          setCorners(pm, r, ax, ay, az, delta);
+          // level by level while the next level fits
+          for (int level = 0; level < EBG_STACK_DEPTH; level++) {
+            int  nn = 0; // the next level's entries, gathered in w
+            bool any = false;
+            for (int f = 0; f < frontN && nn <= PACKET_FRONT; f += 8) {
+              const int      g = lane >> 2, i = f + g;
+              const uint32_t ref = i < frontN ? pm.front[i] : EBG_LEAF_BIT;
+              const bool     leaf = (ref & EBG_LEAF_BIT) != 0u;
+              uint32_t       child = ref, cw = i < frontN ? pm.frontCount[i] : 0u;
+              float          d2;
+              bool           keep = i < frontN && leaf && (lane & 3) == 0;
+              if (!leaf) {
+                keep = childReach(m, pm, r, ref, lane & 3, child, cw, d2);
+              }
+              any |= __any_sync(FULL, !leaf) != 0;
+              const unsigned mk = __ballot_sync(FULL, keep);
+              if (keep && nn + __popc(mk) <= PACKET_FRONT) {
+                w.leafRef[nn + __popc(mk & lt)]   = child;
+                w.leafCount[nn + __popc(mk & lt)] = cw;
+              }
+              nn += __popc(mk);
+            }
+            __syncwarp();
+            if (nn > PACKET_FRONT || nn == 0 || !any) {
+              break;
+            }
+            if (lane < nn) {
+              pm.front[lane]      = w.leafRef[lane];
+              pm.frontCount[lane] = w.leafCount[lane];
+            }
+            frontN = nn;
+            __syncwarp();
+          }
+        }
+      }
+    }
+    if (pk >= numPackets) {
+      break;
+    }
+    const int64_t  pos   = int64_t(pk) * 32 + lane;
+    const bool     valid = pos < a.n;
+    const int64_t  src   = valid ? pos : a.n - 1;
+    const uint32_t id    = a.order ? __ldg(a.order + src) : uint32_t(src);
+    const float    px = __ldg(a.points + 3 * size_t(id)), py = __ldg(a.points + 3 * size_t(id) + 1),
+                pz = __ldg(a.points + 3 * size_t(id) + 2);
+    const bool finite = isfinite(px) && isfinite(py) && isfinite(pz);
+    const bool live   = valid && finite;
+    if (valid && !finite) {
+      atomicOr(a.status, ST_INPUT);
+    }
+    float best  = -1.f; // a lane without a live point needs nothing
+    int   prev  = besttri, err = 0;
+    bool  later = false; // the lane's point is on the list for kMeshListed
+    besttri     = -1;
+    // ranges [b, e) of lanes, each compact enough for one box
+    int  b = 0, e = 32;
+    while (b < 32 && err == 0) {
+      const bool  in  = live && lane >= b && lane < e;
+      const float mnx = warpMin(in ? px : inf), mny = warpMin(in ? py : inf), mnz = warpMin(in ? pz : inf);
+      const float mxx = warpMax(in ? px : -inf), mxy = warpMax(in ? py : -inf), mxz = warpMax(in ? pz : -inf);
+      Reach       r;
+      r.cx = 0.5f * mnx + 0.5f * mxx, r.cy = 0.5f * mny + 0.5f * mxy, r.cz = 0.5f * mnz + 0.5f * mxz;
+      r.hx = fmaxf(mxx - r.cx, r.cx - mnx), r.hy = fmaxf(mxy - r.cy, r.cy - mny), r.hz = fmaxf(mxz - r.cz, r.cz - mnz);
+      const float hm  = fmaxf(r.hx, fmaxf(r.hy, r.hz));
+      bool        box = hm <= split && !__any_sync(FULL, in && !(fabsf(px) + fabsf(py) + fabsf(pz) < 1e12f));
+      if (!box && e - b > 4 && hm <= 16.f * split) {
+        // divide at the widest step from one point to the next
+        const float ux = __shfl_up_sync(FULL, px, 1), uy = __shfl_up_sync(FULL, py, 1), uz = __shfl_up_sync(FULL, pz, 1);
+        const float dx = px - ux, dy = py - uy, dz = pz - uz;
+        const float step = lane > b && lane < e ? fmaf(dx, dx, fmaf(dy, dy, dz * dz)) : -1.f;
+        const float most = warpMax(step);
+        e                = most >= 0.f ? __ffs(int(__ballot_sync(FULL, step == most))) - 1 : b + 1;
+        continue;
+      }
+      box = box && e - b > 2;
+      if (box) {
+        // the mesh point `a` nearest to c among the winners of the packet before and of the ranges
+        // before; the lane's own one is its first bound
+        int            cand = besttri >= 0 ? besttri : prev;
+        const int      own  = CELLS ? cellAnchor(a.cells, px, py, pz) : -1;
+        cand                = CELLS && own >= 0 ? own : cand;
+        const float4   last = pm.last;
+        if (!__any_sync(FULL, own >= 0) && fmaxf(fabsf(r.cx - last.x), fmaxf(fabsf(r.cy - last.y), fabsf(r.cz - last.z))) > 4.f * (hm + last.w)) {
+          // a step of the ordering to somewhere else: those winners are far from nearest here
+          float bd2;
+          err |= pointNearest32<true>(m, __shfl_sync(FULL, px, b), __shfl_sync(FULL, py, b), __shfl_sync(FULL, pz, b), delta, w,
+                                bd2, cand);
+        }
+        const unsigned have = __ballot_sync(FULL, cand >= 0);
+        const int      alt  = __shfl_sync(FULL, cand, have ? __ffs(int(have)) - 1 : 0);
+        cand                = cand >= 0 ? cand : alt;
+        float ax = inf, ay = inf, az = inf;
+        if (in) {
+          best = FLT_MAX;
+        }
+        if (cand >= 0) {
+          const float4* h  = reinterpret_cast<const float4*>(m.hot + cand);
+          const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+          float         s, t;
+          int           reg;
+          const float   dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, reg);
+          if (in && dd <= FLT_MAX) {
+            best    = dd;
+            besttri = cand;
+          }
+          triPoint(h0, h1, h2, s, t, ax, ay, az);
+          const float ex = r.cx - ax, ey = r.cy - ay, ez = r.cz - az, dc = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+          const int from = (__ffs(int(__ballot_sync(FULL, dc == warpMin(dc)))) - 1) & 31;
+          ax             = __shfl_sync(FULL, ax, from);
+          ay             = __shfl_sync(FULL, ay, from);
+          az             = __shfl_sync(FULL, az, from);
+        }
+        setCorners(pm, r, ax, ay, az, delta);
+        pm.key[lane] = (unsigned long long)__float_as_uint(best) << 32 | uint32_t(besttri);
+        if (lane == 0) {
+          pm.last = make_float4(r.cx, r.cy, r.cz, hm);
+        }
+        int sp = 0, nl = 0, np = 0, listed = 0;
+        {
+          // the group's frontier, one entry per lane
+          uint32_t child = EBG_LEAF_BIT, cw = 0u;
+          float    d2    = 0.f;
+          bool     need  = lane < frontN;
+          if (need) {
+            child = pm.front[lane];
+            cw    = pm.frontCount[lane];
+          }
+          const bool leaf = (child & EBG_LEAF_BIT) != 0u;
+          if (need && (leaf || (cw & EBG_NODE_HAS_OBB))) {
+            need = cornersReachObb(
+              pm.corner[0], pm.corner[1], r.hx, r.hy, r.hz,
+              reinterpret_cast<const float4*>(leaf ? m.obb + (cw >> EBG_COUNT_BITS) : m.node_obb + child), r.cx, r.cy, r.cz, d2);
+          }
+          const unsigned ml = __ballot_sync(FULL, need && leaf), mn = __ballot_sync(FULL, need && !leaf);
+          if (need && leaf) {
+            const int p    = __popc(ml & lt);
+            w.leafRef[p]   = child;
+            w.leafCount[p] = cw;
+            w.leafKey[p]   = d2;
+          }
+          if (need && !leaf) {
+            w.ref[__popc(mn & lt)] = child;
+          }
+          nl = __popc(ml);
+          sp = __popc(mn);
+          __syncwarp();
+        }
+        uint32_t iters = 0;
+#pragma unroll 1
+        while (sp > 0 || nl > 0) {
+          if (++iters > MAX_ITERS) {
+            err |= ST_ITERS;
+            break;
+          }
+          if (nl >= 32 || sp == 0) {
+            if (listed == 0) {
+              // the two leaves nearest to c first: they bring the lanes' bounds near their final values
+              const int reps = sp == 0 && nl <= 3 ? nl : 2; // all of a short list
+              for (int rep = 0; rep < reps && nl > 0; rep++) {
+                const float k0 = lane < nl ? w.leafKey[lane] : inf, k1 = lane + 32 < nl ? w.leafKey[lane + 32] : inf;
+                const float kk = fminf(k0, k1);
+                const int   from = (__ffs(int(__ballot_sync(FULL, kk == warpMin(kk)))) - 1) & 31;
+                const int   at   = __shfl_sync(FULL, k0 <= k1 ? lane : lane + 32, from);
+                const uint32_t t0 = w.leafRef[at] & ~EBG_LEAF_BIT, cw = w.leafCount[at];
+                const float4*  ob = reinterpret_cast<const float4*>(m.obb + (cw >> EBG_COUNT_BITS));
+                const bool     nd = obbDist2(__ldg(ob), __ldg(ob + 1), __ldg(ob + 2), __ldg(ob + 3), px, py, pz) <= best;
+                const uint32_t te = t0 + (__any_sync(FULL, in && nd) ? cw & EBG_COUNT_MASK : 0u);
+#pragma unroll 1
+                for (uint32_t tt = t0; tt < te; tt++) {
+                  const float4* h  = reinterpret_cast<const float4*>(m.hot + tt);
+                  const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+                  float         s, t;
+                  int           reg;
+                  const float   dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, reg);
+                  if (in && (dd < best || (dd == best && int(tt) < besttri))) {
+                    best    = dd;
+                    besttri = int(tt);
+                  }
+                }
+                nl--;
+                __syncwarp();
+                if (lane == 0) {
+                  w.leafRef[at]   = w.leafRef[nl];
+                  w.leafCount[at] = w.leafCount[nl];
+                  w.leafKey[at]   = w.leafKey[nl];
+                }
+                __syncwarp();
+                listed++;
+              }
+              pm.key[lane] = (unsigned long long)__float_as_uint(best) << 32 | uint32_t(besttri);
+              if (nl == 0) {
+                __syncwarp();
+                continue;
+              }
+            }
+            // 32 leaves (or the last ones): a lane per leaf finds the lanes that need it
+            __syncwarp();
+            pm.query[lane] = make_float4(px, py, pz, in ? __uint_as_float(uint32_t(pm.key[lane] >> 32)) : -1.f);
+            __syncwarp();
+            const int take = nl < 32 ? nl : 32;
+            uint32_t  ref = 0, cw = 0;
+            unsigned  mask = 0u;
+            if (lane < take) {
+              ref = w.leafRef[nl - 1 - lane] & ~EBG_LEAF_BIT;
+              cw  = w.leafCount[nl - 1 - lane];
+              mask = lanesReach(reinterpret_cast<const float4*>(m.obb + (cw >> EBG_COUNT_BITS)), pm.query, b, e);
+            }
+            nl -= take;
+            listed += take;
+            // their pairs join the waiting ones, as many leaves at a time as there is room for, and
+            // go 32 at a time
+            const uint32_t cnt5 = (cw & EBG_COUNT_MASK) << 5;
+            while (__any_sync(FULL, mask != 0u)) {
+              const int mine = __popc(mask);
+              int       at   = mine;
+#pragma unroll
+              for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(FULL, at, o);
+                at += lane >= o ? v : 0;
+              }
+              const bool fits = np + at <= PACKET_PAIRS;
+              const int  end  = np + int(__reduce_max_sync(FULL, fits ? uint32_t(at) : 0u));
+              if (fits) {
+                at += np - mine;
+                while (mask != 0u) {
+                  pm.pairTri[at]    = ref;
+                  pm.pairLane[at++] = uint16_t(cnt5 | uint32_t(__ffs(int(mask)) - 1));
+                  mask &= mask - 1u;
+                }
+              }
+              np = end;
+              __syncwarp();
+              while (np >= 32) {
+                np -= 32;
+                testPairs(m, pm, np, 32);
+              }
+              __syncwarp();
+            }
+            if (listed > limit * (e - b)) {
+              box   = false;
+              limit = sparse ? limit : (limit > 12 ? 16 : 8);
+              break;
+            }
+            continue;
+          }
+          const int take = sp <= POINT_WIDE ? (sp < 8 ? sp : 8) : 1;
+          const int  g = lane >> 2;
+          uint32_t   child = 0, cw = 0;
+          float      d2;
+          const bool need = g < take && childReach(m, pm, r, w.ref[g < take ? sp - 1 - g : 0], lane & 3, child, cw, d2);
+          const bool leaf = (child & EBG_LEAF_BIT) != 0u;
+          sp -= take;
+          const unsigned ml = __ballot_sync(FULL, need && leaf), mn = __ballot_sync(FULL, need && !leaf);
+          __syncwarp(); // the taken entries are read before they are overwritten
+          if (need && leaf) {
+            const int p    = nl + __popc(ml & lt);
+            w.leafRef[p]   = child;
+            w.leafCount[p] = cw;
+            w.leafKey[p]   = d2;
+          }
+          if (need && !leaf) {
+            w.ref[sp + __popc(mn & lt)] = child;
+          }
+          nl += __popc(ml);
+          sp += __popc(mn);
+          __syncwarp();
+          if (sp > POINT_NODES - 4) { // never for trees the builder accepts
+            err |= ST_STACK;
+            break;
+          }
+        }
+        if (np > 0) {
+          testPairs(m, pm, 0, np);
+        }
+        __syncwarp();
+        const unsigned long long kb = pm.key[lane];
+        if (in) {
+          best    = __uint_as_float(uint32_t(kb >> 32));
+          besttri = int(uint32_t(kb));
+        }
+      }
+      if (!box) {
+        // too wide, far away, very few points, too many leaves in reach, or no live lane at all: one
+        // warp per point, later
+        const unsigned todo = __ballot_sync(FULL, in);
+        if (todo != 0u) {
+          uint32_t base = 0;
+          if (lane == 0) {
+            base = atomicAdd(a.band_count + 1, uint32_t(__popc(todo)));
+          }
+          base = __shfl_sync(FULL, base, 0);
+          if (in) {
+            a.point_list[base + __popc(todo & lt)] = uint32_t(pos);
+            later                                  = true;
+          }
+        }
+      }
+      b = e;
+      e = 32;
+    }
+
+    if (err && lane == 0) {
+      atomicOr(a.status, err);
+    }
+    if (valid && !later) {
+      store(a, m, besttri, px, py, pz, id, pos);
+    }
+    if (besttri < 0) {
+      besttri = prev; // still a mesh triangle nearby
+    }
+    __syncwarp();
+    pk++;
+  }
+}
+
+} // namespace
+
+namespace {
+__global__ void kNodeChildren(const EbgNode4* __restrict__ nodes, int64_t slots, EbgChild* __restrict__ out)
+{
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < slots; i += int64_t(gridDim.x) * blockDim.x) {
+    const EbgNode4& n = nodes[i >> 2];
+    const int       k = int(i & 3);
+    out[i]            = EbgChild{n.lox[k], n.loy[k], n.loz[k], n.child[k], n.hix[k], n.hiy[k], n.hiz[k], n.count[k]};
+  }
+}
+} // namespace
+
+void launchNodeChildren(const EbgNode4* nodes, int64_t numNodes, EbgChild* children, cudaStream_t s)
+{
+  const int64_t blocks = (4 * numNodes + 255) / 256;
+  if (blocks > 0) {
+    kNodeChildren<<<unsigned(blocks < 4096 ? blocks : 4096), 256, 0, s>>>(nodes, 4 * numNodes, children);
+  }
+}
+
+cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, int64_t numLeaves, int numSms, cudaStream_t s)
+{
+  const int64_t packets = (a.n + 31) / 32;
+  const int64_t need    = (packets + PACKET_WARPS - 1) / PACKET_WARPS;
+  const int64_t most    = int64_t(numSms) * 8;
+  const int64_t grid    = need < most ? need : most;
+  a.chunk = a.chunk > 1 ? a.chunk : 8; // packets per group
+  if (a.cells.count != nullptr) {
+    kMeshPacket32<true><<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta, split, packets < numLeaves);
+  }
+  else {
+    kMeshPacket32<false><<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta, split, packets < numLeaves);
+  }
+  kMeshListed<<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta);
+  return cudaGetLastError();
+}
+
+} // namespace ebg

@@ -52,8 +52,9 @@ __device__ __forceinline__ float boxMinMax2(float lx, float ly, float lz, float 
 // Runs `tris(active, triangle)` -- all 32 lanes together -- over the triangles of every leaf whose
 // boxes lie within `bound` (squared, warp-uniform; the callback lowers it).  With UPPER, boxes lower
 // it too: an upper bound r of the distance becomes r * 1.00001 + slack, which covers the FP32 error
-// of the triangle distances that are compared with it.  Returns ST_* bits.
-template <bool UPPER, class TriFn>
+// of the triangle distances that are compared with it.  With FIRST the search ends after the first
+// leaves, the nearest found so far: a near triangle, not always the nearest.  Returns ST_* bits.
+template <bool UPPER, bool FIRST = false, class TriFn>
 __device__ __forceinline__ int pointSearch(const EbgMeshView& m, float px, float py, float pz, float& bound, float slack,
                                            PointMem& w, TriFn&& tris)
 {
@@ -135,24 +136,25 @@ __device__ __forceinline__ int pointSearch(const EbgMeshView& m, float px, float
         const int j = t + (lane & 7);
         tris(j < cnt, t0 + uint32_t(j < cnt ? j : 0));
       }
+      if (FIRST) {
+        return 0;
+      }
       continue;
     }
     const int  take = sp <= POINT_WIDE ? (sp < 8 ? sp : 8) : 1;
     const int  g    = lane >> 2, k = lane & 3;
     bool       need = g < take && w.key[g < take ? sp - 1 - g : 0] <= bound;
-    uint32_t   ref = 0, child = 0, cw = 0;
+    uint32_t   child = 0, cw = 0;
     float      d2 = inf, up = inf;
     if (need) {
-      ref               = w.ref[sp - 1 - g];
-      const EbgNode4* nd = m.nodes + ref;
-      const float lx = __ldg(nd->lox + k), ly = __ldg(nd->loy + k), lz = __ldg(nd->loz + k);
-      const float hx = __ldg(nd->hix + k), hy = __ldg(nd->hiy + k), hz = __ldg(nd->hiz + k);
-      child = __ldg(nd->child + k);
-      cw    = __ldg(nd->count + k);
+      const float4* sl = reinterpret_cast<const float4*>(m.children + 4 * size_t(w.ref[sp - 1 - g]) + k);
+      const float4  lo = __ldg(sl), hi = __ldg(sl + 1);
+      child = __float_as_uint(lo.w);
+      cw    = __float_as_uint(hi.w);
       need  = (child | cw) != 0u; // an empty slot
       if (need) {
-        d2 = boxDist2(lx, ly, lz, hx, hy, hz, px, py, pz);
-        up = boxMinMax2(lx, ly, lz, hx, hy, hz, px, py, pz);
+        d2 = boxDist2(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, px, py, pz);
+        up = boxMinMax2(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, px, py, pz);
       }
     }
     sp -= take;
@@ -189,6 +191,155 @@ __device__ __forceinline__ int pointSearch(const EbgMeshView& m, float px, float
     }
   }
   return 0;
+}
+
+// ---- eight lanes per point ---------------------------------------------------------------------------
+//
+// With more points than warps the 32 lanes of pointSearch are too many for one point: most rounds
+// have fewer than 32 children worth testing.  Here four points share a warp, each with eight lanes:
+// a round takes the two entries on top of the group's stack, pushes the children in order of
+// distance (nearest on top) and then tests the leaf on top, if one is.
+
+// Entries per group: a round of two nodes starts at or below GROUP_WIDE entries and adds at most 6;
+// above it a round takes one node, which adds at most 3 entries per tree level.
+constexpr int GROUP_WIDE  = 24;
+constexpr int GROUP_STACK = GROUP_WIDE + 6 + EBG_STACK_DEPTH;
+
+struct GroupMem
+{
+  uint32_t ref[GROUP_STACK], count[GROUP_STACK];
+  float    key[GROUP_STACK];
+};
+
+// The least value of x over the eight lanes of each group.
+__device__ __forceinline__ float groupMin(float x)
+{
+  x = fminf(x, __shfl_xor_sync(FULL, x, 1));
+  x = fminf(x, __shfl_xor_sync(FULL, x, 2));
+  return fminf(x, __shfl_xor_sync(FULL, x, 4));
+}
+
+// The nearest triangle (FP32, ties to the lower leaf position) of each group's point; groups without
+// a point pass on = false.  All 32 lanes call it together; `g` is the group's memory.  Returns ST_* bits.
+__device__ __forceinline__ int groupNearest(const EbgMeshView& m, bool on, float px, float py, float pz, float slack,
+                                            GroupMem& g, float& bd2, int& bt)
+{
+  const int      lane = threadIdx.x & 31, sub = lane & 7, base = lane & 24;
+  const unsigned mine = 0xffu << base;
+  const float    inf  = __int_as_float(0x7f800000);
+  float          bound = FLT_MAX;
+  int            sp = on ? 1 : 0;
+  bd2               = inf;
+  bt                = -1;
+  if (on && sub == 0) {
+    g.ref[0]   = m.root_ref;
+    g.count[0] = m.root_count;
+    g.key[0]   = boxDist2(m.root_lo[0], m.root_lo[1], m.root_lo[2], m.root_hi[0], m.root_hi[1], m.root_hi[2], px, py, pz);
+  }
+  __syncwarp();
+  uint32_t iters = 0;
+#pragma unroll 1
+  while (true) {
+    // down to the topmost entry still within the bound, eight at a time
+    {
+      const int      i   = sp - 1 - sub;
+      const unsigned ok  = (__ballot_sync(FULL, i >= 0 && g.key[i >= 0 ? i : 0] <= bound) & mine) >> base;
+      sp                 = ok != 0u ? sp - (__ffs(int(ok)) - 1) : (sp > 8 ? sp - 8 : 0);
+      if (!__any_sync(FULL, sp > 0)) {
+        return 0;
+      }
+      if (++iters > MAX_ITERS) {
+        return ST_ITERS;
+      }
+    }
+    // the node on top and the entry below it, if that is a node as well
+    const uint32_t top  = sp > 0 ? g.ref[sp - 1] : EBG_LEAF_BIT;
+    const bool     node = !(top & EBG_LEAF_BIT) && (sp > 0 && g.key[sp > 0 ? sp - 1 : 0] <= bound);
+    if (__any_sync(FULL, node)) {
+      const uint32_t below = node && sp > 1 && sp <= GROUP_WIDE ? g.ref[sp - 2] : EBG_LEAF_BIT;
+      const bool     two   = !(below & EBG_LEAF_BIT);
+      const uint32_t ref   = sub < 4 ? top : below;
+      bool           need  = node && (sub < 4 || two);
+      uint32_t       child = 0, cw = 0;
+      float          d2 = inf, up = inf;
+      if (need) {
+        const float4* sl = reinterpret_cast<const float4*>(m.children + 4 * size_t(ref) + (sub & 3));
+        const float4  lo = __ldg(sl), hi = __ldg(sl + 1);
+        child = __float_as_uint(lo.w);
+        cw    = __float_as_uint(hi.w);
+        need  = (child | cw) != 0u; // an empty slot
+        if (need) {
+          d2 = boxDist2(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, px, py, pz);
+          up = boxMinMax2(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, px, py, pz);
+        }
+      }
+      const float r = sqrtf(groupMin(up)) * 1.00001f + slack; // see pointSearch
+      bound         = fminf(bound, r * r);
+      need          = need && d2 <= bound;
+      const bool leaf = (child & EBG_LEAF_BIT) != 0u;
+      if (need && (leaf || (cw & EBG_NODE_HAS_OBB))) {
+        const float4* ob = reinterpret_cast<const float4*>(leaf ? m.obb + (cw >> EBG_COUNT_BITS) : m.node_obb + child);
+        d2   = fmaxf(d2, obbDist2(__ldg(ob), __ldg(ob + 1), __ldg(ob + 2), __ldg(ob + 3), px, py, pz));
+        need = d2 <= bound;
+      }
+      // farther children deeper (ties by lane)
+      const float mk   = need ? d2 : -1.f;
+      int         rank = 0, all = 0;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const float ok = __shfl_sync(FULL, mk, i, 8);
+        rank += int(ok > mk || (ok == mk && i < sub));
+        all += int(ok >= 0.f);
+      }
+      sp -= node ? (two ? 2 : 1) : 0;
+      __syncwarp(); // the taken entries are read before they are overwritten
+      if (need) {
+        g.ref[sp + rank]   = child;
+        g.count[sp + rank] = cw;
+        g.key[sp + rank]   = d2;
+      }
+      sp += all;
+      __syncwarp();
+      if (__any_sync(FULL, sp > GROUP_STACK - 8)) { // never for trees the builder accepts
+        return ST_STACK;
+      }
+    }
+    // the leaf on top
+    const uint32_t lr   = sp > 0 ? g.ref[sp - 1] : 0u;
+    const bool     test = (lr & EBG_LEAF_BIT) && g.key[sp > 0 ? sp - 1 : 0] <= bound;
+    if (__any_sync(FULL, test)) {
+      const uint32_t t0  = lr & ~EBG_LEAF_BIT;
+      const int      cnt = test ? int(g.count[sp - 1] & EBG_COUNT_MASK) : 0;
+      sp -= test ? 1 : 0;
+      __syncwarp(); // read before it is overwritten
+      const int most = int(__reduce_max_sync(FULL, uint32_t(cnt)));
+      float     dd = inf;
+      int       tri = 0x7fffffff;
+      for (int t = sub; t < most; t += 8) {
+        if (t < cnt) {
+          const float4* h  = reinterpret_cast<const float4*>(m.hot + t0 + t);
+          const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+          float         s_, t_;
+          int           r_;
+          const float   d = triDist2<false>(h0, h1, h2, px, py, pz, s_, t_, r_);
+          if (d < dd) {
+            dd  = d;
+            tri = int(t0) + t;
+          }
+        }
+      }
+      const float dm = groupMin(dd);
+      tri            = dd == dm ? tri : 0x7fffffff;
+      tri            = min(tri, __shfl_xor_sync(FULL, tri, 1));
+      tri            = min(tri, __shfl_xor_sync(FULL, tri, 2));
+      tri            = min(tri, __shfl_xor_sync(FULL, tri, 4));
+      if (test && (dm < bd2 || (dm == bd2 && tri < bt))) {
+        bd2   = dm;
+        bt    = tri;
+        bound = fminf(bound, bd2);
+      }
+    }
+  }
 }
 
 // Lower bound of the distance from p to a triangle from the closest point that triDist2 found: with

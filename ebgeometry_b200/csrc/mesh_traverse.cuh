@@ -159,6 +159,95 @@ __device__ __forceinline__ float lds1(uint32_t addr)
 // its 64-byte oriented box.
 constexpr uint32_t TOP_NODE_BYTES = 192;
 
+// Tests the triangles [t0, t0 + cnt) of one leaf for the lanes of needMask (this lane's bit is
+// needObb): updates their best squared distance and triangle.  All 32 lanes call it together; `pts`
+// is the warp's 32-entry scratch.
+template <bool STATS>
+__device__ __forceinline__ void packetLeaf(const EbgMeshView& m, uint32_t t0, uint32_t cnt, bool needObb,
+                                           unsigned needMask, float px, float py, float pz, float& best, int& besttri,
+                                           float4* pts, TraversalCounters& cnt_)
+{
+  const int lane = threadIdx.x & 31;
+  // Few lanes need the leaf: spread their (lane, triangle) pairs over the warp, 32 / cnt
+  // lanes per pass, instead of every lane testing every triangle.  A pass costs about two
+  // triangle tests, so this runs when it needs at most cnt / 2 passes (level-8 step:
+  // 103.7 ms seeded, 185.4 plain; at most cnt - 2 passes: 104.6, 186.6; at most cnt / 3:
+  // 104.7, 186.0).
+  const int nNeed  = __popc(needMask);
+  const int lpp    = int(c_lanesPer[cnt]);
+  const int passes = divSmall(nNeed + lpp - 1, lpp);
+  if (STATS && needObb) {
+    cnt_.leaf++;
+    cnt_.tri += cnt;
+  }
+  if (STATS) {
+    cnt_.pleaf++;
+    cnt_.ptri += 2 * passes <= int(cnt) ? uint32_t(passes) : cnt;
+    cnt_.precs += cnt;
+  }
+  if (2 * passes <= int(cnt)) {
+    const int rank = __popc(needMask & ((1u << lane) - 1u));
+    if (needObb) {
+      pts[rank] = make_float4(px, py, pz, 0.f);
+    }
+    __syncwarp();
+    const int     li = divSmall(lane, int(cnt)), ti = lane - li * int(cnt);
+    const float4* h  = reinterpret_cast<const float4*>(m.hot + t0 + uint32_t(ti));
+#pragma unroll 1
+    for (int ps = 0; ps < passes; ps++) {
+      const int slot = ps * lpp + li;
+      float     dd   = __int_as_float(0x7f800000);
+      int       bi   = ti;
+      if (li < lpp && slot < nNeed) {
+        const float4 q  = pts[slot];
+        const float4 h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+        float        s, t;
+        int          r;
+        dd = triDist2<false>(h0, h1, h2, q.x, q.y, q.z, s, t, r);
+      }
+      // minimum of (d2, triangle) over the cnt threads serving one lane; the first thread
+      // of the segment ends with it (offsets of cnt or more reach no segment partner)
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        if (off >= int(cnt)) {
+          continue;
+        }
+        const float od = __shfl_down_sync(FULL, dd, off);
+        const int   oi = __shfl_down_sync(FULL, bi, off);
+        if (ti + off < int(cnt) && (od < dd || (od == dd && oi < bi))) {
+          dd = od;
+          bi = oi;
+        }
+      }
+      const int  seg  = rank - ps * lpp;
+      const bool mine = needObb && seg >= 0 && seg < lpp;
+      const int  from = mine ? seg * int(cnt) : 0;
+      const float rd = __shfl_sync(FULL, dd, from);
+      const int   ri = __shfl_sync(FULL, bi, from);
+      // ties go to the lower leaf position, so the winner does not depend on the order
+      // in which packets meet the triangles
+      if (mine && (rd < best || (rd == best && int(t0) + ri < besttri))) {
+        best    = rd;
+        besttri = int(t0) + ri;
+      }
+    }
+    __syncwarp();
+    return;
+  }
+#pragma unroll 1
+  for (uint32_t tt = t0; tt < t0 + cnt; ++tt) {
+    const float4* h = reinterpret_cast<const float4*>(m.hot + tt);
+    const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+    float         s, t;
+    int           r;
+    const float   dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
+    if (dd < best || (dd == best && int(tt) < besttri)) {
+      best    = dd;
+      besttri = int(tt);
+    }
+  }
+}
+
 // Packet traversal of mesh m from the `sp` entries already on the warp's stack (the top entry is
 // popped first): each lane's best squared distance `best` (its pruning bound, already seeded or
 // FLT_MAX) and winning triangle `besttri` (leaf order) are updated.  Children are ordered by their
@@ -210,84 +299,7 @@ __device__ __forceinline__ void traverseFrom(const EbgMeshView& m, float px, flo
           if (needMask == 0u) {
             continue;
           }
-          // Few lanes need the leaf: spread their (lane, triangle) pairs over the warp, 32 / cnt
-          // lanes per pass, instead of every lane testing every triangle.  A pass costs about two
-          // triangle tests, so this runs when it needs at most cnt / 2 passes (level-8 step:
-          // 103.7 ms seeded, 185.4 plain; at most cnt - 2 passes: 104.6, 186.6; at most cnt / 3:
-          // 104.7, 186.0).
-          const int nNeed  = __popc(needMask);
-          const int lpp    = int(c_lanesPer[cnt]);
-          const int passes = divSmall(nNeed + lpp - 1, lpp);
-          if (STATS && needObb) {
-            cnt_.leaf++;
-            cnt_.tri += cnt;
-          }
-          if (STATS) {
-            cnt_.pleaf++;
-            cnt_.ptri += 2 * passes <= int(cnt) ? uint32_t(passes) : cnt;
-            cnt_.precs += cnt;
-          }
-          if (2 * passes <= int(cnt)) {
-            const int rank = __popc(needMask & ((1u << lane) - 1u));
-            if (needObb) {
-              pts[rank] = make_float4(px, py, pz, 0.f);
-            }
-            __syncwarp();
-            const int     li = divSmall(lane, int(cnt)), ti = lane - li * int(cnt);
-            const float4* h  = reinterpret_cast<const float4*>(m.hot + t0 + uint32_t(ti));
-#pragma unroll 1
-            for (int ps = 0; ps < passes; ps++) {
-              const int slot = ps * lpp + li;
-              float     dd   = __int_as_float(0x7f800000);
-              int       bi   = ti;
-              if (li < lpp && slot < nNeed) {
-                const float4 q  = pts[slot];
-                const float4 h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-                float        s, t;
-                int          r;
-                dd = triDist2<false>(h0, h1, h2, q.x, q.y, q.z, s, t, r);
-              }
-              // minimum of (d2, triangle) over the cnt threads serving one lane; the first thread
-              // of the segment ends with it (offsets of cnt or more reach no segment partner)
-#pragma unroll
-              for (int off = 16; off > 0; off >>= 1) {
-                if (off >= int(cnt)) {
-                  continue;
-                }
-                const float od = __shfl_down_sync(FULL, dd, off);
-                const int   oi = __shfl_down_sync(FULL, bi, off);
-                if (ti + off < int(cnt) && (od < dd || (od == dd && oi < bi))) {
-                  dd = od;
-                  bi = oi;
-                }
-              }
-              const int  seg  = rank - ps * lpp;
-              const bool mine = needObb && seg >= 0 && seg < lpp;
-              const int  from = mine ? seg * int(cnt) : 0;
-              const float rd = __shfl_sync(FULL, dd, from);
-              const int   ri = __shfl_sync(FULL, bi, from);
-              // ties go to the lower leaf position, so the winner does not depend on the order
-              // in which packets meet the triangles
-              if (mine && (rd < best || (rd == best && int(t0) + ri < besttri))) {
-                best    = rd;
-                besttri = int(t0) + ri;
-              }
-            }
-            __syncwarp();
-            continue;
-          }
-#pragma unroll 1
-          for (uint32_t tt = t0; tt < t0 + cnt; ++tt) {
-            const float4* h = reinterpret_cast<const float4*>(m.hot + tt);
-            const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-            float         s, t;
-            int           r;
-            const float   dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
-            if (dd < best || (dd == best && int(tt) < besttri)) {
-              best    = dd;
-              besttri = int(tt);
-            }
-          }
+          packetLeaf<STATS>(m, t0, cnt, needObb, needMask, px, py, pz, best, besttri, pts, cnt_);
         }
         else if constexpr (W == 8) {
           static_assert(!TOP, "the shared-memory top tree is a 4-wide option");
