@@ -1,5 +1,6 @@
 // FP64 evaluation of mesh triangles for the near-surface passes (sm_100a), shared by the mesh band
-// kernel (mesh_band64.cu) and the CSG union's band kernel (scene_band64.cu).  Include it only from
+// kernels (mesh_band64.cu), the search of few points (mesh_point.cu) and the CSG union's band kernel
+// (scene_band64.cu).  Include it only from
 // translation units compiled with -fmad=false: the point-triangle arithmetic keeps the reference's
 // separate multiplies and adds in the reference's order.
 //
@@ -187,26 +188,21 @@ __device__ double dcelFaceUd2(const double* __restrict__ tri, const double* __re
 // One packet's FP64 search of mesh m.  Each lane has its FP64 point P, the FP32 point (px, py, pz)
 // at which boxes are tested (`shift` from P), its squared search bound `bound` (FP32, at the FP32
 // point) and its running FP64 result (best, bt: the value of smallest |d| and its triangle, leaf
-// order; DBL_MAX / -1 before the first).  Triangles are tested in FP64 with the Triangle test
-// (EVAL 0, TriMeshSDF) or the DCEL face (EVAL 1, MeshSDF); each winner shrinks the lane's bound.
-// Leaves and nodes are pruned by their axis-aligned and oriented boxes (padded to bound the exact
-// distance of every triangle inside from below).  All 32 lanes call it together; `stk` is the
-// warp's stack (STACK entries).  The search starts from the `sp0` entries already on the stack
-// (a cell's cut, the top entry popped first), or from the root when sp0 is 0.
-template <int EVAL, int STACK = EBG_STACK_DEPTH>
+// order; DBL_MAX / -1 before the first).  Triangles are tested in FP64 with the Triangle test; each winner
+// shrinks the lane's bound.  Leaves and nodes are pruned by their axis-aligned and oriented boxes (padded
+// to bound the exact distance of every triangle inside from below).  All 32 lanes call it together;
+// `stk` is the warp's stack (STACK entries).
+template <int STACK = EBG_STACK_DEPTH>
 __device__ void band64Mesh(const EbgMeshView& m, D3 P, float px, float py, float pz, float shift, float& bound,
-                           double& best, int& bt, float4* stk, uint32_t& iters, int& err, int sp0 = 0)
+                           double& best, int& bt, float4* stk, uint32_t& iters, int& err)
 {
   const int lane = threadIdx.x & 31;
-  int sp = sp0;
-  if (sp0 == 0) {
-    sp = 1;
-    if (lane == 0) {
-      stk[0] = make_float4(m.root_lo[0], m.root_lo[1], m.root_lo[2], __uint_as_float(m.root_ref));
-      stk[1] = make_float4(m.root_hi[0], m.root_hi[1], m.root_hi[2], __uint_as_float(m.root_count));
-    }
-    __syncwarp();
+  int       sp   = 1;
+  if (lane == 0) {
+    stk[0] = make_float4(m.root_lo[0], m.root_lo[1], m.root_lo[2], __uint_as_float(m.root_ref));
+    stk[1] = make_float4(m.root_hi[0], m.root_hi[1], m.root_hi[2], __uint_as_float(m.root_count));
   }
+  __syncwarp();
   while (sp > 0) {
     if (++iters > MAX_ITERS) {
       err |= ST_ITERS;
@@ -233,8 +229,7 @@ __device__ void band64Mesh(const EbgMeshView& m, D3 P, float px, float py, float
     if (ref & EBG_LEAF_BIT) {
       const uint32_t t0 = ref & ~EBG_LEAF_BIT;
       for (uint32_t tt = t0; tt < t0 + cnt; ++tt) {
-        const double d = EVAL == 0 ? triSd64(m.tri64 + 30 * size_t(tt), P)
-                                   : dcelFaceSd(m.tri64 + 30 * size_t(tt), m.dcel_n + 3 * size_t(tt), P);
+        const double d = triSd64(m.tri64 + 30 * size_t(tt), P);
         // strict < as the reference's leaf loop, ties to the lower leaf position (the winner is
         // then independent of the traversal order)
         if (fabs(d) < fabs(best) || (fabs(d) == fabs(best) && int(tt) < bt)) {

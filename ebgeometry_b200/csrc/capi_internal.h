@@ -11,6 +11,7 @@
 #include "cells_kernels.h"
 #include "ebg_layout.h"
 #include "ebgeometry_b200.h"
+#include "mesh_kernels.h"
 #include "seed_kernels.h"
 
 struct ebg_mesh
@@ -117,6 +118,14 @@ inline uint32_t   topNodesFor(const ebg_mesh* m, const ebg_query_opts* opts, boo
   t         = t < m->info.num_nodes ? t : m->info.num_nodes;
   return uint32_t(t);
 }
+
+// The FP32 pass of a query (see the definition for which search it takes); fp32Triangles: the caller
+// asked for closest triangles in FP32.
+cudaError_t launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool fp32Triangles, int warpsPerBlock,
+                           int occupancy, float delta, cudaStream_t s);
+
+// The half-extent up to which a packet of points shares one box.
+float packetSplit(const ebg_mesh* m);
 
 // The mesh query pipeline (ordering, optional seed inference, FP32 traversal, FP64 band pass) on
 // device buffers, asynchronous on s.  With pts64/out64 (the caller's FP64 points, of which pts is

@@ -508,6 +508,15 @@ bool pointPath(int64_t n, const ebg_query_opts* opts, const unsigned long long* 
          !(opts && (opts->timings || opts->top_nodes > 0 || opts->node_width > 0));
 }
 
+} // namespace
+
+float ebg::packetSplit(const ebg_mesh* m)
+{
+  // packets up to three mean leaf sizes wide share one box (the extent of a leaf on a surface of
+  // about the diagonal's square): 6 measured the same on dense points, 2-5 % slower on sparse ones
+  return 3.f * float(m->info.diagonal / std::sqrt(double(std::max<int64_t>(1, m->info.num_leaves))));
+}
+
 // The FP32 pass by packet boxes (mesh_packet.cu) or by the packet walk (mesh_sdf.cu).  The walk keeps
 //  - what only it has: counters, radius hints, the shared-memory top of the tree, the 8-wide copy;
 //  - meshes of fewer than 4,096 triangles, whose walk is short (4 M points on 1,280 triangles: 0.37
@@ -515,13 +524,15 @@ bool pointPath(int64_t n, const ebg_query_opts* opts, const unsigned long long* 
 //    1.8 ms everywhere);
 //  - FP32 calls that ask for the closest triangles: of triangles at exactly the same distance the walk
 //    names the one that its order and box rounding leave (2 points of 8 M differed).
-bool packetPath(const ebg_mesh* m, const MeshQueryArgs& a, int width, bool fp32Triangles)
+cudaError_t ebg::launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool fp32Triangles, int wpb, int occ,
+                                float delta, cudaStream_t s)
 {
-  return a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && width == 4 && !fp32Triangles &&
-         m->info.num_triangles >= 4096;
+  if (a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && a.node_width != 8 && !fp32Triangles &&
+      m->info.num_triangles >= 4096) {
+    return launchMeshPacket32(a, delta, packetSplit(m), m->info.num_leaves, m->numSms, s);
+  }
+  return launchMeshSdf32(a, wpb, m->numSms, s, occ);
 }
-
-} // namespace
 
 ebg_status ebg::meshQuery(const ebg_mesh*       m,
                           const float*          pts,
@@ -607,7 +618,8 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
 
   Workspace ws(s);
   uint32_t* order = nullptr;
-  uint32_t* pointList = nullptr; // points that the packet search puts aside
+  // what the packet searches put aside: points of the FP32 one, band entries of the FP64 one
+  uint32_t *pointList = nullptr, *later = nullptr;
   if (sort) {
     uint32_t* keysIn  = ws.get<uint32_t>(n);
     uint32_t* keysOut = ws.get<uint32_t>(n);
@@ -628,6 +640,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
       return setError(EBG_ERR_CUDA, "query sort failed");
     }
     pointList = idsIn; // free again after the sort
+    later     = keysIn;
   }
   // The band list: the traversal flags each sorted position, and a compaction of the flags gives
   // the list in position (Morton) order, so that each FP64 packet holds 32 neighbouring queries.
@@ -635,8 +648,11 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   // packets in flight.)
   if (pointList == nullptr) {
     pointList = ws.get<uint32_t>(n);
+    later     = ws.get<uint32_t>(n);
   }
-  unsigned long long* counters = ws.get<unsigned long long>(2); // [0] packets, [1] band count (u32)
+  int32_t* tri32 = fp64all ? ws.get<int32_t>(n) : nullptr;
+  unsigned long long* counters = ws.get<unsigned long long>(3); // [0] packets, [1] band and point list
+                                                                             // counts (u32), [2] FP64 leftovers (u32)
   uint32_t*           bandList = band64 ? ws.get<uint32_t>(n) : nullptr;
   uint8_t*            bandFlag = band64 ? ws.get<uint8_t>(n) : nullptr;
   size_t              selBytes = 0;
@@ -649,7 +665,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   if (!ws.ok) {
     return setError(EBG_ERR_NO_MEMORY, "query workspace allocation failed");
   }
-  cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), s);
+  cudaMemsetAsync(counters, 0, 3 * sizeof(unsigned long long), s);
   if (tm) {
     cudaEventRecord(ev[1], s);
   }
@@ -671,6 +687,8 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   a.band_count = reinterpret_cast<uint32_t*>(counters + 1);
   a.band_d32   = nullptr;
   a.point_list = pointList;
+  a.later       = later;
+  a.later_count = reinterpret_cast<uint32_t*>(counters + 2);
   a.band_flag  = bandFlag;
   a.work       = counters;
   a.status     = m->dStatus;
@@ -687,17 +705,20 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     a.top_nodes  = 0;
   }
   const float delta = float(2e-6 * fp32ErrorScale(m)) + 1e-30f;
-  if (packetPath(m, a, width, outTri != nullptr && !fp64all)) {
-    // packets up to three mean leaf sizes wide share one box (the extent of a leaf on a surface of
-    // about the diagonal's square): 6 measured the same on dense points, 2-5 % slower on sparse ones
-    const float leafSize = float(m->info.diagonal / std::sqrt(double(std::max<int64_t>(1, m->info.num_leaves))));
-    if (launchMeshPacket32(a, delta, 3.f * leafSize, m->info.num_leaves, m->numSms, s) != cudaSuccess) {
-      return setError(EBG_ERR_CUDA, std::string("traversal launch failed: ") + cudaGetErrorString(cudaGetLastError()));
+  if (tri32) {
+    if (outTri) {
+      cudaMemsetAsync(outTri, 0xff, size_t(n) * sizeof(int32_t), s); // -1: what is not finite keeps it
     }
+    // the FP32 winners are only the FP64 pass's starting points
+    a.out_tri  = tri32;
+    a.tri_leaf = 1;
   }
-  else if (launchMeshSdf32(a, wpb, m->numSms, s, occ) != cudaSuccess) {
+  if (launchMeshFp32(m, a, outTri != nullptr && !fp64all, wpb, occ, delta, s) != cudaSuccess) {
     return setError(EBG_ERR_CUDA, std::string("traversal launch failed: ") + cudaGetErrorString(cudaGetLastError()));
   }
+  a.out_tri    = outTri;
+  a.tri_leaf   = triLeafOrder ? 1 : 0;
+  a.tri32      = tri32;
   a.mesh       = m->view;
   a.node_width = 4;
   if (tm) {
@@ -710,7 +731,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     }
     // delta bounds the FP32 distance error: 2e-6 of the mesh's diagonal, or of its coordinates'
     // magnitude for a mesh far from the origin (about 17 FP32 roundings of either)
-    if (launchMeshBand64(a, delta, m->numSms, s) != cudaSuccess) {
+    if (launchMeshBand64(a, delta, packetSplit(m), m->numSms, s) != cudaSuccess) {
       return setError(EBG_ERR_CUDA, "band launch failed");
     }
     if (statsDev) {

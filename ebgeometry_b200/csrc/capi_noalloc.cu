@@ -137,7 +137,7 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
     off += align256(bytes);
     return p;
   };
-  auto* counters = reinterpret_cast<unsigned long long*>(take(2 * sizeof(unsigned long long)));
+  auto* counters = reinterpret_cast<unsigned long long*>(take(3 * sizeof(unsigned long long)));
   auto* keysIn   = reinterpret_cast<uint32_t*>(take(u32n));
   auto* keysOut  = reinterpret_cast<uint32_t*>(take(u32n));
   auto* idsIn    = reinterpret_cast<uint32_t*>(take(u32n));
@@ -162,7 +162,7 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
 
   // the array keeps the previous call's contents: clear what must start at zero (a stale packet
   // counter would make the traversal skip every packet)
-  if (cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess) {
+  if (cudaMemsetAsync(counters, 0, 3 * sizeof(unsigned long long), s) != cudaSuccess) {
     return cudaFailed("clearing the allocation-free counters");
   }
   if (sort) {
@@ -196,7 +196,11 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
     a.cells = m->cellsView; // the attached model's entry cuts live with the mesh
   }
   a.top_nodes = topNodesFor(m, opts, seed != nullptr);
-  if (launchMeshSdf32(a, wpb, m->numSms, s, occ) != cudaSuccess) {
+  a.point_list  = idsIn; // free after the sort
+  a.later       = keysIn;
+  a.later_count = reinterpret_cast<uint32_t*>(counters + 2);
+  const float delta = float(2e-6 * fp32ErrorScale(m)) + 1e-30f;
+  if (launchMeshFp32(m, a, closest_tri_dev != nullptr, wpb, occ, delta, s) != cudaSuccess) {
     return cudaFailed("traversal launch");
   }
   if (b64) {
@@ -205,7 +209,7 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
                                    bandCnt, int(n), s) != cudaSuccess) {
       return cudaFailed("band list compaction");
     }
-    if (launchMeshBand64(a, float(2e-6 * fp32ErrorScale(m)) + 1e-30f, m->numSms, s) != cudaSuccess) {
+    if (launchMeshBand64(a, delta, packetSplit(m), m->numSms, s) != cudaSuccess) {
       return cudaFailed("band launch");
     }
   }

@@ -28,6 +28,10 @@ struct MeshQueryArgs
   uint32_t*          band_count;
   uint32_t*          point_list; // sorted positions that the packet search leaves to one warp each; their
                                  // number is counted in band_count[1] (zeroed before the launch)
+  uint32_t*          later;       // entries of band_list that the packets of the FP64 pass leave to groups of
+                                  // lanes, counted in later_count (nullable: every entry takes a group)
+  uint32_t*          later_count; // zeroed before the launch
+  const int32_t*     tri32;       // the FP32 pass's winning triangles, leaf order, caller order (nullable)
   float*             band_d32;   // FP32 distance of each band entry (nullable: read out_d instead)
   uint8_t*           band_flag;  // per sorted position, 1 = needs FP64 (nullable: the traversal
                                  // appends to band_list itself, in completion order)
@@ -57,8 +61,8 @@ cudaError_t launchMeshSdf32(const MeshQueryArgs& a, int warpsPerBlock, int numSm
 // or 8-wide copy); delta as for launchMeshBand64; packets with a half-extent above split are divided.
 cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, int64_t numLeaves, int numSms, cudaStream_t s);
 
-// FP64 re-evaluation of the band list (reads band_count on the device).
-cudaError_t launchMeshBand64(const MeshQueryArgs& a, float delta, int numSms, cudaStream_t s);
+// FP64 re-evaluation of the band list (reads band_count on the device); split as for launchMeshPacket32.
+cudaError_t launchMeshBand64(const MeshQueryArgs& a, float delta, float split, int numSms, cudaStream_t s);
 
 // The whole query (FP64 results when a.out_d64 is set, else FP32 with the FP64 band pass if band64) with
 // one warp per point, for calls of few points; reads a.mesh, points / points64, n, band, eval and the

@@ -219,18 +219,18 @@ __device__ __forceinline__ float groupMin(float x)
   return fminf(x, __shfl_xor_sync(FULL, x, 4));
 }
 
-// The nearest triangle (FP32, ties to the lower leaf position) of each group's point; groups without
-// a point pass on = false.  All 32 lanes call it together; `g` is the group's memory.  Returns ST_* bits.
-__device__ __forceinline__ int groupNearest(const EbgMeshView& m, bool on, float px, float py, float pz, float slack,
-                                            GroupMem& g, float& bd2, int& bt)
+// Runs `leaf(test, t0, cnt, most)` for the leaves of each group's point whose boxes lie within the group's
+// `bound` (squared; the callback lowers it): triangles [t0, t0 + cnt) where `test`, `most` the warp's
+// largest cnt.  Groups without a point pass on = false.  UPPER and slack as for pointSearch.  All 32
+// lanes call it together; `g` is the group's memory.  Returns ST_* bits.
+template <bool UPPER, class LeafFn>
+__device__ __forceinline__ int groupSearch(const EbgMeshView& m, bool on, float px, float py, float pz, float& bound,
+                                           float slack, GroupMem& g, LeafFn&& leaf)
 {
   const int      lane = threadIdx.x & 31, sub = lane & 7, base = lane & 24;
   const unsigned mine = 0xffu << base;
   const float    inf  = __int_as_float(0x7f800000);
-  float          bound = FLT_MAX;
-  int            sp = on ? 1 : 0;
-  bd2               = inf;
-  bt                = -1;
+  int            sp   = on ? 1 : 0;
   if (on && sub == 0) {
     g.ref[0]   = m.root_ref;
     g.count[0] = m.root_count;
@@ -270,15 +270,19 @@ __device__ __forceinline__ int groupNearest(const EbgMeshView& m, bool on, float
         need  = (child | cw) != 0u; // an empty slot
         if (need) {
           d2 = boxDist2(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, px, py, pz);
-          up = boxMinMax2(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, px, py, pz);
+          if (UPPER) {
+            up = boxMinMax2(lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, px, py, pz);
+          }
         }
       }
-      const float r = sqrtf(groupMin(up)) * 1.00001f + slack; // see pointSearch
-      bound         = fminf(bound, r * r);
-      need          = need && d2 <= bound;
-      const bool leaf = (child & EBG_LEAF_BIT) != 0u;
-      if (need && (leaf || (cw & EBG_NODE_HAS_OBB))) {
-        const float4* ob = reinterpret_cast<const float4*>(leaf ? m.obb + (cw >> EBG_COUNT_BITS) : m.node_obb + child);
+      if (UPPER) {
+        const float r = sqrtf(groupMin(up)) * 1.00001f + slack;
+        bound         = fminf(bound, r * r);
+      }
+      need             = need && d2 <= bound;
+      const bool isLeaf = (child & EBG_LEAF_BIT) != 0u;
+      if (need && (isLeaf || (cw & EBG_NODE_HAS_OBB))) {
+        const float4* ob = reinterpret_cast<const float4*>(isLeaf ? m.obb + (cw >> EBG_COUNT_BITS) : m.node_obb + child);
         d2   = fmaxf(d2, obbDist2(__ldg(ob), __ldg(ob + 1), __ldg(ob + 2), __ldg(ob + 3), px, py, pz));
         need = d2 <= bound;
       }
@@ -312,34 +316,49 @@ __device__ __forceinline__ int groupNearest(const EbgMeshView& m, bool on, float
       const int      cnt = test ? int(g.count[sp - 1] & EBG_COUNT_MASK) : 0;
       sp -= test ? 1 : 0;
       __syncwarp(); // read before it is overwritten
-      const int most = int(__reduce_max_sync(FULL, uint32_t(cnt)));
-      float     dd = inf;
-      int       tri = 0x7fffffff;
-      for (int t = sub; t < most; t += 8) {
-        if (t < cnt) {
-          const float4* h  = reinterpret_cast<const float4*>(m.hot + t0 + t);
-          const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-          float         s_, t_;
-          int           r_;
-          const float   d = triDist2<false>(h0, h1, h2, px, py, pz, s_, t_, r_);
-          if (d < dd) {
-            dd  = d;
-            tri = int(t0) + t;
-          }
-        }
-      }
-      const float dm = groupMin(dd);
-      tri            = dd == dm ? tri : 0x7fffffff;
-      tri            = min(tri, __shfl_xor_sync(FULL, tri, 1));
-      tri            = min(tri, __shfl_xor_sync(FULL, tri, 2));
-      tri            = min(tri, __shfl_xor_sync(FULL, tri, 4));
-      if (test && (dm < bd2 || (dm == bd2 && tri < bt))) {
-        bd2   = dm;
-        bt    = tri;
-        bound = fminf(bound, bd2);
-      }
+      leaf(test, t0, cnt, int(__reduce_max_sync(FULL, uint32_t(cnt))));
     }
   }
+}
+
+// The nearest triangle (FP32, ties to the lower leaf position) of each group's point.
+__device__ __forceinline__ int groupNearest(const EbgMeshView& m, bool on, float px, float py, float pz, float slack,
+                                            GroupMem& g, float& bd2, int& bt)
+{
+  const int   sub   = threadIdx.x & 7;
+  const float inf   = __int_as_float(0x7f800000);
+  float       bound = FLT_MAX, b = inf;
+  int         best  = -1;
+  const int   err   = groupSearch<true>(m, on, px, py, pz, bound, slack, g, [&](bool test, uint32_t t0, int cnt, int most) {
+    float dd  = inf;
+    int   tri = 0x7fffffff;
+    for (int t = sub; t < most; t += 8) {
+      if (t < cnt) {
+        const float4* h  = reinterpret_cast<const float4*>(m.hot + t0 + t);
+        const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+        float         s_, t_;
+        int           r_;
+        const float   d = triDist2<false>(h0, h1, h2, px, py, pz, s_, t_, r_);
+        if (d < dd) {
+          dd  = d;
+          tri = int(t0) + t;
+        }
+      }
+    }
+    const float dm = groupMin(dd);
+    tri            = dd == dm ? tri : 0x7fffffff;
+    tri            = min(tri, __shfl_xor_sync(FULL, tri, 1));
+    tri            = min(tri, __shfl_xor_sync(FULL, tri, 2));
+    tri            = min(tri, __shfl_xor_sync(FULL, tri, 4));
+    if (test && (dm < b || (dm == b && tri < best))) {
+      b     = dm;
+      best  = tri;
+      bound = fminf(bound, b);
+    }
+  });
+  bd2 = b;
+  bt  = best;
+  return err;
 }
 
 // Lower bound of the distance from p to a triangle from the closest point that triDist2 found: with

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(128, 4) kSceneBand64(const SceneQueryArgs a, f
           float        bound = r * r;
           double       mb    = DBL_MAX;
           int          mbt   = -1;
-          band64Mesh<0>(mv, L, lx, ly, lz, shift, bound, mb, mbt, istk, iters, err);
+          band64Mesh(mv, L, lx, ly, lz, shift, bound, mb, mbt, istk, iters, err);
           if (err) {
             break;
           }

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from ebgeometry_b200 import EbgError, SeedModel, TriMeshSDF
+from ebgeometry_b200 import EbgError, MeshSDF, SeedModel, TriMeshSDF
 from ebgeometry_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +77,21 @@ def test_attached_model_and_refit():
     d_walk, _ = m.stats(p)
     assert torch.equal(m.signed_distance(p), d_walk)
     m.check_status()
+
+
+@pytest.mark.parametrize("cls", [TriMeshSDF, MeshSDF])
+@pytest.mark.parametrize("level,leaf,kind,n", [(5, 8, "uniform", 70001), (5, 32, "near", 131073), (6, 1, "grid", 100033),
+                                               (5, 8, "centre", 66001), (3, 8, "pairs", 65537), (5, 8, "same", 65568)])
+def test_fp64_pass_in_packets_equals_point_by_point(cls, level, leaf, kind, n):
+    """Calls of at most LIMIT points search point by point (tested against the exhaustive oracle);
+    a larger one takes the packets of the FP64 pass and the groups that they leave points to."""
+    v, f = W.displaced_icosphere(level, 9)
+    m = cls(v, f, leaf_size=leaf)
+    p = torch.from_numpy(_points(kind, v, f, n).astype(np.float64) + 1e-9).cuda()
+    tri = torch.empty(n, dtype=torch.int32, device="cuda")
+    d = m.signed_distance(p, closest_tri=tri)[0].clone()
+    m.check_status()
+    for b in range(0, n, LIMIT):
+        t = torch.empty(min(LIMIT, n - b), dtype=torch.int32, device="cuda")
+        part = m.signed_distance(p[b:b + LIMIT].contiguous(), closest_tri=t)[0]
+        assert torch.equal(d[b:b + LIMIT], part) and torch.equal(tri[b:b + LIMIT], t)
