@@ -11,12 +11,20 @@
 //   corner[num_corners][9]  the corner's position, its vertex pseudonormal, the pseudonormal of the
 //                           edge from it to the next corner
 //   face_id[num_faces]      int32: the face's index in the caller's soup
+//   face_disc, node_disc, slot_disc (32 B each, FP32): a disc that bounds from below what the faces under
+//                           it can return (see PolyDisc)
 //
 // MeshSDF: one warp per 32 Morton-ordered queries, boxes tested in FP32 at the FP32 rounding of the
 // point (bound r = (|best| + shift) (1 + 1e-6), shift = |P64 - P32|), faces evaluated in FP64; the
 // smallest |d| wins, ties to the lower leaf position.  FlatMeshSDF (MeshT::DirectSignedDistance2,
 // DCEL_MeshImplem.hpp:574-595): one thread per point over every face, the first face in soup order
 // with the smallest unsigned distance, then its signed distance.
+//
+// A face that is not quite planar can return less than the distance to its box (its value inside is the
+// distance to the plane through its centroid), so the result depends on which boxes were within the
+// bound when they came off the stack, as the reference's does.  The packet's stack order and box tests
+// are therefore fixed; what may be left out is the evaluation of faces that cannot lower a lane's
+// minimum, and that is what the discs are for.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -37,8 +45,22 @@
 namespace ebg {
 namespace {
 
+// A disc with centre c, unit normal n, half-thickness h and radius R that holds every point whose distance a
+// face below it can return: its corners, and -- for a face that is not planar -- its corners moved along
+// the axis its inside test drops onto the plane through its centroid (the foot of a point that tests
+// inside lies within those).  Padded for its own rounding.
+struct alignas(16) PolyDisc
+{
+  float cx, cy, cz, h;
+  float nx, ny, nz, R;
+};
+
 struct PolyView
 {
+  const PolyDisc* faceDisc;
+  const PolyDisc* nodeDisc; // per node
+  const PolyDisc* slotDisc; // per child slot, 4 per node
+  float           slack; // FP32 rounding of coordinates in a disc's bound
   const EbgNode4* nodes;
   const uint2*    face;
   const double*   faceRec;
@@ -59,6 +81,7 @@ struct PolyArgs
   double*         out;
   int32_t*        outFace;
   int*            status;
+  unsigned long long* work; // packet counter (zeroed before the launch)
 };
 
 struct P3
@@ -66,7 +89,7 @@ struct P3
   double x, y, z;
 };
 __device__ __forceinline__ P3 ld(const double* p) { return {p[0], p[1], p[2]}; }
-__device__ __forceinline__ P3 sub(P3 a, P3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
+__device__ __forceinline__ P3 sub_(P3 a, P3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ P3 add(P3 a, P3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ P3 scl(double s, P3 a) { return {s * a.x, s * a.y, s * a.z}; }
 __device__ __forceinline__ double dot(P3 a, P3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
@@ -84,7 +107,7 @@ __device__ bool polyInside(const double* __restrict__ cr, uint32_t N, P3 n, P3 c
   if (az > (ig == 0 ? ax : ay)) {
     ig = 2;
   }
-  const P3     q  = sub(P, scl(dot(n, sub(P, c)), n));
+  const P3     q  = sub_(P, scl(dot(n, sub_(P, c)), n));
   const double qx = ig == 0 ? q.y : q.x, qy = ig == 2 ? q.y : q.z;
   int          cn = 0;
   for (uint32_t i = 0; i < N; i++) {
@@ -105,7 +128,7 @@ __device__ bool polyInside(const double* __restrict__ cr, uint32_t N, P3 n, P3 c
 
 __device__ __forceinline__ double vertexSd(P3 x, P3 vn, P3 P)
 {
-  const P3 d = sub(P, x);
+  const P3 d = sub_(P, x);
   return len(d) * ((dot(vn, d) > 0.0) ? 1.0 : -1.0);
 }
 
@@ -117,15 +140,15 @@ __device__ double polyFaceSd(const PolyView& m, uint32_t f, P3 P)
   const double* cr = m.corner + 9 * size_t(fc.x);
   const P3      n = ld(fr), c = ld(fr + 3);
   if (polyInside(cr, fc.y, n, c, P)) {
-    return dot(n, sub(P, c));
+    return dot(n, sub_(P, c));
   }
   double best = CUDART_INF;
   for (uint32_t i = 0; i < fc.y; i++) {
     const double* a    = cr + 9 * size_t(i);
     const double* b    = cr + 9 * size_t(i + 1 == fc.y ? 0 : i + 1);
     const P3      xi   = ld(a), xj = ld(b);
-    const P3      x2x1 = sub(xj, xi);
-    const double  t    = dot(sub(P, xi), x2x1) / dot(x2x1, x2x1);
+    const P3      x2x1 = sub_(xj, xi);
+    const double  t    = dot(sub_(P, xi), x2x1) / dot(x2x1, x2x1);
     double        d;
     if (t <= 0.0) {
       d = vertexSd(xi, ld(a + 3), P);
@@ -134,7 +157,7 @@ __device__ double polyFaceSd(const PolyView& m, uint32_t f, P3 P)
       d = vertexSd(xj, ld(b + 3), P);
     }
     else {
-      const P3 delta = sub(P, add(xi, scl(t, x2x1)));
+      const P3 delta = sub_(P, add(xi, scl(t, x2x1)));
       d              = ((dot(ld(a + 6), delta) > 0.0) ? 1.0 : -1.0) * len(delta);
     }
     best = fabs(d) < fabs(best) ? d : best;
@@ -150,34 +173,142 @@ __device__ double polyFaceUd2(const PolyView& m, uint32_t f, P3 P)
   const double* cr = m.corner + 9 * size_t(fc.x);
   const P3      n = ld(fr), c = ld(fr + 3);
   if (polyInside(cr, fc.y, n, c, P)) {
-    const double nd = dot(n, sub(P, c));
+    const double nd = dot(n, sub_(P, c));
     return nd * nd;
   }
   double best = CUDART_INF;
   for (uint32_t i = 0; i < fc.y; i++) {
     const P3 xi   = ld(cr + 9 * size_t(i));
-    const P3 x2x1 = sub(ld(cr + 9 * size_t(i + 1 == fc.y ? 0 : i + 1)), xi);
-    double   t    = dot(sub(P, xi), x2x1) / dot(x2x1, x2x1);
+    const P3 x2x1 = sub_(ld(cr + 9 * size_t(i + 1 == fc.y ? 0 : i + 1)), xi);
+    double   t    = dot(sub_(P, xi), x2x1) / dot(x2x1, x2x1);
     t             = t < 0.0 ? 0.0 : (t > 1.0 ? 1.0 : t);
-    const P3     delta = sub(P, add(xi, scl(t, x2x1)));
+    const P3     delta = sub_(P, add(xi, scl(t, x2x1)));
     const double d2    = dot(delta, delta);
     best               = d2 < best ? d2 : best;
   }
   return best;
 }
 
-__global__ void __launch_bounds__(128) kPolySdf64(const PolyArgs a)
+// Whether a face under the disc may return a magnitude of at most `most` (rounded up, FP32) at p, which lies
+// `shift` from the FP64 point: the distance to the disc, less its rounding.
+__device__ __forceinline__ bool discReaches(const PolyDisc* __restrict__ disc, float px, float py, float pz, float most,
+                                            float slack)
 {
-  __shared__ float4 smem[4 * 2 * EBG_STACK_DEPTH];
-  const int         lane   = threadIdx.x & 31;
-  float4*           stk    = smem + (threadIdx.x >> 5) * (2 * EBG_STACK_DEPTH);
-  const PolyView&   m      = a.m;
-  const int64_t     numPk  = (a.n + 31) / 32;
-  const int64_t     warpId = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t     nWarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+  const float4 c = __ldg(reinterpret_cast<const float4*>(disc)), n = __ldg(reinterpret_cast<const float4*>(disc) + 1);
+  const float  dx = px - c.x, dy = py - c.y, dz = pz - c.z;
+  const float  s  = fmaf(n.x, dx, fmaf(n.y, dy, n.z * dz));
+  const float  d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+  const float  u  = fmaxf(fabsf(s) - c.w, 0.f);
+  const float  v  = fmaxf(sqrtf(fmaxf(fmaf(-s, s, d2 * 0.999999f), 0.f)) - n.w, 0.f);
+  return !(sqrtf(fmaf(u, u, v * v)) * 0.999996f - slack > most);
+}
 
-  for (int64_t pk = warpId; pk < numPk; pk += nWarps) {
-    const int64_t j     = pk * 32 + lane;
+// polyFaceSd with four lanes per face, an edge each (edges i, i + 4, ... on lane i of the four): the same
+// values, the first edge of least |d| wins.  All 32 lanes call it together; lanes without a face pass
+// N = 0 and any valid pointers.  Returns the face's value on each of its four lanes.
+__device__ __forceinline__ double polyFaceSd4(const double* __restrict__ fr, const double* __restrict__ cr, uint32_t N, P3 P)
+{
+  const uint32_t sub = threadIdx.x & 3u;
+  const uint32_t most = __reduce_max_sync(FULL, N);
+  const P3       n = ld(fr), c = ld(fr + 3);
+  const double   ax = fabs(n.x), ay = fabs(n.y), az = fabs(n.z);
+  int            ig = 0;
+  if (ay > ax) {
+    ig = 1;
+  }
+  if (az > (ig == 0 ? ax : ay)) {
+    ig = 2;
+  }
+  const double h  = dot(n, sub_(P, c));
+  const P3     q  = sub_(P, scl(h, n));
+  const double qx = ig == 0 ? q.y : q.x, qy = ig == 2 ? q.y : q.z;
+  int          cn = 0;
+  for (uint32_t i = sub; i - sub < most; i += 4) {
+    if (i < N) {
+      const double* a   = cr + 9 * size_t(i);
+      const double* b   = cr + 9 * size_t(i + 1 == N ? 0 : i + 1);
+      const double  ax2 = ig == 0 ? a[1] : a[0], ay2 = ig == 2 ? a[1] : a[2];
+      const double  bx2 = ig == 0 ? b[1] : b[0], by2 = ig == 2 ? b[1] : b[2];
+      const bool    up = (ay2 <= qy) && (by2 > qy), down = (ay2 > qy) && (by2 <= qy);
+      if (up || down) {
+        const double t = (qy - ay2) / (by2 - ay2);
+        if (qx < ax2 + t * (bx2 - ax2)) {
+          cn++;
+        }
+      }
+    }
+  }
+  cn += __shfl_xor_sync(FULL, cn, 1);
+  cn += __shfl_xor_sync(FULL, cn, 2);
+  const bool inside = (cn & 1) != 0;
+  double     best   = CUDART_INF;
+  uint32_t   bi     = 0xffffffffu;
+  if (__any_sync(FULL, !inside && N != 0u)) {
+    for (uint32_t i = sub; i - sub < most; i += 4) {
+      if (i < N && !inside) {
+        const double* a    = cr + 9 * size_t(i);
+        const double* b    = cr + 9 * size_t(i + 1 == N ? 0 : i + 1);
+        const P3      xi   = ld(a), xj = ld(b);
+        const P3      x2x1 = sub_(xj, xi);
+        const double  t    = dot(sub_(P, xi), x2x1) / dot(x2x1, x2x1);
+        // the vertex or the edge point: the same length and sign rule for all three
+        const P3      base  = t <= 0.0 ? xi : (t >= 1.0 ? xj : add(xi, scl(t, x2x1)));
+        const double* nrm   = t <= 0.0 ? a + 3 : (t >= 1.0 ? b + 3 : a + 6);
+        const P3      delta = sub_(P, base);
+        const double  d     = len(delta) * ((dot(ld(nrm), delta) > 0.0) ? 1.0 : -1.0);
+        if (fabs(d) < fabs(best)) {
+          best = d;
+          bi   = i;
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {
+      const double   od = __shfl_xor_sync(FULL, best, o);
+      const uint32_t oi = __shfl_xor_sync(FULL, bi, o);
+      if (fabs(od) < fabs(best) || (fabs(od) == fabs(best) && oi < bi)) {
+        best = od;
+        bi   = oi;
+      }
+    }
+  }
+  return inside ? h : best;
+}
+
+struct PolyMem
+{
+  float4   stk[2 * EBG_STACK_DEPTH];
+  double   px[32], py[32], pz[32];
+  double   res[8];
+  uint16_t pair[32 * EBG_MAX_LEAF]; // (face within the leaf, lane)
+};
+
+constexpr int POLY_WARPS  = 4;
+constexpr int POLY_BLOCKS = 8; // per SM
+
+// Bound by the latency of its FP64 evaluations (crossing number, divisions and square roots of every
+// edge: thousands of cycles), so they are made only where a face's disc reaches the lane's minimum,
+// four threads for each (lane, face) pair.  B200, 200,003 points on 24,576 quads: 25.0 -> 2.8 ms.
+__global__ void __launch_bounds__(32 * POLY_WARPS) kPolySdf64(const PolyArgs a)
+{
+  extern __shared__ float4 polySmem[];
+  PolyMem&        w     = reinterpret_cast<PolyMem*>(polySmem)[threadIdx.x >> 5];
+  float4*         stk   = w.stk;
+  const int       lane  = threadIdx.x & 31;
+  const unsigned  lt    = (1u << lane) - 1u;
+  const PolyView& m     = a.m;
+  const int64_t   numPk = (a.n + 31) / 32;
+
+  while (true) {
+    unsigned long long pk = 0;
+    if (lane == 0) {
+      pk = atomicAdd(a.work, 1ull);
+    }
+    pk = __shfl_sync(FULL, pk, 0);
+    if (int64_t(pk) >= numPk) {
+      break;
+    }
+    const int64_t j     = int64_t(pk) * 32 + lane;
     const bool    valid = j < a.n;
     const int64_t jj    = valid ? j : a.n - 1;
     const int64_t id    = a.order ? int64_t(a.order[jj]) : jj;
@@ -189,12 +320,17 @@ __global__ void __launch_bounds__(128) kPolySdf64(const PolyArgs a)
     }
     const double ex = P.x - double(px), ey = P.y - double(py), ez = P.z - double(pz);
     const float  shift = float(sqrt(ex * ex + ey * ey + ez * ez)) * 1.0001f;
+    const float  slack = m.slack + shift;
     float        bound = __int_as_float(0x7f800000);
+    float        most  = __int_as_float(0x7f800000); // |best| rounded up
     double       best  = CUDART_INF;
     int          bt    = -1;
     uint32_t     iters = 0;
 
     int sp = 1;
+    w.px[lane] = P.x;
+    w.py[lane] = P.y;
+    w.pz[lane] = P.z;
     if (lane == 0) {
       stk[0] = make_float4(m.rootLo[0], m.rootLo[1], m.rootLo[2], __uint_as_float(m.rootRef));
       stk[1] = make_float4(m.rootHi[0], m.rootHi[1], m.rootHi[2], __uint_as_float(m.rootCount));
@@ -214,61 +350,93 @@ __global__ void __launch_bounds__(128) kPolySdf64(const PolyArgs a)
       }
       const uint32_t ref = __float_as_uint(A.w), cntw = __float_as_uint(B.w);
       if (ref & EBG_LEAF_BIT) {
-        const uint32_t f0 = ref & ~EBG_LEAF_BIT, cnt = cntw & EBG_COUNT_MASK;
-        if (need) {
-          for (uint32_t f = f0; f < f0 + cnt; f++) {
-            const double d = polyFaceSd(m, f, P);
-            // strict < as the reference's leaf loop, ties to the lower leaf position
-            if (fabs(d) < fabs(best) || (fabs(d) == fabs(best) && int(f) < bt)) {
-              best               = d;
-              bt                 = int(f);
-              const float rb     = (float(fabs(d)) + shift) * 1.000001f + 1e-30f;
-              bound              = fminf(bound, rb * rb);
-            }
+        const uint32_t f0 = ref & ~EBG_LEAF_BIT;
+        const int      cnt = int(cntw & EBG_COUNT_MASK);
+        // the (lane, face) pairs to evaluate, face by face
+        int pairs = 0;
+        for (int f = 0; f < cnt; f++) {
+          const bool     ev = need && discReaches(m.faceDisc + f0 + f, px, py, pz, most, slack);
+          const unsigned mk = __ballot_sync(FULL, ev);
+          if (ev) {
+            w.pair[pairs + __popc(mk & lt)] = uint16_t(f << 5 | lane);
           }
-        }
-      }
-      else {
-        const EbgNode4& nd = m.nodes[ref];
-        int             o[4], np = 0;
-        float           key[4];
-        for (int k = 0; k < 4; k++) {
-          const float dk = boxDist2(nd.lox[k], nd.loy[k], nd.loz[k], nd.hix[k], nd.hiy[k], nd.hiz[k], px, py, pz);
-          // empty slot: child 0 and count 0 (node 0 is the root and never a child)
-          if (__any_sync(FULL, valid && dk <= bound) && (nd.child[k] | nd.count[k]) != 0u) {
-            o[np]   = k;
-            key[np] = dk;
-            np++;
-          }
-        }
-        // nearest first by the packet's smallest distance to each child
-        for (int i = 0; i < np; i++) {
-          key[i] = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(valid ? key[i] : FLT_MAX)));
-        }
-        for (int i = 1; i < np; i++) {
-          for (int q = i; q > 0 && key[q - 1] < key[q]; q--) {
-            const float tk = key[q];
-            key[q]         = key[q - 1];
-            key[q - 1]     = tk;
-            const int to   = o[q];
-            o[q]           = o[q - 1];
-            o[q - 1]       = to;
-          }
-        }
-        if (sp + np > EBG_STACK_DEPTH) {
-          err |= ST_STACK;
-          break;
-        }
-        for (int i = 0; i < np; i++) {
-          const int k = o[i];
-          if (lane == 0) {
-            stk[2 * sp]     = make_float4(nd.lox[k], nd.loy[k], nd.loz[k], __uint_as_float(nd.child[k]));
-            stk[2 * sp + 1] = make_float4(nd.hix[k], nd.hiy[k], nd.hiz[k], __uint_as_float(nd.count[k]));
-          }
-          sp++;
+          pairs += __popc(mk);
         }
         __syncwarp();
+        for (int p = 0; p < pairs; p += 8) {
+          const int      i  = p + (lane >> 2);
+          const uint32_t v  = w.pair[i < pairs ? i : p], q = v & 31u;
+          const uint2    fc = m.face[f0 + (v >> 5)];
+          const double   d  = polyFaceSd4(m.faceRec + 6 * size_t(f0 + (v >> 5)), m.corner + 9 * size_t(fc.x),
+                                          i < pairs ? fc.y : 0u, P3{w.px[q], w.py[q], w.pz[q]});
+          if ((lane & 3) == 0) {
+            w.res[lane >> 2] = d;
+          }
+          __syncwarp();
+          const int n = pairs - p < 8 ? pairs - p : 8;
+          for (int k = 0; k < n; k++) {
+            const uint32_t u = w.pair[p + k];
+            if (int(u & 31u) == lane) {
+              const double d1 = w.res[k];
+              const int    f  = int(f0 + (u >> 5));
+              // strict < as the reference's leaf loop, ties to the lower leaf position
+              if (fabs(d1) < fabs(best) || (fabs(d1) == fabs(best) && f < bt)) {
+                best           = d1;
+                bt             = f;
+                const float rb = (float(fabs(d1)) + shift) * 1.000001f + 1e-30f;
+                bound          = fminf(bound, rb * rb);
+                most           = float(fabs(d1)) * 1.000001f;
+              }
+            }
+          }
+          __syncwarp();
+        }
+        continue;
       }
+      // lanes whose minimum a face below may lower: the others' evaluations would change nothing (the
+      // node's loads are issued with its disc's)
+      const EbgNode4& nd    = m.nodes[ref];
+      const float4*   nv    = reinterpret_cast<const float4*>(&nd);
+      const float4    lx = __ldg(nv), ly = __ldg(nv + 1), lz = __ldg(nv + 2);
+      const float4    hx = __ldg(nv + 3), hy = __ldg(nv + 4), hz = __ldg(nv + 5);
+      const bool      reach = need && discReaches(m.nodeDisc + ref, px, py, pz, most, slack);
+      if (!__any_sync(FULL, reach)) {
+        continue;
+      }
+      const float clx[4] = {lx.x, lx.y, lx.z, lx.w}, cly[4] = {ly.x, ly.y, ly.z, ly.w}, clz[4] = {lz.x, lz.y, lz.z, lz.w};
+      const float chx[4] = {hx.x, hx.y, hx.z, hx.w}, chy[4] = {hy.x, hy.y, hy.z, hy.w}, chz[4] = {hz.x, hz.y, hz.z, hz.w};
+      float       key[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const float dk = boxDist2(clx[k], cly[k], clz[k], chx[k], chy[k], chz[k], px, py, pz);
+        // empty slot: child 0 and count 0 (node 0 is the root and never a child)
+        const bool  nk = __any_sync(FULL, reach && dk <= bound &&
+                                           discReaches(m.slotDisc + 4 * size_t(ref) + k, px, py, pz, most, slack)) &&
+                        (nd.child[k] | nd.count[k]) != 0u;
+        // nearest first by the packet's smallest distance to each child
+        key[k] = nk ? __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(valid ? dk : FLT_MAX))) : -1.f;
+      }
+      const int np = int(key[0] >= 0.f) + int(key[1] >= 0.f) + int(key[2] >= 0.f) + int(key[3] >= 0.f);
+      if (sp + np > EBG_STACK_DEPTH) {
+        err |= ST_STACK;
+        break;
+      }
+      // lane k (< 4) writes child k into its slot, farther children deeper (ties by slot index)
+      if (lane < 4) {
+        const float kk = lane == 0 ? key[0] : (lane == 1 ? key[1] : (lane == 2 ? key[2] : key[3]));
+        if (kk >= 0.f) {
+          int rank = 0;
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            rank += int(key[i] >= 0.f && (key[i] > kk || (key[i] == kk && i < lane)));
+          }
+          float4* e = stk + 2 * (sp + rank);
+          e[0]      = make_float4(nd.lox[lane], nd.loy[lane], nd.loz[lane], __uint_as_float(nd.child[lane]));
+          e[1]      = make_float4(nd.hix[lane], nd.hiy[lane], nd.hiz[lane], __uint_as_float(nd.count[lane]));
+        }
+      }
+      sp += np;
+      __syncwarp();
     }
     err = __reduce_or_sync(FULL, valid ? err : 0);
     if (err && lane == 0) {
@@ -280,6 +448,7 @@ __global__ void __launch_bounds__(128) kPolySdf64(const PolyArgs a)
         a.outFace[id] = bt >= 0 ? m.faceId[bt] : -1;
       }
     }
+    __syncwarp();
   }
 }
 
@@ -331,6 +500,9 @@ struct ebg_polymesh
   double*        dFaceRec   = nullptr;
   double*        dCorner    = nullptr;
   int32_t*       dFaceId    = nullptr;
+  ebg::PolyDisc* dFaceDisc  = nullptr;
+  ebg::PolyDisc* dSlotDisc  = nullptr;
+  ebg::PolyDisc* dNodeDisc  = nullptr;
   int*           dStatus    = nullptr;
   float          mortonLo[3]    = {0, 0, 0};
   float          mortonScale[3] = {1, 1, 1};
@@ -339,6 +511,33 @@ struct ebg_polymesh
 using namespace ebg;
 
 namespace {
+
+// The disc of a set of points (three doubles each): centre their mean, normal n, padded by `pad`.
+PolyDisc discOf(const std::vector<double>& x, const double* n, double pad)
+{
+  const size_t k = x.size() / 3;
+  double       c[3] = {0, 0, 0};
+  for (size_t i = 0; i < k; i++) {
+    for (int a = 0; a < 3; a++) {
+      c[a] += x[3 * i + a] / double(k);
+    }
+  }
+  const double l = std::sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+  PolyDisc     d;
+  d.cx = float(c[0]), d.cy = float(c[1]), d.cz = float(c[2]);
+  d.nx = l > 0 ? float(n[0] / l) : 0.f, d.ny = l > 0 ? float(n[1] / l) : 0.f, d.nz = l > 0 ? float(n[2] / l) : 1.f;
+  double h = 0, R = 0;
+  for (size_t i = 0; i < k; i++) {
+    const double dx = x[3 * i] - d.cx, dy = x[3 * i + 1] - d.cy, dz = x[3 * i + 2] - d.cz;
+    const double s  = dx * d.nx + dy * d.ny + dz * d.nz;
+    const double tx = dx - s * d.nx, ty = dy - s * d.ny, tz = dz - s * d.nz;
+    h               = std::max(h, std::fabs(s));
+    R               = std::max(R, std::sqrt(tx * tx + ty * ty + tz * tz));
+  }
+  d.h = float(h * 1.000001 + pad);
+  d.R = float(R * 1.000001 + pad);
+  return d;
+}
 
 ebg_status buildPoly(const double* V, int64_t nv, const int64_t* off, const int32_t* idx, int64_t nf,
                      const ebg_build_opts* opts, ebg_polymesh** out)
@@ -441,6 +640,57 @@ ebg_status buildPoly(const double* V, int64_t nv, const int64_t* off, const int3
       }
     }
   }
+  // the discs of faces, leaves and nodes over each face's corners and, moved along the axis of its
+  // largest normal component, their places in the plane through its centroid
+  double scale = 0;
+  for (int a = 0; a < 3; a++) {
+    scale = std::max(scale, std::max(bvh.hi[a] - bvh.lo[a], std::max(std::fabs(bvh.lo[a]), std::fabs(bvh.hi[a]))));
+  }
+  const double pad = 2e-6 * scale;
+  auto         addFace = [&](int64_t p, std::vector<double>& x, double* n) {
+    const uint2   fc = face[p];
+    const double* fr = &faceRec[6 * p];
+    int           ig = std::fabs(fr[1]) > std::fabs(fr[0]) ? 1 : 0;
+    ig               = std::fabs(fr[2]) > std::fabs(fr[ig]) ? 2 : ig;
+    for (uint32_t k = fc.x; k < fc.x + fc.y; k++) {
+      const double* c = &corner[9 * size_t(k)];
+      const double  s = (c[0] - fr[3]) * fr[0] + (c[1] - fr[4]) * fr[1] + (c[2] - fr[5]) * fr[2];
+      double        q[3] = {c[0], c[1], c[2]};
+      q[ig] -= s / fr[ig];
+      x.insert(x.end(), {c[0], c[1], c[2], q[0], q[1], q[2]});
+    }
+    for (int a = 0; a < 3; a++) {
+      n[a] += fr[a];
+    }
+  };
+  auto discOfRange = [&](int64_t b, int64_t e) {
+    std::vector<double> x;
+    double              n[3] = {0, 0, 0};
+    for (int64_t p = b; p < e; p++) {
+      addFace(p, x, n);
+    }
+    return discOf(x, n, pad);
+  };
+  std::vector<PolyDisc> faceDisc(nf), leafDisc(bvh.leafFirst.size()), nodeDisc(bvh.nodes.size()),
+    slotDisc(4 * bvh.nodes.size());
+#pragma omp parallel for schedule(static)
+  for (int64_t p = 0; p < nf; p++) {
+    faceDisc[p] = discOfRange(p, p + 1);
+  }
+#pragma omp parallel for schedule(static)
+  for (int64_t i = 0; i < int64_t(leafDisc.size()); i++) {
+    leafDisc[i] = discOfRange(bvh.leafFirst[i], int64_t(bvh.leafFirst[i]) + bvh.leafCount[i]);
+  }
+#pragma omp parallel for schedule(dynamic, 16)
+  for (int64_t i = 0; i < int64_t(nodeDisc.size()); i++) {
+    nodeDisc[i] = discOfRange(bvh.nodeFirst[i], bvh.nodeEnd[i]);
+  }
+  for (size_t i = 0; i < slotDisc.size(); i++) {
+    const uint32_t child = bvh.nodes[i / 4].child[i % 4], cw = bvh.nodes[i / 4].count[i % 4];
+    if ((child | cw) != 0u) {
+      slotDisc[i] = (child & EBG_LEAF_BIT) ? leafDisc[cw >> EBG_COUNT_BITS] : nodeDisc[child];
+    }
+  }
   auto* m   = new ebg_polymesh;
   m->device = device;
   cudaDeviceGetAttribute(&m->numSms, cudaDevAttrMultiProcessorCount, device);
@@ -455,6 +705,9 @@ ebg_status buildPoly(const double* V, int64_t nv, const int64_t* off, const int3
       !up((void**)&m->dFaceRec, faceRec.data(), faceRec.size() * sizeof(double)) ||
       !up((void**)&m->dCorner, corner.data(), corner.size() * sizeof(double)) ||
       !up((void**)&m->dFaceId, faceId.data(), faceId.size() * sizeof(int32_t)) ||
+      !up((void**)&m->dFaceDisc, faceDisc.data(), faceDisc.size() * sizeof(PolyDisc)) ||
+      !up((void**)&m->dSlotDisc, slotDisc.data(), slotDisc.size() * sizeof(PolyDisc)) ||
+      !up((void**)&m->dNodeDisc, nodeDisc.data(), nodeDisc.size() * sizeof(PolyDisc)) ||
       cudaMalloc((void**)&m->dStatus, sizeof(int)) != cudaSuccess ||
       cudaMemset(m->dStatus, 0, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
@@ -462,6 +715,10 @@ ebg_status buildPoly(const double* V, int64_t nv, const int64_t* off, const int3
     return setError(EBG_ERR_NO_MEMORY, "device allocation or upload failed for the polygon mesh");
   }
   PolyView& v  = m->view;
+  v.faceDisc   = m->dFaceDisc;
+  v.nodeDisc   = m->dNodeDisc;
+  v.slotDisc   = m->dSlotDisc;
+  v.slack      = float(2e-6 * scale) + 1e-30f;
   v.nodes      = m->dNodes;
   v.face       = m->dFace;
   v.faceRec    = m->dFaceRec;
@@ -490,7 +747,8 @@ ebg_status buildPoly(const double* V, int64_t nv, const int64_t* off, const int3
   m->info.depth         = bvh.depth;
   m->info.leaf_size     = leafSize;
   m->info.diagonal      = std::sqrt(d2);
-  m->info.device_bytes  = int64_t(bvh.nodes.size() * sizeof(EbgNode4) + size_t(nf) * (8 + 48 + 4) + size_t(nc) * 72);
+  m->info.device_bytes  = int64_t(bvh.nodes.size() * sizeof(EbgNode4) + (nodeDisc.size() + slotDisc.size()) * sizeof(PolyDisc) +
+                                     size_t(nf) * (8 + 48 + 4 + sizeof(PolyDisc)) + size_t(nc) * 72);
   *out                  = m;
   return EBG_OK;
 }
@@ -529,8 +787,9 @@ ebg_status polyQuery(const ebg_polymesh* m, const double* pts, int64_t n, double
   auto*  ord  = static_cast<uint32_t*>(get(4 * size_t(n)));
   size_t tb   = 0;
   cub::DeviceRadixSort::SortPairs(nullptr, tb, kin, kout, iin, ord, int(n), 0, 30, s);
-  void* tmp = get(tb);
-  if (!p32 || !kin || !kout || !iin || !ord || !tmp) {
+  void* tmp  = get(tb);
+  auto* work = static_cast<unsigned long long*>(get(sizeof(unsigned long long)));
+  if (!work || !p32 || !kin || !kout || !iin || !ord || !tmp) {
     for (void* p : ws) {
       cudaFreeAsync(p, s);
     }
@@ -541,7 +800,11 @@ ebg_status polyQuery(const ebg_polymesh* m, const double* pts, int64_t n, double
   cub::DeviceRadixSort::SortPairs(tmp, tb, kin, kout, iin, ord, int(n), 0, 30, s);
   a.pts32 = p32;
   a.order = ord;
-  kPolySdf64<<<unsigned(m->numSms * 8), 128, 0, s>>>(a);
+  a.work = work;
+  cudaMemsetAsync(work, 0, sizeof(unsigned long long), s);
+  const int64_t need = (n + 32 * POLY_WARPS - 1) / (32 * POLY_WARPS);
+  kPolySdf64<<<unsigned(std::min<int64_t>(need, int64_t(m->numSms) * POLY_BLOCKS)), 32 * POLY_WARPS,
+               POLY_WARPS * sizeof(PolyMem), s>>>(a);
   const cudaError_t e = cudaGetLastError();
   for (void* p : ws) {
     cudaFreeAsync(p, s);
@@ -705,6 +968,9 @@ ebg_status ebg_polymesh_destroy(ebg_polymesh* m)
   DeviceGuard guard;
   cudaSetDevice(m->device);
   cudaFree(m->dNodes);
+  cudaFree(m->dFaceDisc);
+  cudaFree(m->dSlotDisc);
+  cudaFree(m->dNodeDisc);
   cudaFree(m->dFace);
   cudaFree(m->dFaceRec);
   cudaFree(m->dCorner);
