@@ -16,8 +16,8 @@
 //   every box spatially compact.  (Fixed runs of L points grouped four at a time in Morton order --
 //   the balanced tree kept as the fallback for clouds whose radix tree is too deep for the
 //   traversal stack -- make long, thin boxes across those jumps that every nearby query opens.)
-// Query: Morton-sorted queries, one per lane, each walking the tree with its own stack and keeping
-// its k best (d2, index) pairs sorted in registers.  Order is lexicographic on
+// Query: Morton-sorted queries, one per lane or per four lanes, walking the tree with their own stack and
+// keeping the k best (d2, index) pairs sorted in registers.  Order is lexicographic on
 // (d2, index), so equal distances resolve to the lowest index, and d2 is the reference's float
 // arithmetic (PointSoAImplem.hpp:214-230): dx = q - p, d2 = (dx*dx + dy*dy) + dz*dz, each operation
 // rounded separately (no fused multiply-add).  Box distances use the same association, which makes
@@ -356,17 +356,17 @@ __device__ __forceinline__ bool lexLess(float da, uint32_t ia, float db, uint32_
   return da < db || (da == db && ia < ib);
 }
 
-// One query per lane.  Each lane walks the tree on its own, nearest child first, with a private
-// stack of (ref, count, box distance) entries (in local memory: at most 3 x depth + 1 of them); a
-// popped entry whose distance exceeds the lane's k-th best is skipped.  Warps take packets of 32
-// consecutive (Morton-ordered) queries from the work counter, so a warp's lanes walk nearby paths
-// and mostly read the same node and point lines.  (A warp walking one shared stack for its 32
-// queries opens every node any lane needs -- about four times what each lane needs on the k-NN
-// workloads -- and costs more than the divergence of separate walks.)
+// One query per lane (k <= 8, many queries).  Each lane walks the tree nearest child first with its own stack
+// of (ref, count, box distance) entries (in local memory: at most 3 x depth + 1 of them); a popped entry
+// whose distance exceeds the lane's k-th best is skipped.  Warps take packets of 32 consecutive
+// (Morton-ordered) queries from the work counter, so a warp's lanes walk nearby paths and mostly read
+// the same node and point lines.  (A warp walking one shared stack for its 32 queries opens every node
+// any lane needs -- about four times what each lane needs on the k-NN workloads -- and costs more than
+// the divergence of separate walks.)
 // SELF: the queries are cloud points (self_pos), each excluded from its own neighbours
 // (nearestNeighbors / allNearestNeighbors, PointCloudBVHImplem.hpp:455-507).
 template <int K, bool SELF>
-__global__ void __launch_bounds__(128, (K <= 2 ? 16 : (K <= 8 ? 10 : 1))) kCloudKnn(const CloudQueryArgs a)
+__global__ void __launch_bounds__(128, (K <= 2 ? 16 : 10)) kCloudKnn(const CloudQueryArgs a)
 {
   const int           lane       = threadIdx.x & 31;
   const EbgCloudView& c          = a.cloud;
@@ -514,8 +514,231 @@ __global__ void __launch_bounds__(128, (K <= 2 ? 16 : (K <= 8 ? 10 : 1))) kCloud
   }
 }
 
+// Four lanes per query, eight queries per warp.  A group's lanes take the four children of a node, then
+// the points of a leaf, four at a time; its stack is in shared memory.
+// The k best sit sorted across the group, K / 4 on each lane.  A group that has finished its query
+// takes the next of the warp's run of consecutive (Morton-ordered) queries once REFILL groups wait.
+//
+// With a query per lane 7 of 32 lanes are active (k = 8, clustered cloud; 10 at k = 1): lanes at nodes wait
+// for lanes at leaves and for one lane's insertion, which grows with k.  But those lanes read the same
+// lines at the same time; keeping more of them active by serving nodes and leaves by majority and
+// refilling finished lanes made the walk 1.4 to 2 times slower on 16 M points, a loop that descends to a
+// leaf first 1.3 times.  So short lists of many queries keep it (launchCloudKnn).
+constexpr int KNN_WARPS  = 4;
+constexpr int KNN_GROUPS = 8;
+constexpr int KNN_REFILL = 3;
+
 template <int K, bool SELF>
-cudaError_t launchKnnKS(const CloudQueryArgs& a, int numSms, cudaStream_t s)
+__global__ void __launch_bounds__(32 * KNN_WARPS, (K <= 8 ? 10 : (K <= 16 ? 8 : 6)))
+  kCloudKnnGroups(const __grid_constant__ CloudQueryArgs a, int cap, int run)
+{
+  constexpr int      E = K / 4; // list entries per lane
+  extern __shared__ uint32_t knnSmem[];
+  const int           lane = threadIdx.x & 31, sub = lane & 3, grp = lane >> 2, base = lane & 28;
+  const EbgCloudView& c    = a.cloud;
+  const float         inf  = __int_as_float(0x7f800000);
+  // entry e of group g at [e * KNN_GROUPS + g]
+  uint32_t* sRef = knnSmem + (threadIdx.x >> 5) * (3 * KNN_GROUPS * cap) + grp;
+  uint32_t* sCnt = sRef + KNN_GROUPS * cap;
+  float*    sKey = reinterpret_cast<float*>(sCnt + KNN_GROUPS * cap);
+  const int pad  = K - a.k;
+
+  int64_t  next = 0, end = 0;      // the warp's run
+  bool     more = true;            // the work counter may have another
+  bool     have = false;           // the group has a query
+  uint32_t id = 0, self = 0xffffffffu, iters = 0;
+  float    px = 0.f, py = 0.f, pz = 0.f;
+  float    kd[E];
+  uint32_t ki[E];
+  float    bd = inf;               // the k-th best
+  uint32_t bi = 0xffffffffu;
+  int      sp = 0;
+#pragma unroll
+  for (int j = 0; j < E; j++) {
+    kd[j] = inf;
+    ki[j] = 0xffffffffu;
+  }
+  while (true) {
+    // finished groups write their results and take new queries
+    const unsigned idle = __ballot_sync(FULL, sub == 0 && sp == 0);
+    if (__popc(idle) >= (more || next < end ? KNN_REFILL : KNN_GROUPS)) {
+      if (have && sp == 0) {
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+          const int r = sub * E + j - pad;
+          if (r >= 0) {
+            const bool   found = ki[j] != 0xffffffffu;
+            const size_t o     = size_t(id) * a.k + r;
+            a.out_idx[o]       = found ? int32_t(ki[j]) : -1;
+            a.out_d2[o]        = found ? kd[j] : inf;
+          }
+        }
+        have = false;
+      }
+      if (next >= end && more) {
+        unsigned long long w = 0;
+        if (lane == 0) {
+          w = atomicAdd(a.work, (unsigned long long)run);
+        }
+        next = int64_t(__shfl_sync(FULL, w, 0));
+        end  = next + run < a.n ? next + run : a.n;
+        more = end < a.n;
+      }
+      const int64_t pos = next + __popc(idle & ((1u << base) - 1u));
+      if (sp == 0 && pos < end) {
+        self = 0xffffffffu;
+        if (SELF) {
+          const uint32_t lp = a.self_pos ? __ldg(a.self_pos + pos) : uint32_t(pos);
+          const float4   qp = __ldg(c.points + lp);
+          px                = qp.x;
+          py                = qp.y;
+          pz                = qp.z;
+          self              = __float_as_uint(qp.w);
+          id                = a.order ? __ldg(a.order + pos) : self;
+        }
+        else {
+          id = a.order ? __ldg(a.order + pos) : uint32_t(pos);
+          px = __ldg(a.queries + 3 * size_t(id));
+          py = __ldg(a.queries + 3 * size_t(id) + 1);
+          pz = __ldg(a.queries + 3 * size_t(id) + 2);
+        }
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+          const bool p = sub * E + j < pad; // never moves
+          kd[j]        = p ? -1.f : inf;
+          ki[j]        = p ? 0u : 0xffffffffu;
+        }
+        bd    = inf;
+        bi    = 0xffffffffu;
+        iters = 0;
+        have  = true;
+        sp    = 1;
+        if (sub == 0) {
+          sRef[0] = c.root_ref;
+          sCnt[0] = c.root_count;
+          sKey[0] = boxD2exact(c.root_lo[0], c.root_lo[1], c.root_lo[2], c.root_hi[0], c.root_hi[1], c.root_hi[2], px, py, pz);
+        }
+      }
+      next += __popc(idle);
+      next = next < end ? next : end;
+      __syncwarp();
+      if (!__any_sync(FULL, sp > 0)) {
+        if (next >= end && !more) {
+          break;
+        }
+        continue;
+      }
+    }
+    // down to the topmost entry within the k-th best, four at a time
+    {
+      const int      i  = sp - 1 - sub;
+      const unsigned ok = (__ballot_sync(FULL, i >= 0 && !(sKey[KNN_GROUPS * (i >= 0 ? i : 0)] > bd)) >> base) & 15u;
+      sp                = ok != 0u ? sp - (__ffs(int(ok)) - 1) : (sp > 4 ? sp - 4 : 0);
+    }
+    if (sp > 0 && ++iters > MAX_ITERS) {
+      if (sub == 0) {
+        atomicOr(a.status, ST_ITERS);
+      }
+      sp = 0;
+    }
+    const int      t   = KNN_GROUPS * (sp > 0 ? sp - 1 : 0);
+    const bool     top = sp > 0 && !(sKey[t] > bd);
+    const uint32_t ref = sRef[t];
+    const bool     node = top && !(ref & EBG_LEAF_BIT);
+    if (__any_sync(FULL, node)) {
+      float    d = -1.f; // an empty slot or a child beyond the bound
+      uint32_t ch = 0, cn = 0;
+      if (node) {
+        const EbgNode4* nd = c.nodes + ref;
+        const float lx = __ldg(nd->lox + sub), ly = __ldg(nd->loy + sub), lz = __ldg(nd->loz + sub);
+        const float hx = __ldg(nd->hix + sub), hy = __ldg(nd->hiy + sub), hz = __ldg(nd->hiz + sub);
+        ch             = __ldg(nd->child + sub);
+        cn             = __ldg(nd->count + sub);
+        const float dd = boxD2exact(lx, ly, lz, hx, hy, hz, px, py, pz);
+        d                = dd <= bd && (ch | cn) != 0u ? dd : -1.f;
+      }
+      // farthest first onto the stack, so the nearest is on top (ties by slot)
+      int rank = 0, all = 0;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const float o = __shfl_sync(FULL, d, i, 4);
+        rank += int(o > d || (o == d && i < sub));
+        all += int(o >= 0.f);
+      }
+      sp -= node ? 1 : 0;
+      __syncwarp(); // the top is read before it is overwritten
+      if (node && sp + all > cap) { // never: the builder's depth bounds the stack
+        if (sub == 0) {
+          atomicOr(a.status, ST_STACK);
+        }
+        sp  = 0;
+        all = 0;
+        d   = -1.f;
+      }
+      if (d >= 0.f) {
+        const int e = KNN_GROUPS * (sp + rank);
+        sRef[e]     = ch;
+        sCnt[e]     = cn;
+        sKey[e]     = d;
+      }
+      sp += node ? all : 0;
+      __syncwarp();
+    }
+    // the leaf on top
+    const int      u  = KNN_GROUPS * (sp > 0 ? sp - 1 : 0);
+    const uint32_t lr = sRef[u];
+    const bool     leaf = sp > 0 && (lr & EBG_LEAF_BIT) && !(sKey[u] > bd);
+    if (__any_sync(FULL, leaf)) {
+      const uint32_t p0  = lr & ~EBG_LEAF_BIT;
+      const uint32_t cnt = leaf ? sCnt[u] : 0u;
+      sp -= leaf ? 1 : 0;
+      __syncwarp(); // read before it is overwritten
+      const uint32_t most = __reduce_max_sync(FULL, cnt);
+      for (uint32_t s = 0; s < most; s += 4) {
+        float    dd = inf;
+        uint32_t ii = 0xffffffffu;
+        if (s + sub < cnt) {
+          const float4 q = __ldg(c.points + p0 + s + sub);
+          dd             = d2exact(px - q.x, py - q.y, pz - q.z);
+          ii             = __float_as_uint(q.w);
+        }
+        bool cand = s + sub < cnt && (!SELF || ii != self) && lexLess(dd, ii, bd, bi);
+        // one candidate per group at a time into the sorted list
+        unsigned mk = (__ballot_sync(FULL, cand) >> base) & 15u;
+        while (__any_sync(FULL, mk != 0u)) {
+          const int      from = mk != 0u ? __ffs(int(mk)) - 1 : 0;
+          const float    cd = __shfl_sync(FULL, dd, from, 4);
+          const uint32_t ci = __shfl_sync(FULL, ii, from, 4);
+          const float    ld = __shfl_up_sync(FULL, kd[E - 1], 1, 4);
+          const uint32_t li = __shfl_up_sync(FULL, ki[E - 1], 1, 4);
+          if (mk != 0u && lexLess(cd, ci, kd[E - 1], ki[E - 1])) {
+            // this lane's part shifts: in comes the candidate, or what the lane before pushes out
+            const bool push = sub > 0 && lexLess(cd, ci, ld, li);
+            kd[E - 1]       = push ? ld : cd;
+            ki[E - 1]       = push ? li : ci;
+#pragma unroll
+            for (int j = E - 1; j > 0; j--) {
+              if (lexLess(kd[j], ki[j], kd[j - 1], ki[j - 1])) {
+                const float    td = kd[j];
+                const uint32_t ti = ki[j];
+                kd[j]             = kd[j - 1];
+                ki[j]             = ki[j - 1];
+                kd[j - 1]         = td;
+                ki[j - 1]         = ti;
+              }
+            }
+          }
+          bd = __shfl_sync(FULL, kd[E - 1], 3, 4);
+          bi = __shfl_sync(FULL, ki[E - 1], 3, 4);
+          mk &= mk - 1u;
+        }
+      }
+    }
+  }
+}
+
+template <int K, bool SELF>
+cudaError_t launchLanesKS(const CloudQueryArgs& a, int numSms, cudaStream_t s)
 {
   int perSm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kCloudKnn<K, SELF>, 128, 0);
@@ -523,15 +746,50 @@ cudaError_t launchKnnKS(const CloudQueryArgs& a, int numSms, cudaStream_t s)
   const int64_t need = ((int64_t(a.n) + 31) / 32 + 3) / 4;
   int64_t       grid = int64_t(numSms) * perSm;
   grid               = grid < need ? grid : need;
-  grid               = grid < 1 ? 1 : grid;
-  kCloudKnn<K, SELF><<<unsigned(grid), 128, 0, s>>>(a);
+  kCloudKnn<K, SELF><<<unsigned(grid < 1 ? 1 : grid), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 template <int K>
-cudaError_t launchKnnK(const CloudQueryArgs& a, bool self, int numSms, cudaStream_t s)
+cudaError_t launchLanesK(const CloudQueryArgs& a, bool self, int numSms, cudaStream_t s)
 {
-  return self ? launchKnnKS<K, true>(a, numSms, s) : launchKnnKS<K, false>(a, numSms, s);
+  return self ? launchLanesKS<K, true>(a, numSms, s) : launchLanesKS<K, false>(a, numSms, s);
+}
+
+template <int K, bool SELF>
+cudaError_t launchGroupsKS(const CloudQueryArgs& a, int depth, int numSms, cudaStream_t s)
+{
+  // 3 x depth + 1 entries
+  const int    cap  = 3 * depth + 1;
+  const size_t smem = size_t(KNN_WARPS) * 3 * KNN_GROUPS * cap * sizeof(uint32_t);
+  int          perSm = 0;
+  cudaError_t  e     = cudaSuccess;
+  if (smem > 48 * 1024) {
+    e = cudaFuncSetAttribute(kCloudKnnGroups<K, SELF>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  }
+  if (e == cudaSuccess) {
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kCloudKnnGroups<K, SELF>, 32 * KNN_WARPS, smem);
+  }
+  if (e != cudaSuccess) {
+    return e;
+  }
+  perSm = perSm < 1 ? 1 : perSm;
+  // runs of up to 8 queries, so that the warps of the GPU are in one region of the cloud (16: 4 % slower at
+  // k = 32, 64: 22 %); shorter ones where that leaves warps without work
+  const int64_t warps = int64_t(numSms) * perSm * KNN_WARPS;
+  int64_t       run   = a.n / (2 * warps);
+  run                 = run < 1 ? 1 : (run > 8 ? 8 : run);
+  const int64_t need  = (a.n + run * KNN_WARPS - 1) / (run * KNN_WARPS);
+  int64_t       grid  = int64_t(numSms) * perSm;
+  grid                = grid < need ? grid : need;
+  kCloudKnnGroups<K, SELF><<<unsigned(grid), 32 * KNN_WARPS, smem, s>>>(a, cap, int(run));
+  return cudaGetLastError();
+}
+
+template <int K>
+cudaError_t launchGroupsK(const CloudQueryArgs& a, bool self, int depth, int numSms, cudaStream_t s)
+{
+  return self ? launchGroupsKS<K, true>(a, depth, numSms, s) : launchGroupsKS<K, false>(a, depth, numSms, s);
 }
 
 // inv[cloud index] = leaf position
@@ -755,22 +1013,28 @@ cudaError_t buildCloud(const float* points, int64_t n, int L, bool balanced, flo
   return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
 }
 
-cudaError_t launchCloudKnn(const CloudQueryArgs& a, int kTemplate, int numSms, cudaStream_t s, bool self)
+cudaError_t launchCloudKnn(const CloudQueryArgs& a, int depth, int numSms, cudaStream_t s, bool self)
 {
-  switch (kTemplate) {
-  case 1:
-    return launchKnnK<1>(a, self, numSms, s);
-  case 2:
-    return launchKnnK<2>(a, self, numSms, s);
-  case 4:
-    return launchKnnK<4>(a, self, numSms, s);
-  case 8:
-    return launchKnnK<8>(a, self, numSms, s);
-  case 16:
-    return launchKnnK<16>(a, self, numSms, s);
-  default:
-    return launchKnnK<32>(a, self, numSms, s);
+  // A query per lane where its neighbours share the lines it reads and its list is short; four lanes per
+  // query otherwise (4 M clustered queries of 16 M points, lanes against groups: k = 1 2.0 / 3.3 ms, k = 8
+  // 5.2 / 7.4; 1 M uniform queries of 4 M points, k = 16: 4.2 / 2.9; 262,144 of 1 M, k = 32: 4.9 / 2.1; 16,000
+  // queries of 16 M points, k = 4: 208 / 82 us; 290,000 of 1 M, k = 4: 384 / 336 us).
+  constexpr int64_t KNN_LANES = 262144;
+  if (a.k <= 8 && a.n > KNN_LANES) {
+    return a.k == 1 ? launchLanesK<1>(a, self, numSms, s)
+                    : (a.k == 2 ? launchLanesK<2>(a, self, numSms, s)
+                                : (a.k <= 4 ? launchLanesK<4>(a, self, numSms, s) : launchLanesK<8>(a, self, numSms, s)));
   }
+  if (a.k <= 4) {
+    return launchGroupsK<4>(a, self, depth, numSms, s);
+  }
+  if (a.k <= 8) {
+    return launchGroupsK<8>(a, self, depth, numSms, s);
+  }
+  if (a.k <= 16) {
+    return launchGroupsK<16>(a, self, depth, numSms, s);
+  }
+  return launchGroupsK<32>(a, self, depth, numSms, s);
 }
 
 void launchInvertOrder(const float4* pts, int64_t n, uint32_t* inv, cudaStream_t s)

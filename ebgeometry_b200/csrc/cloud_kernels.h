@@ -29,7 +29,7 @@ struct CloudQueryArgs
   const uint32_t*     self_pos; // self queries: sorted position -> the query's leaf position in
                                 // cloud.points (nullptr = identity: every cloud point in leaf order)
   int64_t             n;
-  int                 k;       // neighbours written per query (<= template K)
+  int                 k;       // neighbours written per query
   int32_t*            out_idx; // n x k, caller order
   float*              out_d2;  // n x k
   unsigned long long* work;
@@ -52,7 +52,8 @@ struct CloudTree
 // device memory runs out, else the first failing call's error or cudaSuccess.
 cudaError_t buildCloud(const float* points, int64_t n, int L, bool balanced, float4* leafPts, CloudTree& tree,
                        cudaStream_t s);
-cudaError_t launchCloudKnn(const CloudQueryArgs& a, int kTemplate, int numSms, cudaStream_t s, bool self = false);
+// k-NN of a.n queries (a.k <= 32) in a tree of `depth` node levels.
+cudaError_t launchCloudKnn(const CloudQueryArgs& a, int depth, int numSms, cudaStream_t s, bool self = false);
 
 // inv[cloud index] = leaf position, from the leaf points' index words.
 void launchInvertOrder(const float4* pts, int64_t n, uint32_t* inv, cudaStream_t s);
