@@ -7,8 +7,8 @@
 // for a flat box), coarsened until the grid holds at most 64 + 8 n cells, as the reference sizes
 // it; cell coordinates floor((p - lo) / h) in FP64, clamped; a radix sort of (cell, index) makes
 // every cell a contiguous range of points (float4: xyz and the index bits).
-// Query: one thread per query (queries in Morton order), k best in registers; shells of cells at
-// Chebyshev distance r = 0, 1, ... around the query's cell.  After shell r, every point not yet seen
+// Query: one thread per query (more than 1 M queries in Morton order), k best in registers; shells of cells
+// at Chebyshev distance r = 0, 1, ... around the query's cell.  After shell r, every point not yet seen
 // lies outside the box of cells [c - r, c + r]; its distance is at least the distance from the query
 // to the nearest open side of that box (FP64, minus a relative 1e-9 of h).  The search stops once
 // the k-th best squared distance is strictly below that bound squared, so no point that could
@@ -121,6 +121,8 @@ struct GridQueryArgs
   int32_t*        outIdx;
   float*          outD2;
   int*            status;
+  uint32_t*       later;      // positions of the queries whose search goes beyond shell 1 (nullptr: go on there)
+  uint32_t*       laterCount; // their number, zero before the launch
 };
 
 // The distance from q to the nearest open side of the searched cells [c - r, c + r] along one axis
@@ -139,16 +141,45 @@ __device__ __forceinline__ void sideBound(double q, int c, int r, int n, double 
   }
 }
 
-// 12 blocks per SM for k <= 2 and 8 for k <= 8 (at most 42 and 64 registers): the walk waits on
-// the latency of its cell-bound and point loads, and the extra warps hide more of it (2-10 % faster
-// than the compiler's own 56 and 71 registers).
-template <int K>
-__global__ void __launch_bounds__(128, (K <= 2 ? 12 : (K <= 8 ? 8 : 1))) kGridKnn(const GridQueryArgs a)
+// One query per thread.  The search waits on the latency of its cell-bound and point loads, and on the
+// lanes of a warp whose rows hold more points or that go on to farther shells.  So
+//   FIRST  searches shells 0 and 1 of every query, going through the points of all its rows in one loop
+//          (a lane with empty rows does not wait for the others') with the next point's load under way,
+//          and lists the queries that need shell 2 or more (one in seven at k = 4 on a uniform cloud);
+//   LATER  goes on with the listed ones, which then fill whole warps, from the lists FIRST wrote;
+//   ALL    does all shells at once: one launch, no list; for small calls and for k = 1 (the rule is at
+//          the launch).
+// Rows and planes of cells that lie farther than the k-th best are left out, and long rows are read BATCH
+// points at a time.  1 M queries of 4 M uniform points, k = 4: 500 -> 320 us (FIRST 209, LATER 105); k = 8,
+// 1 M points among themselves: 627 -> 505 us; 1 M clustered points among themselves, k = 8: 3.3 -> 2.6 ms.
+// (Four lanes per query, as the tree search has them for long lists, were slower here: 0.65x at k = 4.)
+//
+// 12 blocks per SM for k <= 2 and 8 for k <= 8 (at most 42 and 64 registers): the extra warps hide more of
+// the latency (2-10 % faster than the compiler's own 56 and 71 registers).
+enum GridMode
 {
-  const GridView& g = a.g;
-  for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < a.n; t += int64_t(gridDim.x) * blockDim.x) {
-    float    qx, qy, qz;
-    uint32_t self = 0xffffffffu, row;
+  ALL,
+  FIRST,
+  LATER
+};
+constexpr int gridOccupancy(int K, int mode) { return K <= 2 ? (mode == LATER ? 8 : 12) : (K <= 8 ? 8 : 1); }
+
+template <int K, int MODE>
+__global__ void __launch_bounds__(128, gridOccupancy(K, MODE)) kGridKnn(const __grid_constant__ GridQueryArgs a)
+{
+  const GridView& g   = a.g;
+  const float     inf = __int_as_float(0x7f800000);
+  __shared__ uint32_t segB[MODE == FIRST ? 10 : 1][128], segE[MODE == FIRST ? 10 : 1][128];
+  // points of a row that are loaded together (the insertions of longer lists are unrolled as often, and
+  // ALL holds eleven copies of the row loop, which would no longer fit the instruction cache: k = 8 with
+  // four, 587 -> 2469 us)
+  constexpr int BATCH = MODE == ALL ? (K == 1 ? 2 : 1) : (K <= 8 ? 4 : 2);
+  const int     tid = threadIdx.x;
+  const int64_t n   = MODE == LATER ? int64_t(*a.laterCount) : a.n;
+  for (int64_t i = int64_t(blockIdx.x) * 128 + tid; i < n; i += int64_t(gridDim.x) * 128) {
+    const int64_t t = MODE == LATER ? int64_t(a.later[i]) : i;
+    float         qx, qy, qz;
+    uint32_t      self = 0xffffffffu, row;
     if (a.queries == nullptr && a.pointIds == nullptr) {
       const float4 q = g.points[t];
       qx             = q.x;
@@ -164,7 +195,7 @@ __global__ void __launch_bounds__(128, (K <= 2 ? 12 : (K <= 8 ? 8 : 1))) kGridKn
         atomicOr(a.status, ST_INPUT);
         for (int j = 0; j < a.k; j++) {
           a.outIdx[size_t(row) * a.k + j] = -1;
-          a.outD2[size_t(row) * a.k + j]  = __int_as_float(0x7f800000);
+          a.outD2[size_t(row) * a.k + j]  = inf;
         }
         continue;
       }
@@ -191,8 +222,14 @@ __global__ void __launch_bounds__(128, (K <= 2 ? 12 : (K <= 8 ? 8 : 1))) kGridKn
     const int pad = K - a.k;
 #pragma unroll
     for (int j = 0; j < K; j++) {
-      kd[j] = j < pad ? -1.f : __int_as_float(0x7f800000);
+      kd[j] = j < pad ? -1.f : inf;
       ki[j] = j < pad ? 0u : 0xffffffffu;
+      if (MODE == LATER && j >= pad) {
+        // the best of shells 0 and 1, as the first launch left them
+        const size_t o = size_t(row) * a.k + (j - pad);
+        kd[j]          = a.outD2[o];
+        ki[j]          = uint32_t(a.outIdx[o]);
+      }
     }
     const double Qx = double(qx), Qy = double(qy), Qz = double(qz);
     const int    cx = cellCoord(Qx, g.lo[0], g.invH, g.n[0]);
@@ -200,27 +237,44 @@ __global__ void __launch_bounds__(128, (K <= 2 ? 12 : (K <= 8 ? 8 : 1))) kGridKn
     const int    cz = cellCoord(Qz, g.lo[2], g.invH, g.n[2]);
     const int    rMax = max(max(max(cx, g.n[0] - 1 - cx), max(cy, g.n[1] - 1 - cy)), max(cz, g.n[2] - 1 - cz));
     // one point into the sorted k-best list (lowest index on equal distances)
-    auto scan = [&](uint32_t b, uint32_t e) {
-#pragma unroll 1
-      for (uint32_t s = b; s < e; s++) {
-        const float4   p  = __ldg(g.points + s);
-        const uint32_t ii = __float_as_uint(p.w);
-        const float    dd = gridD2(p.x, p.y, p.z, qx, qy, qz);
-        if (ii != self && lexLessG(dd, ii, kd[K - 1], ki[K - 1])) {
-          kd[K - 1] = dd;
-          ki[K - 1] = ii;
+    auto take = [&](const float4& p) {
+      const uint32_t ii = __float_as_uint(p.w);
+      const float    dd = gridD2(p.x, p.y, p.z, qx, qy, qz);
+      if (ii != self && lexLessG(dd, ii, kd[K - 1], ki[K - 1])) {
+        kd[K - 1] = dd;
+        ki[K - 1] = ii;
 #pragma unroll
-          for (int j = K - 1; j > 0; j--) {
-            if (lexLessG(kd[j], ki[j], kd[j - 1], ki[j - 1])) {
-              const float    td = kd[j];
-              const uint32_t ti = ki[j];
-              kd[j]             = kd[j - 1];
-              ki[j]             = ki[j - 1];
-              kd[j - 1]         = td;
-              ki[j - 1]         = ti;
-            }
+        for (int j = K - 1; j > 0; j--) {
+          if (lexLessG(kd[j], ki[j], kd[j - 1], ki[j - 1])) {
+            const float    td = kd[j];
+            const uint32_t ti = ki[j];
+            kd[j]             = kd[j - 1];
+            ki[j]             = ki[j - 1];
+            kd[j - 1]         = td;
+            ki[j - 1]         = ti;
           }
         }
+      }
+    };
+    auto scan = [&](uint32_t b, uint32_t e) {
+      uint32_t s = b;
+      if (BATCH > 1) {
+#pragma unroll 1
+        for (; s + BATCH <= e; s += BATCH) {
+          float4 p[BATCH];
+#pragma unroll
+          for (int u = 0; u < BATCH; u++) {
+            p[u] = __ldg(g.points + s + u);
+          }
+#pragma unroll
+          for (int u = 0; u < BATCH; u++) {
+            take(p[u]);
+          }
+        }
+      }
+#pragma unroll 1
+      for (; s < e; s++) {
+        take(__ldg(g.points + s));
       }
     };
     // After shell r: stop once the k-th best is below every distance a later shell can hold (a point
@@ -242,12 +296,21 @@ __global__ void __launch_bounds__(128, (K <= 2 ? 12 : (K <= 8 ? 8 : 1))) kGridKn
       lb = fmax(0.0, lb);
       return double(kd[K - 1]) < lb * lb * (1.0 - 1e-6);
     };
+    // a float no more than the distance along one axis from q to the cells at c + d (the error terms
+    // as in sideBound), and whether points that far (squared) can be among the k best: the float sums of
+    // at most three squares and their distances round by less than 2e-6 of their value together
+    auto gap = [&](double q, int c, int d, double lo) {
+      const double err  = 1e-15 * (fabs(q) + fabs(lo) + double(c + abs(d) + 2) * g.h) + 1e-9 * g.h;
+      const double side = d < 0 ? q - (lo + double(c + d + 1) * g.h) : (lo + double(c + d) * g.h) - q;
+      return d == 0 ? 0.f : fmaxf(0.f, __double2float_rd(side - err));
+    };
+    auto reach = [&](float lb2) { return !(lb2 * (1.f - 2e-6f) > kd[K - 1]); };
+    bool stop = false;
     // Shells 0 and 1: the query's cell, then the rest of the 3 x 3 rows around it, x from cx - 1 to
     // cx + 1 (each row a contiguous range of sorted points).  The bounds of all nine rows and of the
     // query's cell are loaded before any point, so those reads overlap instead of following one
     // another; the check after shell 0 keeps dense cells from scanning their neighbours.
-    bool stop;
-    {
+    if (MODE == ALL) {
       const int      xlo = max(0, cx - 1), xhi = min(g.n[0] - 1, cx + 1);
       uint32_t       rb[9], re[9];
       const uint32_t rowc = (uint32_t(cz) * uint32_t(g.n[1]) + uint32_t(cy)) * uint32_t(g.n[0]);
@@ -278,34 +341,127 @@ __global__ void __launch_bounds__(128, (K <= 2 ? 12 : (K <= 8 ? 8 : 1))) kGridKn
         stop = done(1);
       }
     }
+    if (MODE == FIRST) {
+      const int      xlo = max(0, cx - 1), xhi = min(g.n[0] - 1, cx + 1);
+      const uint32_t rowc = (uint32_t(cz) * uint32_t(g.n[1]) + uint32_t(cy)) * uint32_t(g.n[0]);
+      const uint32_t cb = __ldg(g.cellStart + rowc + cx), ce = __ldg(g.cellStart + rowc + cx + 1);
+      uint32_t       total = 0;
+#pragma unroll
+      for (int j = 0; j < 9; j++) {
+        const int iz = cz - 1 + j / 3, iy = cy - 1 + j % 3;
+        const int o = j == 4 ? 0 : (j & 1) ? 2 + j / 2 : 6 + (j < 4 ? j / 2 : j / 2 - 1); // the near rows first
+        uint32_t  b = 0, e = 0;
+        if (iz >= 0 && iz < g.n[2] && iy >= 0 && iy < g.n[1]) {
+          const uint32_t row0 = (uint32_t(iz) * uint32_t(g.n[1]) + uint32_t(iy)) * uint32_t(g.n[0]);
+          b                   = __ldg(g.cellStart + row0 + xlo);
+          e                   = __ldg(g.cellStart + row0 + xhi + 1);
+        }
+        segB[o][tid] = b;
+        segE[o][tid] = j == 4 ? cb : e;
+        if (j == 4) {
+          segB[1][tid] = ce;
+          segE[1][tid] = e;
+        }
+        total += e - b;
+      }
+      scan(cb, ce);
+      stop = done(0);
+      if (!stop) {
+        // Row by row where cells are dense: lanes of the same cell then read the same points together,
+        // and rows beyond the k-th best are left out.  (A uniform cloud has about 27 points here.)
+        if (__any_sync(__activemask(), total > 64)) {
+          const float gy0 = gap(Qy, cy, -1, g.lo[1]), gy2 = gap(Qy, cy, 1, g.lo[1]);
+          const float gz0 = gap(Qz, cz, -1, g.lo[2]), gz2 = gap(Qz, cz, 1, g.lo[2]);
 #pragma unroll 1
-    for (int r = 2; !stop && r <= rMax; r++) {
-      // the shell at Chebyshev radius r: on its two z faces and two y faces a whole x row of cells
-      // (contiguous in the sorted points), elsewhere the two cells at x = cx -/+ r
-      const int xlo = max(0, cx - r), xhi = min(g.n[0] - 1, cx + r);
-      const int ylo = max(0, cy - r), yhi = min(g.n[1] - 1, cy + r);
-      const int zlo = max(0, cz - r), zhi = min(g.n[2] - 1, cz + r);
-#pragma unroll 1
-      for (int iz = zlo; iz <= zhi; iz++) {
-        const bool zEdge = (iz == cz - r) || (iz == cz + r);
-#pragma unroll 1
-        for (int iy = ylo; iy <= yhi; iy++) {
-          const bool     yEdge = (iy == cy - r) || (iy == cy + r);
-          const uint32_t row0  = (uint32_t(iz) * uint32_t(g.n[1]) + uint32_t(iy)) * uint32_t(g.n[0]);
-          if (zEdge || yEdge) {
-            scan(g.cellStart[row0 + xlo], g.cellStart[row0 + xhi + 1]);
-          }
-          else {
-            if (cx - r >= 0) {
-              scan(g.cellStart[row0 + cx - r], g.cellStart[row0 + cx - r + 1]);
-            }
-            if (cx + r < g.n[0]) {
-              scan(g.cellStart[row0 + cx + r], g.cellStart[row0 + cx + r + 1]);
+          for (int j = 0; j < 10; j++) {
+            const int   y = j < 2 ? 1 : (j < 6 ? (j == 3 ? 0 : j == 4 ? 2 : 1) : (j & 1 ? 2 : 0));
+            const int   z = j < 2 ? 1 : (j < 6 ? (j == 2 ? 0 : j == 5 ? 2 : 1) : (j < 8 ? 0 : 2));
+            const float dy = y == 0 ? gy0 : (y == 2 ? gy2 : 0.f), dz = z == 0 ? gz0 : (z == 2 ? gz2 : 0.f);
+            if (reach(dy * dy + dz * dz)) {
+              scan(segB[j][tid], segE[j][tid]);
             }
           }
         }
+        else {
+          uint32_t s = 0, e = 0;
+          int      j    = 0;
+          auto     next = [&]() {
+            while (s == e && j < 10) {
+              s = segB[j][tid];
+              e = segE[j][tid];
+              j++;
+            }
+            return s != e;
+          };
+          bool   more = next();
+          float4 p    = make_float4(0, 0, 0, 0);
+          if (more) {
+            p = __ldg(g.points + s);
+          }
+#pragma unroll 1
+          while (more) {
+            const float4 c = p;
+            s++;
+            more = next();
+            if (more) {
+              p = __ldg(g.points + s);
+            }
+            take(c);
+          }
+        }
+        stop = done(1);
       }
-      stop = done(r);
+      if (!stop && rMax >= 2) {
+        const unsigned m    = __activemask();
+        const int      lead = __ffs(m) - 1;
+        uint32_t       at   = 0;
+        if ((tid & 31) == lead) {
+          at = atomicAdd(a.laterCount, uint32_t(__popc(m)));
+        }
+        at = __shfl_sync(m, at, lead);
+        a.later[at + __popc(m & ((1u << (tid & 31)) - 1u))] = uint32_t(t);
+      }
+    }
+    else {
+#pragma unroll 1
+      for (int r = 2; !stop && r <= rMax; r++) {
+        // the shell at Chebyshev radius r: on its two z faces and two y faces a whole x row of cells
+        // (contiguous in the sorted points), elsewhere the two cells at x = cx -/+ r
+        const int xlo = max(0, cx - r), xhi = min(g.n[0] - 1, cx + r);
+        const int ylo = max(0, cy - r), yhi = min(g.n[1] - 1, cy + r);
+        const int zlo = max(0, cz - r), zhi = min(g.n[2] - 1, cz + r);
+        const float gl = gap(Qx, cx, -r, g.lo[0]), gr = gap(Qx, cx, r, g.lo[0]);
+#pragma unroll 1
+        for (int iz = zlo; iz <= zhi; iz++) {
+          const bool  zEdge = (iz == cz - r) || (iz == cz + r);
+          const float gz    = gap(Qz, cz, iz - cz, g.lo[2]);
+          if (!reach(gz * gz)) {
+            continue;
+          }
+#pragma unroll 1
+          for (int iy = ylo; iy <= yhi; iy++) {
+            const float gy  = gap(Qy, cy, iy - cy, g.lo[1]);
+            const float gyz = gy * gy + gz * gz;
+            if (!reach(gyz)) {
+              continue;
+            }
+            const bool     yEdge = (iy == cy - r) || (iy == cy + r);
+            const uint32_t row0  = (uint32_t(iz) * uint32_t(g.n[1]) + uint32_t(iy)) * uint32_t(g.n[0]);
+            if (zEdge || yEdge) {
+              scan(__ldg(g.cellStart + row0 + xlo), __ldg(g.cellStart + row0 + xhi + 1));
+            }
+            else {
+              if (cx - r >= 0 && reach(gyz + gl * gl)) {
+                scan(__ldg(g.cellStart + row0 + cx - r), __ldg(g.cellStart + row0 + cx - r + 1));
+              }
+              if (cx + r < g.n[0] && reach(gyz + gr * gr)) {
+                scan(__ldg(g.cellStart + row0 + cx + r), __ldg(g.cellStart + row0 + cx + r + 1));
+              }
+            }
+          }
+        }
+        stop = done(r);
+      }
     }
 #pragma unroll
     for (int j = 0; j < K; j++) {
@@ -313,37 +469,34 @@ __global__ void __launch_bounds__(128, (K <= 2 ? 12 : (K <= 8 ? 8 : 1))) kGridKn
         const bool   found = ki[j] != 0xffffffffu;
         const size_t o     = size_t(row) * a.k + (j - pad);
         a.outIdx[o]        = found ? int32_t(ki[j]) : -1;
-        a.outD2[o]         = found ? kd[j] : __int_as_float(0x7f800000);
+        a.outD2[o]         = found ? kd[j] : inf;
       }
     }
   }
 }
 
+// a.later == nullptr: one launch; else the queries that go beyond shell 1 are searched in a second one
 template <int K>
 cudaError_t launchGridK(const GridQueryArgs& a, int numSms, cudaStream_t s)
 {
-  int64_t blocks = (a.n + 127) / 128;
-  blocks         = std::min<int64_t>(blocks, int64_t(numSms) * 32);
-  kGridKnn<K><<<unsigned(std::max<int64_t>(blocks, 1)), 128, 0, s>>>(a);
+  const int64_t blocks = std::max<int64_t>(std::min<int64_t>((a.n + 127) / 128, int64_t(numSms) * 32), 1);
+  if (a.later == nullptr) {
+    kGridKnn<K, ALL><<<unsigned(blocks), 128, 0, s>>>(a);
+    return cudaGetLastError();
+  }
+  kGridKnn<K, FIRST><<<unsigned(blocks), 128, 0, s>>>(a);
+  kGridKnn<K, LATER><<<unsigned(blocks), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
-cudaError_t launchGridKnn(const GridQueryArgs& a, int kt, int numSms, cudaStream_t s)
+cudaError_t launchGridKnn(const GridQueryArgs& a, int numSms, cudaStream_t s)
 {
-  switch (kt) {
-  case 1:
-    return launchGridK<1>(a, numSms, s);
-  case 2:
-    return launchGridK<2>(a, numSms, s);
-  case 4:
-    return launchGridK<4>(a, numSms, s);
-  case 8:
-    return launchGridK<8>(a, numSms, s);
-  case 16:
-    return launchGridK<16>(a, numSms, s);
-  default:
-    return launchGridK<32>(a, numSms, s);
-  }
+  return a.k <= 1    ? launchGridK<1>(a, numSms, s)
+         : a.k <= 2  ? launchGridK<2>(a, numSms, s)
+         : a.k <= 4  ? launchGridK<4>(a, numSms, s)
+         : a.k <= 8  ? launchGridK<8>(a, numSms, s)
+         : a.k <= 16 ? launchGridK<16>(a, numSms, s)
+                     : launchGridK<32>(a, numSms, s);
 }
 
 unsigned gridBlocks(int64_t n) { return unsigned(std::min<int64_t>(std::max<int64_t>((n + 255) / 256, 1), 1 << 20)); }
@@ -555,15 +708,20 @@ ebg_status ebg_grid_info(const ebg_grid* G, int32_t* cells_xyz, double* cell_siz
   return EBG_OK;
 }
 
+// External queries are put in Morton order from this count on.  Below it the order costs more than the
+// nearer reads give: 4 M points, 262,144 queries with and without it 208 and 131 us, 1 M queries (k = 4)
+// 395 and 333, (k = 1) 258 and 195; 16 M points, 4 M queries 942 and 1494.
+static constexpr int64_t GRID_ORDERED = (1 << 20) + 1;
+// Calls of this many queries (any number for k > 8, none for k = 1) put those that go beyond shell 1 into a
+// second launch.  4 M points, k = 4, without and with it: 131,072 queries 73 and 92 us, 262,144 132 and 128,
+// 1 M 419 and 328; k = 16, 3000 and 262,144 queries 152 and 147 us, 1002 and 711; k = 1, 1 M: 205 and 310.
+static constexpr int64_t GRID_SPLIT = 1 << 18;
+
 // The three query forms: external points (queries), self queries of listed cloud indices (ids) and
 // self queries of every point (neither).  Asynchronous on s.
 static ebg_status gridQuery(const ebg_grid* G, const float* queries_dev, const int64_t* ids_dev, int64_t nq, int32_t k,
                             int32_t* idx_dev, float* d2_dev, cudaStream_t s)
 {
-  int kt = 1;
-  while (kt < k) {
-    kt *= 2;
-  }
   std::vector<void*> ws;
   auto get = [&](size_t bytes) -> void* {
     void* p = nullptr;
@@ -580,7 +738,7 @@ static ebg_status gridQuery(const ebg_grid* G, const float* queries_dev, const i
     }
   };
   uint32_t* order = nullptr;
-  if (queries_dev) {
+  if (queries_dev && nq >= GRID_ORDERED) {
     // Morton order of the queries over the grid's box, so that a warp's queries visit nearby cells
     auto* kin  = static_cast<uint32_t*>(get(4 * size_t(nq)));
     auto* kout = static_cast<uint32_t*>(get(4 * size_t(nq)));
@@ -613,7 +771,18 @@ static ebg_status gridQuery(const ebg_grid* G, const float* queries_dev, const i
   a.outIdx   = idx_dev;
   a.outD2    = d2_dev;
   a.status   = G->dStatus;
-  const cudaError_t e = launchGridKnn(a, kt, G->numSms, s);
+  if (k > 1 && (k > 8 || nq >= GRID_SPLIT)) {
+    a.later      = static_cast<uint32_t*>(get(4 * size_t(nq)));
+    a.laterCount = static_cast<uint32_t*>(get(4));
+    if (a.later && a.laterCount) {
+      cudaMemsetAsync(a.laterCount, 0, 4, s);
+    }
+    else {
+      cudaGetLastError(); // no memory for the list: one launch does without it
+      a.later = nullptr;
+    }
+  }
+  const cudaError_t e = launchGridKnn(a, G->numSms, s);
   release();
   if (e != cudaSuccess) {
     return setError(EBG_ERR_CUDA, std::string("grid k-NN launch failed: ") + cudaGetErrorString(e));
