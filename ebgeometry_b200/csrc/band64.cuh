@@ -7,14 +7,14 @@
 //  - triSd64: a lane-by-lane restatement of the AVX W=4 double path of TriangleSoAT::signedDistance
 //    (TriangleSoAImplem.hpp:1029-1180, sign-bit convention of :1076-1082);
 //  - dcelFaceSd / dcelFaceUd2: one triangle as a DCEL face, the algorithm of MeshSDF and FlatMeshSDF;
-//  - band64Mesh: one packet's FP64 search of a mesh for the triangle of smallest |d| within each
-//    lane's bound (strict <, MeshDistanceFunctionsImplem.hpp:492-502).
+//  - pointSearch64: the FP64 search of a mesh for one point.
 #ifndef EBG_BAND64_CUH
 #define EBG_BAND64_CUH
 
 #include <cfloat>
 
 #include "ebg_device.cuh"
+#include "mesh_point.cuh"
 #include "mesh_traverse.cuh"
 
 namespace ebg {
@@ -185,108 +185,60 @@ __device__ double dcelFaceUd2(const double* __restrict__ tri, const double* __re
   return best;
 }
 
-// One packet's FP64 search of mesh m.  Each lane has its FP64 point P, the FP32 point (px, py, pz)
-// at which boxes are tested (`shift` from P), its squared search bound `bound` (FP32, at the FP32
-// point) and its running FP64 result (best, bt: the value of smallest |d| and its triangle, leaf
-// order; DBL_MAX / -1 before the first).  Triangles are tested in FP64 with the Triangle test; each winner
-// shrinks the lane's bound.  Leaves and nodes are pruned by their axis-aligned and oriented boxes (padded
-// to bound the exact distance of every triangle inside from below).  All 32 lanes call it together;
-// `stk` is the warp's stack (STACK entries).
-template <int STACK = EBG_STACK_DEPTH>
-__device__ void band64Mesh(const EbgMeshView& m, D3 P, float px, float py, float pz, float shift, float& bound,
-                           double& best, int& bt, float4* stk, uint32_t& iters, int& err)
+// The triangle of smallest |d| in FP64 within `bound` of the FP32 point (px, py, pz), which lies
+// `shift` from P (strict <, MeshDistanceFunctionsImplem.hpp:492-502; ties
+// to the lower leaf position): all lanes on one point (mesh_point.cuh), whose FP32 distances select the
+// triangles worth an FP64 test.  `best` DBL_MAX and `bt` -1 if there is none.
+template <int EVAL, bool UPPER>
+__device__ int pointSearch64(const EbgMeshView& m, D3 P, float px, float py, float pz, float shift, float delta,
+                             float bound, double& best, int& bt, PointMem& w)
 {
-  const int lane = threadIdx.x & 31;
-  int       sp   = 1;
-  if (lane == 0) {
-    stk[0] = make_float4(m.root_lo[0], m.root_lo[1], m.root_lo[2], __uint_as_float(m.root_ref));
-    stk[1] = make_float4(m.root_hi[0], m.root_hi[1], m.root_hi[2], __uint_as_float(m.root_count));
-  }
-  __syncwarp();
-  while (sp > 0) {
-    if (++iters > MAX_ITERS) {
-      err |= ST_ITERS;
-      break;
+  const float inf   = __int_as_float(0x7f800000);
+  const float slack = delta + 2.f * shift;
+  best              = DBL_MAX;
+  bt                = -1;
+  return pointSearch<UPPER>(m, px, py, pz, bound, slack, w, [&](bool active, uint32_t tri) {
+    float dd = inf, low = inf;
+    if (active) {
+      const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
+      const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+      float         s, t;
+      int           r;
+      dd  = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
+      low = triLower(h0, h1, h2, px, py, pz, s, t, dd);
     }
-    --sp;
-    const float4 A = stk[2 * sp], B = stk[2 * sp + 1];
-    const float  d2 = boxDist2(A.x, A.y, A.z, B.x, B.y, B.z, px, py, pz);
-    if (!__any_sync(FULL, d2 <= bound)) {
-      continue;
+    const float near = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(dd)));
+    const float rn   = (sqrtf(near) * 1.00001f + slack) * 1.000001f;
+    bound            = fminf(bound, rn * rn);
+    // (not "low <= ...": a point on the triangle has no direction and a NaN bound)
+    const bool cand = active && !(low > sqrtf(bound) * 1.00001f + delta);
+    if (!__any_sync(FULL, cand)) {
+      return;
     }
-    const uint32_t cntw = __float_as_uint(B.w);
-    const uint32_t ref = __float_as_uint(A.w), cnt = cntw & EBG_COUNT_MASK;
-    // the leaf's or node's oriented box (padded to bound the exact distance of every triangle
-    // inside from below) before its triangles or children
-    const EbgObb* obx = (ref & EBG_LEAF_BIT) ? m.obb + (cntw >> EBG_COUNT_BITS)
-                                             : ((cntw & EBG_NODE_HAS_OBB) ? m.node_obb + ref : nullptr);
-    if (obx != nullptr) {
-      const float4* ob = reinterpret_cast<const float4*>(obx);
-      if (!__any_sync(FULL, obbDist2(__ldg(ob), __ldg(ob + 1), __ldg(ob + 2), __ldg(ob + 3), px, py, pz) <= bound)) {
-        continue;
-      }
+    double d = DBL_MAX;
+    if (cand) {
+      d = EVAL == 0 ? triSd64(m.tri64 + 30 * size_t(tri), P)
+                    : dcelFaceSd(m.tri64 + 30 * size_t(tri), m.dcel_n + 3 * size_t(tri), P);
     }
-    if (ref & EBG_LEAF_BIT) {
-      const uint32_t t0 = ref & ~EBG_LEAF_BIT;
-      for (uint32_t tt = t0; tt < t0 + cnt; ++tt) {
-        const double d = triSd64(m.tri64 + 30 * size_t(tt), P);
-        // strict < as the reference's leaf loop, ties to the lower leaf position (the winner is
-        // then independent of the traversal order)
-        if (fabs(d) < fabs(best) || (fabs(d) == fabs(best) && int(tt) < bt)) {
-          best = d;
-          bt   = int(tt);
-          // shrink the bound to the FP64 winner (with the same relative margin), measured at the
-          // FP32 point where the boxes are tested
-          const float rb = (float(fabs(d)) + shift) * 1.000001f + 1e-30f;
-          bound          = fminf(bound, rb * rb);
-        }
-      }
+    // the warp's least (|d|, triangle): non-negative doubles order like their words
+    const uint32_t hi = cand ? uint32_t(__double2hiint(fabs(d))) : 0xffffffffu;
+    const uint32_t mh = __reduce_min_sync(FULL, hi);
+    const uint32_t lo = hi == mh ? uint32_t(__double2loint(d)) : 0xffffffffu;
+    const uint32_t ml = __reduce_min_sync(FULL, lo);
+    const uint32_t ti = cand && hi == mh && lo == ml ? tri : 0xffffffffu;
+    const uint32_t mt = __reduce_min_sync(FULL, ti);
+    const unsigned who = __ballot_sync(FULL, ti == mt && cand);
+    if (mt == 0xffffffffu || who == 0u) {
+      return; // only NaN values
     }
-    else {
-      const EbgNode4& nd = m.nodes[ref];
-      int             o[4], np = 0;
-      float           key[4];
-      for (int k = 0; k < 4; k++) {
-        const float dk = boxDist2(nd.lox[k], nd.loy[k], nd.loz[k], nd.hix[k], nd.hiy[k], nd.hiz[k], px, py, pz);
-        // empty slot: child 0 and count 0 (node 0 is the root and never a child)
-        if (__any_sync(FULL, dk <= bound) && (nd.child[k] | nd.count[k]) != 0u) {
-          o[np]   = k;
-          key[np] = dk;
-          np++;
-        }
-      }
-      // per-lane keys differ, so order by lane 0's distance (any fixed order is correct)
-      for (int i = 0; i < np; i++) {
-        key[i] = __shfl_sync(FULL, key[i], 0);
-      }
-      for (int i = 1; i < np; i++) {
-        for (int q = i; q > 0 && key[q - 1] < key[q]; q--) {
-          const float tk = key[q];
-          key[q]         = key[q - 1];
-          key[q - 1]     = tk;
-          const int to   = o[q];
-          o[q]           = o[q - 1];
-          o[q - 1]       = to;
-        }
-      }
-      for (int i = 0; i < np; i++) {
-        if (sp >= STACK) {
-          err |= ST_STACK;
-          break;
-        }
-        const int k = o[i];
-        if (lane == 0) {
-          stk[2 * sp]     = make_float4(nd.lox[k], nd.loy[k], nd.loz[k], __uint_as_float(nd.child[k]));
-          stk[2 * sp + 1] = make_float4(nd.hix[k], nd.hiy[k], nd.hiz[k], __uint_as_float(nd.count[k]));
-        }
-        sp++;
-      }
-      __syncwarp();
-      if (err) {
-        break;
-      }
+    const double dm = __shfl_sync(FULL, d, __ffs(int(who)) - 1);
+    if (fabs(dm) < fabs(best) || (fabs(dm) == fabs(best) && int(mt) < bt)) {
+      best           = dm;
+      bt             = int(mt);
+      const float rb = (float(fabs(dm)) + shift) * 1.000001f + 1e-30f;
+      bound          = fminf(bound, rb * rb);
     }
-  }
+  });
 }
 
 } // namespace

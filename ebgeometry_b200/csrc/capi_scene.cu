@@ -184,6 +184,8 @@ ebg_status sceneQuery(const ebg_scene*      s,
   a.band_flag  = flags;
   a.band_list  = bandList;
   a.band_count = bandCnt;
+  // delta bounds the FP32 error of the union's value: the instance transform and the mesh distance
+  a.delta       = float(4e-6 * s->errScale) + 1e-30f;
   cudaError_t e = launchSceneValue(a, s->numSms, st);
   if (e == cudaSuccess && band64) {
     if (cub::DeviceSelect::Flagged(selTemp, selBytes, thrust::counting_iterator<uint32_t>(0u), flags, bandList,
@@ -192,8 +194,7 @@ ebg_status sceneQuery(const ebg_scene*      s,
       e = e == cudaSuccess ? cudaErrorUnknown : e;
     }
     else {
-      // delta bounds the FP32 error of the union's value: the instance transform and the mesh distance
-      e = launchSceneBand64(a, float(4e-6 * s->errScale) + 1e-30f, s->numSms, st);
+      e = launchSceneBand64(a, s->numSms, st);
     }
   }
   release();
@@ -303,6 +304,8 @@ ebg_status ebg_scene_create(int64_t                num_spheres,
     // world box: the 8 corners of the local box mapped back (p = R^T local + t), grown by the
     // float rounding of the instance transform
     const ebg_mesh_info& inf = meshes[m]->info;
+    o.radius                 = float(inf.diagonal);
+    o.leaves                 = float(inf.num_leaves);
     double               wl[3] = {1e300, 1e300, 1e300}, wh[3] = {-1e300, -1e300, -1e300};
     for (int c = 0; c < 8; c++) {
       const double L[3] = {(c & 1) ? inf.hi[0] : inf.lo[0], (c & 2) ? inf.hi[1] : inf.lo[1],

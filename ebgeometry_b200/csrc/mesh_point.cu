@@ -17,60 +17,6 @@ namespace {
 
 constexpr int POINT_WARPS = 4;
 
-// The triangle of smallest |d| in FP64 within `bound` of the FP32 point (px, py, pz), which lies
-// `shift` from P (see band64Mesh); its FP32 distance selects the triangles worth an FP64 test.
-template <int EVAL, bool UPPER>
-__device__ int pointSearch64(const EbgMeshView& m, D3 P, float px, float py, float pz, float shift, float delta,
-                             float bound, double& best, int& bt, PointMem& w)
-{
-  const float inf   = __int_as_float(0x7f800000);
-  const float slack = delta + 2.f * shift;
-  best              = DBL_MAX;
-  bt                = -1;
-  return pointSearch<UPPER>(m, px, py, pz, bound, slack, w, [&](bool active, uint32_t tri) {
-    float dd = inf, low = inf;
-    if (active) {
-      const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
-      const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-      float         s, t;
-      int           r;
-      dd  = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
-      low = triLower(h0, h1, h2, px, py, pz, s, t, dd);
-    }
-    const float near = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(dd)));
-    const float rn   = (sqrtf(near) * 1.00001f + slack) * 1.000001f;
-    bound            = fminf(bound, rn * rn);
-    // (not "low <= ...": a point on the triangle has no direction and a NaN bound)
-    const bool cand = active && !(low > sqrtf(bound) * 1.00001f + delta);
-    if (!__any_sync(FULL, cand)) {
-      return;
-    }
-    double d = DBL_MAX;
-    if (cand) {
-      d = EVAL == 0 ? triSd64(m.tri64 + 30 * size_t(tri), P)
-                    : dcelFaceSd(m.tri64 + 30 * size_t(tri), m.dcel_n + 3 * size_t(tri), P);
-    }
-    // the warp's least (|d|, triangle): non-negative doubles order like their words
-    const uint32_t hi = cand ? uint32_t(__double2hiint(fabs(d))) : 0xffffffffu;
-    const uint32_t mh = __reduce_min_sync(FULL, hi);
-    const uint32_t lo = hi == mh ? uint32_t(__double2loint(d)) : 0xffffffffu;
-    const uint32_t ml = __reduce_min_sync(FULL, lo);
-    const uint32_t ti = cand && hi == mh && lo == ml ? tri : 0xffffffffu;
-    const uint32_t mt = __reduce_min_sync(FULL, ti);
-    const unsigned who = __ballot_sync(FULL, ti == mt && cand);
-    if (mt == 0xffffffffu || who == 0u) {
-      return; // only NaN values
-    }
-    const double dm = __shfl_sync(FULL, d, __ffs(int(who)) - 1);
-    if (fabs(dm) < fabs(best) || (fabs(dm) == fabs(best) && int(mt) < bt)) {
-      best           = dm;
-      bt             = int(mt);
-      const float rb = (float(fabs(dm)) + shift) * 1.000001f + 1e-30f;
-      bound          = fminf(bound, rb * rb);
-    }
-  });
-}
-
 // F64: FP64 points and results with evaluator EVAL (0 the Triangle test, 1 the DCEL face).  Else
 // FP32 points and results: the FP32 search, and the FP64 one where |d| is within the band.
 // Bound by the latency of its dependent loads (two per tree level and two per leaf batch), so the

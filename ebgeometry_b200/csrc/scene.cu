@@ -9,15 +9,23 @@
 // the mesh kernel).  At an object leaf every lane evaluates every object of the leaf:
 //   sphere: |p - c| - r;
 //   mesh:   the query is moved into the mesh's frame (RotateIF / TranslateIF: local = R (p - t),
-//           TransformImplem.hpp:152-225) and the mesh's own BVH is traversed by the same packet,
-//           on a second stack region.  The nested traversal is seeded with the lane's running
-//           minimum when the local point lies outside the mesh's box (then the point is outside the
-//           mesh, and finding no triangle within the bound proves the mesh cannot lower the
-//           minimum); inside the box it runs unseeded, because a point inside the mesh can have a
-//           large negative distance.
+//           TransformImplem.hpp:152-225) and the mesh is searched for the lanes it can matter to: by the
+//           packet together (mesh_traverse.cuh, on a second stack region) or one query after the other
+//           with a lane per child or triangle (mesh_point.cuh); the rule is at the test.  The search is
+//           seeded with the lane's running minimum when the local point lies outside the mesh's box (then
+//           the point is outside the mesh, and finding no triangle within the bound proves the mesh cannot
+//           lower the minimum); inside the box it runs unseeded, because a point inside the mesh can have
+//           a large negative distance.
+//
+// Objects are small against a packet of scattered points, so what bounds the call is the search of whole
+// meshes for packets that surround them (1.3 ms for one packet with 20,480 triangles, at any number of
+// points).  1024 spheres and 48 meshes of 1280 to 20,480 triangles, packets only -> now: 2 M points 2420
+// -> 1280 us in this kernel, 131,072 points 1540 -> 400; 1,000 points 2280 -> 218 us the whole call.
 #include <cfloat>
 
 #include "ebg_device.cuh"
+#include "mesh_packet.cuh"
+#include "mesh_point.cuh"
 #include "mesh_traverse.cuh"
 #include "scene_kernels.h"
 
@@ -25,6 +33,7 @@ namespace ebg {
 
 namespace {
 
+static_assert(sizeof(PointMem) <= 2 * EBG_STACK_DEPTH * sizeof(float4), "the point search's memory is the mesh stack");
 constexpr int OUTER_DEPTH = 48; // object-BVH stack entries per warp (builder checks the depth)
 
 // A batched call whose batch sizes did not add up to its point count reads no point.
@@ -42,7 +51,7 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
   float4*           istk  = ostk + 2 * OUTER_DEPTH;
   float4*           lpts  = istk + 2 * EBG_STACK_DEPTH; // the warp's 32 spread-leaf points
   const SceneView&  sc    = a.scene;
-  const uint64_t    numPk = (uint64_t(a.n) + 31) / 32;
+  const uint64_t    numPk = (uint64_t(a.n) + a.per - 1) / a.per;
   if (!batchesValid(a)) {
     return;
   }
@@ -61,9 +70,9 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
     if (pk >= numPk) {
       break;
     }
-    const int64_t  pos   = int64_t(pk) * 32 + lane;
-    const bool     valid = pos < a.n;
-    const int64_t  src   = valid ? pos : a.n - 1;
+    const int64_t  pos   = int64_t(pk) * a.per + lane;
+    const bool     valid = lane < a.per && pos < a.n;
+    const int64_t  src   = pos < a.n ? pos : a.n - 1;
     const uint32_t id    = a.order ? __ldg(a.order + src) : uint32_t(src);
     float*         outp  = nullptr;
     const float*   pp    = scenePoint(a, id, &outp);
@@ -111,8 +120,59 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
           const bool seeded = outsideBox && best > 0.f && best < 1e18f;
           float      mb     = seeded ? best * best * 1.000004f : FLT_MAX;
           int        bt     = -1;
-          TraversalCounters tc;
-          traverseMesh<false>(mv, lx, ly, lz, mb, bt, istk, lpts, iters, err, tc);
+          const float    bd   = boxDist2(mv.root_lo[0], mv.root_lo[1], mv.root_lo[2], mv.root_hi[0], mv.root_hi[1],
+                                         mv.root_hi[2], lx, ly, lz);
+          const bool     need = valid && bd <= mb;
+          const unsigned who  = __ballot_sync(FULL, need);
+          if (who == 0u) {
+            continue;
+          }
+          const float inf = __int_as_float(0x7f800000);
+          const float ex = warpMax(need ? lx : -inf) - warpMin(need ? lx : inf);
+          const float ey = warpMax(need ? ly : -inf) - warpMin(need ? ly : inf);
+          const float ez = warpMax(need ? lz : -inf) - warpMin(need ? lz : inf);
+          // The packet opens about as many leaves as lie within the span of its points' nearest points: of
+          // all leaves (span / diagonal)^2, the span shrinking from the points' extent with their distance
+          // from the mesh.  A leaf costs the packet about what the rounds of one query's own search cost per
+          // sixth of it.  1024 spheres and 48 meshes, 2 M points, limits of 1, 2, 4, 6, 8 and 12 leaves per
+          // query: 2267, 2205, 2127, 2122, 2604 and 3190 us; the meshes alone: 6878, 6244, 5815, 5642,
+          // 5544 and 5482 (packets only 5950).  Up to two queries never make a packet.
+          const float far = ob.radius + 3.f * sqrtf(warpMin(need ? bd : inf));
+          if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) * ob.leaves >= (6.f * float(__popc(who)) - 12.f) * far * far) {
+#pragma unroll 1
+            for (unsigned rest = who; rest != 0u; rest &= rest - 1) {
+              const int   l = __ffs(int(rest)) - 1;
+              const float x = __shfl_sync(FULL, lx, l), y = __shfl_sync(FULL, ly, l), z = __shfl_sync(FULL, lz, l);
+              float       bd2 = __shfl_sync(FULL, mb, l), bound = bd2;
+              int         tb  = -1;
+              err |= pointSearch<true>(mv, x, y, z, bound, a.delta, *reinterpret_cast<PointMem*>(istk),
+                                       [&](bool active, uint32_t tri) {
+                float dd = inf;
+                if (active) {
+                  const float4* h  = reinterpret_cast<const float4*>(mv.hot + tri);
+                  const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+                  float         s_, t_;
+                  int           r_;
+                  dd = triDist2<false>(h0, h1, h2, x, y, z, s_, t_, r_);
+                }
+                // ties go to the lower leaf position, as in the packet traversal
+                const uint32_t m0 = __reduce_min_sync(FULL, __float_as_uint(dd));
+                const uint32_t mt = __reduce_min_sync(FULL, __float_as_uint(dd) == m0 ? tri : 0x7fffffffu);
+                const float    md = __uint_as_float(m0);
+                if (md < bd2 || (md == bd2 && int(mt) < tb)) {
+                  bd2   = md;
+                  tb    = int(mt);
+                  bound = fminf(bound, bd2);
+                }
+              });
+              bt = lane == l ? tb : bt;
+            }
+          }
+          else {
+            TraversalCounters tc;
+            mb = need ? mb : -1.f;
+            traverseMesh<false>(mv, lx, ly, lz, mb, bt, istk, lpts, iters, err, tc);
+          }
           if (err) {
             break;
           }
@@ -232,7 +292,7 @@ cudaError_t launchSceneBatchStarts(const SceneBatch* batches, int32_t nb, int64_
   return cudaGetLastError();
 }
 
-cudaError_t launchSceneValue(const SceneQueryArgs& a, int numSms, cudaStream_t s)
+cudaError_t launchSceneValue(const SceneQueryArgs& args, int numSms, cudaStream_t s)
 {
   // resident blocks per SM, looked up once (the query then issues only stream-ordered work and can
   // be captured in a CUDA graph)
@@ -243,8 +303,14 @@ cudaError_t launchSceneValue(const SceneQueryArgs& a, int numSms, cudaStream_t s
     perSm  = perSm < 1 ? 1 : perSm;
     cached = perSm;
   }
-  const int64_t need = ((int64_t(a.n) + 31) / 32 + 3) / 4;
-  int64_t       grid = int64_t(numSms) * perSm;
+  int64_t        grid = int64_t(numSms) * perSm;
+  SceneQueryArgs a    = args;
+  a.per               = 32;
+  // few queries are spread over all warps, fewer than 32 to each (1,000 points in 32s: 846 us, one each: 218)
+  while (a.per > 1 && a.n / a.per < 4 * grid) {
+    a.per /= 2;
+  }
+  const int64_t need = ((a.n + a.per - 1) / a.per + 3) / 4;
   grid               = grid < need ? grid : need;
   grid               = grid < 1 ? 1 : grid;
   kSceneValue<<<unsigned(grid), 128, 0, s>>>(a);

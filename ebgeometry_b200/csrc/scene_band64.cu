@@ -9,11 +9,16 @@
 // reached is evaluated as the reference does:
 //   sphere:          |p - c| - r;
 //   mesh instance:   TranslateIF(RotateIF(TriMeshSDF)) -- local = rot(p - t) with RotateIF's
-//                    per-axis formulas (TransformImplem.hpp:152-225) -- then the FP64 triangle test
-//                    over every triangle within |d32| + delta of the local point (band64.cuh), whose
-//                    winner is the mesh's exact value whenever the mesh can hold the minimum (a
-//                    winner farther than that is left out: such a mesh cannot).
+//                    per-axis formulas (TransformImplem.hpp:152-225) -- then the FP64 search within
+//                    |d32| + delta of the local point (pointSearch64), whose winner is the mesh's exact
+//                    value whenever the mesh can hold the minimum (a winner farther than that is left
+//                    out: such a mesh cannot).
 // The union's value is the minimum over them (std::min, as the reference's evalLeaf).
+//
+// The band's queries are few and lie scattered on the surfaces, so a packet of 32 is a chain of 32 small
+// searches: bound by latency.  All lanes of a warp work on one query's search, an FP32 lower bound keeps
+// most triangles from the FP64 test, and the queries are spread over all warps.  1024 spheres and 48
+// meshes, 2 M points: 543 us with packets that test every triangle of a leaf in every lane, now 24.
 #include <cfloat>
 
 #include <math_constants.h>
@@ -29,24 +34,31 @@ namespace {
 
 constexpr int BAND_OUTER = 48; // object-BVH stack entries per warp (the scene builder checks the depth)
 
-__global__ void __launch_bounds__(128, 4) kSceneBand64(const SceneQueryArgs a, float delta)
+__global__ void __launch_bounds__(128, 4) kSceneBand64(const SceneQueryArgs a)
 {
-  __shared__ float4 smem[4 * 2 * (BAND_OUTER + EBG_STACK_DEPTH)];
-  const int         lane  = threadIdx.x & 31;
-  float4*           ostk  = smem + (threadIdx.x >> 5) * (2 * (BAND_OUTER + EBG_STACK_DEPTH));
-  float4*           istk  = ostk + 2 * BAND_OUTER;
+  const float       delta = a.delta;
+  __shared__ float4   smem[4 * 2 * BAND_OUTER];
+  __shared__ PointMem mem[4];
+  const int           lane = threadIdx.x & 31;
+  float4*             ostk = smem + (threadIdx.x >> 5) * (2 * BAND_OUTER);
+  PointMem&           w    = mem[threadIdx.x >> 5];
   const SceneView&  sc    = a.scene;
   if (a.batches != nullptr && __ldg(a.batch_start + a.num_batches) != a.n) {
     return;
   }
   const uint32_t count  = *a.band_count;
-  const uint32_t numPk  = (count + 31) / 32;
   const uint32_t warpId = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nWarps = (gridDim.x * blockDim.x) >> 5;
+  // few queries are spread over all warps, fewer than 32 to each
+  uint32_t per = 32;
+  while (per > 1 && count / per < nWarps) {
+    per /= 2;
+  }
+  const uint32_t numPk = (count + per - 1) / per;
 
   for (uint32_t pk = warpId; pk < numPk; pk += nWarps) {
-    const uint32_t j     = pk * 32 + lane;
-    const bool     valid = j < count;
+    const uint32_t j     = pk * per + lane;
+    const bool     valid = lane < int(per) && j < count;
     const uint32_t pos   = a.band_list[valid ? j : count - 1];
     const uint32_t id    = a.order ? a.order[pos] : pos;
     float*         outp  = nullptr;
@@ -110,19 +122,26 @@ __global__ void __launch_bounds__(128, 4) kSceneBand64(const SceneQueryArgs a, f
           const double ex = L.x - double(lx), ey = L.y - double(ly), ez = L.z - double(lz);
           const float  shift = float(sqrt(ex * ex + ey * ey + ez * ez)) * 1.0001f;
           const float  r     = (mr + 2.f * shift) * 1.000001f;
-          float        bound = r * r;
-          double       mb    = DBL_MAX;
-          int          mbt   = -1;
-          band64Mesh(mv, L, lx, ly, lz, shift, bound, mb, mbt, istk, iters, err);
+          const float  bound = r * r;
+          const bool   need  = valid && boxDist2(mv.root_lo[0], mv.root_lo[1], mv.root_lo[2], mv.root_hi[0],
+                                                 mv.root_hi[1], mv.root_hi[2], lx, ly, lz) <= bound;
+#pragma unroll 1
+          for (unsigned rest = __ballot_sync(FULL, need); rest != 0u; rest &= rest - 1) {
+            const int l  = __ffs(int(rest)) - 1;
+            const D3  Ll = {__shfl_sync(FULL, L.x, l), __shfl_sync(FULL, L.y, l), __shfl_sync(FULL, L.z, l)};
+            double    mb;
+            int       mbt;
+            err |= pointSearch64<0, false>(mv, Ll, float(Ll.x), float(Ll.y), float(Ll.z), __shfl_sync(FULL, shift, l),
+                                           delta, __shfl_sync(FULL, bound, l), mb, mbt, w);
+            // Within mr is the mesh's exact value; beyond it (a leaf in reach is tested as a whole) the
+            // mesh cannot hold the minimum (its value is above d32 + delta, or below d32 - delta, which
+            // the minimum is not) and is left out.
+            if (lane == l && mbt >= 0 && fabs(mb) <= double(mr)) {
+              best = fmin(best, mb);
+            }
+          }
           if (err) {
             break;
-          }
-          // The packet opens a leaf when any lane needs it and every lane tests its triangles, so a
-          // lane can end with a triangle outside its own radius.  Within mr is the mesh's exact
-          // value; beyond it the mesh cannot hold the minimum (its value is above d32 + delta, or
-          // below d32 - delta, which the minimum is not) and is left out.
-          if (mbt >= 0 && fabs(mb) <= double(mr)) {
-            best = fmin(best, mb);
           }
         }
         if (err) {
@@ -164,9 +183,9 @@ __global__ void __launch_bounds__(128, 4) kSceneBand64(const SceneQueryArgs a, f
 
 } // namespace
 
-cudaError_t launchSceneBand64(const SceneQueryArgs& a, float delta, int numSms, cudaStream_t s)
+cudaError_t launchSceneBand64(const SceneQueryArgs& a, int numSms, cudaStream_t s)
 {
-  kSceneBand64<<<unsigned(numSms * 4), 128, 0, s>>>(a, delta);
+  kSceneBand64<<<unsigned(numSms * 4), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 

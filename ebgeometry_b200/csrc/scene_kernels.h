@@ -15,8 +15,8 @@ struct alignas(16) SceneObject
 {
   int32_t kind;
   int32_t mesh;
-  float   radius;
-  float   pad;
+  float   radius;   // of a sphere; of a mesh the diagonal of its box
+  float   leaves;   // of a mesh: the number of its leaves
   float   t[3];
   float   R[9];
 };
@@ -67,6 +67,8 @@ struct SceneQueryArgs
   const uint32_t*     band_list;   // sorted positions needing FP64 (compacted from band_flag)
   const uint32_t*     band_count;
   unsigned long long* work;
+  float               delta;       // bound of the FP32 error of a value
+  int                 per;         // queries per packet (1 .. 32)
   int                 chunk;       // packets taken from the work counter at a time (0, 1: one)
   int*                status;
 };
@@ -97,7 +99,7 @@ int         sceneOuterDepth();
 cudaError_t launchSceneValue(const SceneQueryArgs& a, int numSms, cudaStream_t s);
 // FP64 re-evaluation of the band list (reads band_count on the device); delta bounds the FP32
 // error of the union's value.
-cudaError_t launchSceneBand64(const SceneQueryArgs& a, float delta, int numSms, cudaStream_t s);
+cudaError_t launchSceneBand64(const SceneQueryArgs& a, int numSms, cudaStream_t s);
 // Sort keys of a batched call: the 30-bit Morton code of every point of every batch, and the
 // identity.
 cudaError_t launchSceneBatchKeys(const SceneQueryArgs& a, uint32_t* keys, uint32_t* ids, cudaStream_t s);
