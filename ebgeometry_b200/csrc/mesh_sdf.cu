@@ -6,7 +6,11 @@
 // (strict <, MeshDistanceFunctionsImplem.hpp:480-509); interior -> box distances of the K
 // children, sorted far-to-near, pushed if d2 <= bound.
 //
-// Here one warp traverses a PACKET of 32 queries that were sorted along a Morton curve, so they
+// This is the walk for calls that want what only it has -- counters, radius hints, the shared-memory top
+// of the tree, the 8-wide copy, the closest triangles of an FP32 call -- and for meshes of fewer than 4,096
+// triangles; the other calls take a search per packet's box (mesh_packet.cu) or per point (mesh_point.cu).
+//
+// One warp traverses a PACKET of 32 queries that were sorted along a Morton curve, so they
 // are spatial neighbours:
 //  - the warp shares one stack in shared memory (entries carry the child box, so a popped entry is
 //    re-tested against every lane's current bound without touching global memory);

@@ -88,8 +88,11 @@ typedef struct ebg_query_opts
   int32_t            no_sort;         /* 1: keep the caller's point order (no Morton reordering) */
   int32_t            no_fp64_band;    /* 1: skip the FP64 near-surface re-evaluation */
   const ebg_seed*    seed;            /* learned pruning-radius model (NULL = plain traversal) */
-  int32_t            warps_per_block; /* 0 = tuned default */
-  int32_t            occupancy;       /* traversal register budget: 0 = default (= 1); 1, 2, 3 = at
+  int32_t            warps_per_block; /* 0 = tuned default.  This and occupancy shape the packet walk
+                                         (statistics, radius hints, top_nodes, the 8-wide tree, meshes
+                                         of fewer than 4,096 triangles, FP32 calls that ask for the
+                                         closest triangles); other calls fix their own */
+  int32_t            occupancy;       /* walk's register budget: 0 = default (= 1); 1, 2, 3 = at
                                          most 64, 51, 42 registers per thread (8, 10, 12 blocks of
                                          128 threads per SM; warps_per_block <= 4); 4 = the
                                          compiler's own choice with 256-thread blocks */
