@@ -239,7 +239,7 @@ def l2_read_bandwidth():
     return out.value if rc == 0 else None
 
 
-def traffic_from_csv(path, kernel="kMeshSdf32"):
+def traffic_from_csv(path, kernel="kMeshPacket32"):
     """DRAM bytes (read + write) per launch of `kernel`, averaged over the launches an ncu CSV
     (--metrics dram__bytes_read.sum,dram__bytes_write.sum --csv) recorded."""
     import csv
@@ -529,9 +529,10 @@ def run_ours(args, rank, world, local_rank):
     if rank != 0:
         return 0
 
-    # roofline of the traversal kernel (the launch timed as the "traverse" phase): the bytes its warps
-    # load per call, counted per packet from the measured run's own counters, over the phase's
-    # event-timed duration, against the measured HBM copy roof and the measured L2 read roof
+    # roofline of the FP32 search (the launches timed as the "traverse" phase): the bytes that a walk of
+    # the tree by packets loads per call, counted by the statistics entry point on the same queries (the
+    # timed kernel searches by packet boxes and loads less), over the phase's event-timed duration,
+    # against the measured HBM copy roof and the measured L2 read roof
     hbm_peak, peak_kind = measured_peaks()
     l2_gbs = l2_read_bandwidth()
     st_run = st_seed if seed is not None else st
@@ -615,23 +616,24 @@ def run_ours(args, rank, world, local_rank):
                      "frac": achieved / hbm_peak, "traffic": traffic, "peak_kind": peak_kind,
                      "traffic_source": (f"ncu capture {os.path.basename(args.traffic_csv)}" if traffic is not None
                                         else "none in this run (pass --traffic-csv from an ncu capture of it)"),
-                     "kernel": "kMeshSdf32 (FP32 packet traversal" + (", seeded)" if seed is not None else ")"),
+                     "kernel": "kMeshPacket32 (FP32 search by packet boxes" + (", seeded)" if seed is not None else ")"),
                      "bytes_per_query": bytes_call / nq,
-                     "bytes_basis": "per packet: 128 B per interior node opened + 64 B per oriented box + 48 B per "
+                     "bytes_basis": "of the packet walk of the same queries, per packet: 128 B per interior node opened + 64 B per oriented box + 48 B per "
                                     "triangle record of an opened leaf + 32 B per cut entry (+60 B per cut); per "
                                     "query: 12 B point + 4 B order + 4 B result + 96 B sign record",
                      "l2_read_gbs_measured": l2_gbs, "frac_of_l2": (achieved / l2_gbs) if l2_gbs else None,
-                     "limiter": "instruction issue and L1/L2 latency on the SMs (ncu: issue-active ~75 %, about "
-                                "2 eligible warps per cycle, L2 throughput a few %), not DRAM or L2 bandwidth",
+                     "limiter": "the L1's data stage and instruction issue on the SMs (ncu: LSU wavefronts 79 % of peak, "
+                                "issue-active 69 %), not DRAM or L2 bandwidth",
                      # the floor: every byte the step must touch once (the mesh's device arrays, the
                      # points in, the distances out) at the measured HBM rate
                      "unique_bytes_per_step": int(mesh.info["device_bytes"]) + 16 * n,
                      "unique_floor_ms": (int(mesh.info["device_bytes"]) + 16 * n) / (hbm_peak * 1e6)},
         "e2e": {"value": n * world / (e2e_ms * 1e-3), "unit": UNIT, "h2d_bytes_per_step": int(pts.nbytes),
                 "d2h_bytes_per_step": int(n * 4), "ms_per_step": e2e_ms, "matches_device_path": same},
-        "gpu_launches": 3 * args.steps,
-        "gpu_launches_note": "per step: Morton-key kernel, FP32 traversal, FP64 band pass (plus the CUB radix-sort "
-                             "and band-list compaction passes)",
+        "gpu_launches": 5 * args.steps,
+        "gpu_launches_note": "per step: Morton-key kernel, FP32 search by packets and of the points it lists, FP64 band "
+                             "pass by packets and of the queries it lists (plus the CUB radix-sort and "
+                             "band-list compaction passes)",
         "clocks": ck,
         "cpu_baseline": cpu,
     }
