@@ -480,12 +480,14 @@ template <int K>
 cudaError_t launchGridK(const GridQueryArgs& a, int numSms, cudaStream_t s)
 {
   const int64_t blocks = std::max<int64_t>(std::min<int64_t>((a.n + 127) / 128, int64_t(numSms) * 32), 1);
-  if (a.later == nullptr) {
+  if (K == 1 || a.later == nullptr) { // (k = 1 never has the list)
     kGridKnn<K, ALL><<<unsigned(blocks), 128, 0, s>>>(a);
     return cudaGetLastError();
   }
-  kGridKnn<K, FIRST><<<unsigned(blocks), 128, 0, s>>>(a);
-  kGridKnn<K, LATER><<<unsigned(blocks), 128, 0, s>>>(a);
+  if constexpr (K > 1) {
+    kGridKnn<K, FIRST><<<unsigned(blocks), 128, 0, s>>>(a);
+    kGridKnn<K, LATER><<<unsigned(blocks), 128, 0, s>>>(a);
+  }
   return cudaGetLastError();
 }
 
