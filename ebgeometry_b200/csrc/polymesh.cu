@@ -190,7 +190,8 @@ __device__ double polyFaceUd2(const PolyView& m, uint32_t f, P3 P)
 }
 
 // Whether a face under the disc may return a magnitude of at most `most` (rounded up, FP32) at p, which lies
-// `shift` from the FP64 point: the distance to the disc, less its rounding.
+// `shift` from the FP64 point: the distance to the disc, less its rounding.  Where the squared distance
+// overflows FP32 (beyond about 1.8e19) the disc says nothing, and the face is evaluated.
 __device__ __forceinline__ bool discReaches(const PolyDisc* __restrict__ disc, float px, float py, float pz, float most,
                                             float slack)
 {
@@ -200,7 +201,7 @@ __device__ __forceinline__ bool discReaches(const PolyDisc* __restrict__ disc, f
   const float  d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
   const float  u  = fmaxf(fabsf(s) - c.w, 0.f);
   const float  v  = fmaxf(sqrtf(fmaxf(fmaf(-s, s, d2 * 0.999999f), 0.f)) - n.w, 0.f);
-  return !(sqrtf(fmaf(u, u, v * v)) * 0.999996f - slack > most);
+  return !(d2 <= FLT_MAX) || !(sqrtf(fmaf(u, u, v * v)) * 0.999996f - slack > most);
 }
 
 // polyFaceSd with four lanes per face, an edge each (edges i, i + 4, ... on lane i of the four): the same
