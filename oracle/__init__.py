@@ -465,15 +465,20 @@ def ref_available() -> bool:
 _ref_timing_cache = None
 
 
+class ReferenceMissing(FileNotFoundError):
+    """The reference oracle's library is not built here (it needs the reference sources)."""
+
+
 def ref(timing: bool = False) -> _Ref:
     """The reference oracle: the parity build, or with ``timing`` the build bench.py times (see
-    ref_lib_path); both are the unmodified reference behind the same extern "C" harness."""
+    ref_lib_path); both are the unmodified reference behind the same extern "C" harness.  Raises
+    ReferenceMissing where it is not built; the tests are then skipped (tests/conftest.py)."""
     global _ref_cache, _ref_timing_cache
     cached = _ref_timing_cache if timing else _ref_cache
     if cached is None:
         path = ref_lib_path(timing)
         if not os.path.exists(path):
-            raise FileNotFoundError(f"{path} missing: run `make -C oracle ref` where the reference sources exist")
+            raise ReferenceMissing(f"{path} missing: run `make -C oracle ref` where the reference sources exist")
         cached = _Ref(path)
         if timing:
             _ref_timing_cache = cached
