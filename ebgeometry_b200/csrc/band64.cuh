@@ -185,60 +185,86 @@ __device__ double dcelFaceUd2(const double* __restrict__ tri, const double* __re
   return best;
 }
 
-// The triangle of smallest |d| in FP64 within `bound` of the FP32 point (px, py, pz), which lies
-// `shift` from P (strict <, MeshDistanceFunctionsImplem.hpp:492-502; ties
-// to the lower leaf position): all lanes on one point (mesh_point.cuh), whose FP32 distances select the
-// triangles worth an FP64 test.  `best` DBL_MAX and `bt` -1 if there is none.
-template <int EVAL, bool UPPER>
+// Whether an FP32 lower bound `low` of a triangle's distance leaves room for it within `reach`; dd its FP32
+// squared distance, from whose root `low` was made: too small a square has underflowed and says nothing.
+// (Not "low <= ...": a point on the triangle has no direction and a NaN bound.)
+__device__ __forceinline__ bool mayReach(float low, float dd, float reach) { return !(dd >= 1e-30f) || !(low > reach); }
+
+// The radius about the FP32 point, `shift` from the FP64 one, that holds an FP64 winner of value d.
+__device__ __forceinline__ float winnerRadius(double d, float shift)
+{
+  return (float(fabs(d)) + shift) * 1.000001f + 1e-30f;
+}
+
+// The triangle of smallest |d| in FP64 within `limit` (squared) of the FP32 point (px, py, pz), which lies
+// `shift` from P (strict <, MeshDistanceFunctionsImplem.hpp:492-502; ties to the lower leaf position): all
+// lanes on one point (mesh_point.cuh), whose FP32 distances shrink the bound and select the triangles worth
+// an FP64 test.  `best` DBL_MAX and `bt` -1 if there is none.
+//
+// FP32 distances can be too small by more than `delta`: those of needle-like triangles, or where squares
+// underflow.  A winner within the bound that the search ended with shows that they were not; without
+// one it runs again with bounds from FP64 values alone.  NEAREST: `limit` itself comes from such a
+// distance, and the nearest triangle is wanted however far it is.
+template <int EVAL, bool UPPER, bool NEAREST>
 __device__ int pointSearch64(const EbgMeshView& m, D3 P, float px, float py, float pz, float shift, float delta,
-                             float bound, double& best, int& bt, PointMem& w)
+                             float limit, double& best, int& bt, PointMem& w)
 {
   const float inf   = __int_as_float(0x7f800000);
-  const float slack = delta + 2.f * shift;
+  float       slack = delta + 2.f * shift, bound = limit;
+  int         err   = 0;
   best              = DBL_MAX;
   bt                = -1;
-  return pointSearch<UPPER>(m, px, py, pz, bound, slack, w, [&](bool active, uint32_t tri) {
-    float dd = inf, low = inf;
-    if (active) {
-      const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
-      const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-      float         s, t;
-      int           r;
-      dd  = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
-      low = triLower(h0, h1, h2, px, py, pz, s, t, dd);
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    err |= pointSearch<UPPER>(m, px, py, pz, bound, slack, w, [&](bool active, uint32_t tri) {
+      float dd = inf, low = inf;
+      if (active) {
+        const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
+        const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+        float         s, t;
+        int           r;
+        dd  = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
+        low = triLower(h0, h1, h2, px, py, pz, s, t, dd);
+      }
+      const float near = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(dd)));
+      const float rn   = (sqrtf(near) * 1.00001f + slack) * 1.000001f;
+      bound            = fminf(bound, rn * rn);
+      const bool cand  = active && mayReach(low, dd, sqrtf(bound) * 1.00001f + delta);
+      if (!__any_sync(FULL, cand)) {
+        return;
+      }
+      double d = DBL_MAX;
+      if (cand) {
+        d = EVAL == 0 ? triSd64(m.tri64 + 30 * size_t(tri), P)
+                      : dcelFaceSd(m.tri64 + 30 * size_t(tri), m.dcel_n + 3 * size_t(tri), P);
+      }
+      // the warp's least (|d|, triangle): non-negative doubles order like their words
+      const uint32_t hi = cand ? uint32_t(__double2hiint(fabs(d))) : 0xffffffffu;
+      const uint32_t mh = __reduce_min_sync(FULL, hi);
+      const uint32_t lo = hi == mh ? uint32_t(__double2loint(d)) : 0xffffffffu;
+      const uint32_t ml = __reduce_min_sync(FULL, lo);
+      const uint32_t ti = cand && hi == mh && lo == ml ? tri : 0xffffffffu;
+      const uint32_t mt = __reduce_min_sync(FULL, ti);
+      const unsigned who = __ballot_sync(FULL, ti == mt && cand);
+      if (mt == 0xffffffffu || who == 0u) {
+        return; // only NaN values
+      }
+      const double dm = __shfl_sync(FULL, d, __ffs(int(who)) - 1);
+      if (fabs(dm) < fabs(best) || (fabs(dm) == fabs(best) && int(mt) < bt)) {
+        best           = dm;
+        bt             = int(mt);
+        const float rb = winnerRadius(dm, shift);
+        bound          = fminf(bound, rb * rb);
+      }
+    });
+    const float rb = winnerRadius(best, shift);
+    if ((bt >= 0 && rb * rb <= bound) || (!NEAREST && bound == limit)) {
+      break;
     }
-    const float near = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(dd)));
-    const float rn   = (sqrtf(near) * 1.00001f + slack) * 1.000001f;
-    bound            = fminf(bound, rn * rn);
-    // (not "low <= ...": a point on the triangle has no direction and a NaN bound)
-    const bool cand = active && !(low > sqrtf(bound) * 1.00001f + delta);
-    if (!__any_sync(FULL, cand)) {
-      return;
-    }
-    double d = DBL_MAX;
-    if (cand) {
-      d = EVAL == 0 ? triSd64(m.tri64 + 30 * size_t(tri), P)
-                    : dcelFaceSd(m.tri64 + 30 * size_t(tri), m.dcel_n + 3 * size_t(tri), P);
-    }
-    // the warp's least (|d|, triangle): non-negative doubles order like their words
-    const uint32_t hi = cand ? uint32_t(__double2hiint(fabs(d))) : 0xffffffffu;
-    const uint32_t mh = __reduce_min_sync(FULL, hi);
-    const uint32_t lo = hi == mh ? uint32_t(__double2loint(d)) : 0xffffffffu;
-    const uint32_t ml = __reduce_min_sync(FULL, lo);
-    const uint32_t ti = cand && hi == mh && lo == ml ? tri : 0xffffffffu;
-    const uint32_t mt = __reduce_min_sync(FULL, ti);
-    const unsigned who = __ballot_sync(FULL, ti == mt && cand);
-    if (mt == 0xffffffffu || who == 0u) {
-      return; // only NaN values
-    }
-    const double dm = __shfl_sync(FULL, d, __ffs(int(who)) - 1);
-    if (fabs(dm) < fabs(best) || (fabs(dm) == fabs(best) && int(mt) < bt)) {
-      best           = dm;
-      bt             = int(mt);
-      const float rb = (float(fabs(dm)) + shift) * 1.000001f + 1e-30f;
-      bound          = fminf(bound, rb * rb);
-    }
-  });
+    slack = inf; // shrinks nothing
+    bound = NEAREST ? (bt >= 0 ? rb * rb : FLT_MAX) : limit;
+  }
+  return err;
 }
 
 } // namespace

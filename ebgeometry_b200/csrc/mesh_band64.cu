@@ -8,8 +8,10 @@
 // (outward-rounded) box lies within |d32| + delta of the point, keeping the value of smallest
 // magnitude with strict < (MeshDistanceFunctionsImplem.hpp:492-502).  delta covers the FP32
 // distance error, so the FP64 winner is never pruned; leaves and nodes are also pruned by their
-// oriented boxes, which bound the exact distance to every triangle inside from below.  An FP64 call
-// evaluates all its queries here, with FP32 distances that only bound the search.
+// oriented boxes, which bound the exact distance to every triangle inside from below.  Of needle-like
+// triangles an FP32 distance can be too small by more than delta: a winner outside the radius, or none,
+// shows it, and the query is searched again with the winner's own distance (none: without a bound).
+// An FP64 call evaluates all its queries here, with FP32 distances that only bound the search.
 //
 // Bound by the L1's wavefronts and the FP64 pipe together: an FP64 test is about 200 instructions at
 // half rate, so it is spent only on triangles whose FP32 lower bound (triLower) reaches the radius --
@@ -86,8 +88,7 @@ __device__ __forceinline__ void bandStore(const MeshQueryArgs& a, const EbgMeshV
 }
 
 // Whether a triangle may hold the FP64 winner of a query with squared bound `bound`: its lower bound
-// in FP32 from the closest point that triDist2 finds.  (Not "triLower <= ...": a point on the triangle
-// has no direction and a NaN bound.)
+// in FP32 from the closest point that triDist2 finds.
 __device__ __forceinline__ bool bandCandidate(const EbgMeshView& m, uint32_t tt, float px, float py, float pz, float bound,
                                               float delta)
 {
@@ -96,7 +97,7 @@ __device__ __forceinline__ bool bandCandidate(const EbgMeshView& m, uint32_t tt,
   float         s, t;
   int           r;
   const float   dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
-  return !(triLower(h0, h1, h2, px, py, pz, s, t, dd) > sqrtf(bound) * 1.00001f + delta);
+  return mayReach(triLower(h0, h1, h2, px, py, pz, s, t, dd), dd, sqrtf(bound) * 1.00001f + delta);
 }
 
 // Eight lanes per band query (groupSearch), from the root with the query's own bound: the queries of the
@@ -151,27 +152,40 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 6) kMeshBandGroups(const __gr
       if (n > 0 && fabs(d) < DBL_MAX && (fabs(d) < fabs(best) || (fabs(d) == fabs(best) && tt < bt))) {
         best           = d;
         bt             = tt;
-        const float rb = (float(fabs(d)) + shift) * 1.000001f + 1e-30f; // at the FP32 point
+        const float rb = winnerRadius(d, shift);
         bound          = fminf(bound, rb * rb);
       }
       __syncwarp(); // read before more are appended
     };
-    const int err = groupSearch<false>(m, on, px, py, pz, bound, 0.f, w.g, [&](bool, uint32_t t0, int cnt, int most) {
-      for (int t = sub; t - sub < most; t += 8) {
-        const bool     cand = t < cnt && bandCandidate(m, t0 + uint32_t(t), px, py, pz, bound, delta);
-        const unsigned mk = (__ballot_sync(FULL, cand) >> base) & 0xffu;
-        if (cand) {
-          w.cand[nc + __popc(mk & ((1u << sub) - 1u))] = t0 + uint32_t(t);
+    int  err  = 0;
+    bool todo = on;
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+      err |= groupSearch<false>(m, todo, px, py, pz, bound, 0.f, w.g, [&](bool, uint32_t t0, int cnt, int most) {
+        for (int t = sub; t - sub < most; t += 8) {
+          const bool     cand = t < cnt && bandCandidate(m, t0 + uint32_t(t), px, py, pz, bound, delta);
+          const unsigned mk = (__ballot_sync(FULL, cand) >> base) & 0xffu;
+          if (cand) {
+            w.cand[nc + __popc(mk & ((1u << sub) - 1u))] = t0 + uint32_t(t);
+          }
+          nc += __popc(mk);
+          __syncwarp();
+          if (__any_sync(FULL, nc >= BAND_CAND - 8)) {
+            evaluate();
+          }
         }
-        nc += __popc(mk);
-        __syncwarp();
-        if (__any_sync(FULL, nc >= BAND_CAND - 8)) {
-          evaluate();
-        }
+      });
+      while (__any_sync(FULL, nc > 0)) {
+        evaluate();
       }
-    });
-    while (__any_sync(FULL, nc > 0)) {
-      evaluate();
+      const float rb = winnerRadius(best, shift);
+      todo           = todo && !(bt >= 0 && rb <= r);
+      if (!__any_sync(FULL, todo)) {
+        break;
+      }
+      if (todo) {
+        bound = bt >= 0 ? rb * rb : FLT_MAX;
+      }
     }
     if (on && sub == 0) {
       if (err) {
@@ -206,7 +220,8 @@ struct BandPacketMem
 // most the distance to a point of one of them; the tighter of the two bounds goes to the corners.
 // The (query, leaf) pairs left are tested a lane each in FP32, and only triangles whose FP32 lower
 // bound is within the radius are evaluated in FP64, 32 candidates at a time.  A packet too wide or
-// with too many leaves in reach leaves its queries to kMeshBandGroups.
+// with too many leaves in reach leaves its queries to kMeshBandGroups, as a query does whose radius did not
+// hold its winner.
 template <int EVAL>
 __global__ void __launch_bounds__(32 * BAND_WARPS, 6) kMeshBand64(const __grid_constant__ MeshQueryArgs a, float delta,
                                                                   float split)
@@ -300,7 +315,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 6) kMeshBand64(const __grid_c
             if (fabs(d) < DBL_MAX && (fabs(d) < fabs(best) || (fabs(d) == fabs(best) && t < bt))) {
               best           = d;
               bt             = t;
-              const float rb = (float(fabs(d)) + shift) * 1.000001f + 1e-30f; // at the FP32 point
+              const float rb = winnerRadius(d, shift);
               bound          = fminf(bound, rb * rb);
             }
           }
@@ -419,19 +434,18 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 6) kMeshBand64(const __grid_c
     if (err && lane == 0) {
       atomicOr(a.status, err);
     }
-    if (ok) {
-      if (on) {
-        bandStore(a, m, id, d32, best, bt);
-      }
+    ok = ok && bt >= 0 && winnerRadius(best, shift) <= r;
+    if (on && ok) {
+      bandStore(a, m, id, d32, best, bt);
     }
-    else {
+    const unsigned mk = __ballot_sync(FULL, on && !ok);
+    if (mk != 0u) {
       uint32_t at = 0;
-      const unsigned mk = __ballot_sync(FULL, on);
       if (lane == 0) {
         at = atomicAdd(a.later_count, uint32_t(__popc(mk)));
       }
       at = __shfl_sync(FULL, at, 0);
-      if (on) {
+      if (on && !ok) {
         a.later[at + __popc(mk & lt)] = j;
       }
     }

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(32 * POINT_WARPS, F64 ? 5 : 8) kMeshPoint(cons
     double       best = DBL_MAX;
     int          bt   = -1, err;
     if (F64) {
-      err = pointSearch64<EVAL, true>(m, P, px, py, pz, shift, delta, FLT_MAX, best, bt, w);
+      err = pointSearch64<EVAL, true, true>(m, P, px, py, pz, shift, delta, FLT_MAX, best, bt, w);
       if (lane == 0) {
         a.out_d64[id] = bt >= 0 ? best : double(FLT_MAX);
         if (a.out_tri) {
@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(32 * POINT_WARPS, F64 ? 5 : 8) kMeshPoint(cons
       if (band64 && bt >= 0 && fabsf(dist) <= a.band) {
         const float r = (fabsf(dist) * 1.00001f + delta) * 1.000001f;
         int         b64;
-        err |= pointSearch64<0, false>(m, P, px, py, pz, 0.f, delta, r * r, best, b64, w);
+        err |= pointSearch64<0, false, true>(m, P, px, py, pz, 0.f, delta, r * r, best, b64, w);
         if (b64 >= 0) {
           dist = float(best);
           tri  = b64;

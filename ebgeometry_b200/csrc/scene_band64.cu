@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128, 4) kSceneBand64(const SceneQueryArgs a)
             const D3  Ll = {__shfl_sync(FULL, L.x, l), __shfl_sync(FULL, L.y, l), __shfl_sync(FULL, L.z, l)};
             double    mb;
             int       mbt;
-            err |= pointSearch64<0, false>(mv, Ll, float(Ll.x), float(Ll.y), float(Ll.z), __shfl_sync(FULL, shift, l),
+            err |= pointSearch64<0, false, false>(mv, Ll, float(Ll.x), float(Ll.y), float(Ll.z), __shfl_sync(FULL, shift, l),
                                            delta, __shfl_sync(FULL, bound, l), mb, mbt, w);
             // Within mr is the mesh's exact value; beyond it (a leaf in reach is tested as a whole) the
             // mesh cannot hold the minimum (its value is above d32 + delta, or below d32 - delta, which
