@@ -49,35 +49,12 @@ namespace {
 constexpr int PACKET_WARPS = 4;
 constexpr int PACKET_PAIRS = 256; // (lane, leaf) pairs waiting for their triangle tests
 
-// The nearest triangle of one point (all lanes on the same point), or with FIRST a near one.
-template <bool FIRST>
-__device__ __noinline__ int pointNearest32(const EbgMeshView& m, float px, float py, float pz, float delta, PointMem& w,
-                                           float& bd2, int& bt)
+// A mesh triangle near a point (all lanes on the same point; -1 if none is found).
+__device__ __noinline__ int nearTriangle(const EbgMeshView& m, float px, float py, float pz, float delta, PointMem& w, int& bt)
 {
-  const float inf   = __int_as_float(0x7f800000);
-  float       bound = FLT_MAX, b = inf;
-  int         t = -1;
-  const int   err = pointSearch<true, FIRST>(m, px, py, pz, bound, delta, w, [&](bool active, uint32_t tri) {
-    float dd = inf;
-    if (active) {
-      const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
-      const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-      float         s_, t_;
-      int           r_;
-      dd = triDist2<false>(h0, h1, h2, px, py, pz, s_, t_, r_);
-    }
-    const uint32_t mb = __reduce_min_sync(FULL, __float_as_uint(dd));
-    const uint32_t mt = __reduce_min_sync(FULL, __float_as_uint(dd) == mb ? tri : 0x7fffffffu);
-    const float    md = __uint_as_float(mb);
-    if (md < b || (md == b && int(mt) < t)) {
-      b     = md;
-      t     = int(mt);
-      bound = fminf(bound, b);
-    }
-  });
-  bd2 = b;
-  bt  = t;
-  return err;
+  float bd2 = FLT_MAX;
+  bt        = -1;
+  return pointNearest<true>(m, px, py, pz, delta, w, bd2, bt);
 }
 
 constexpr int PACKET_FRONT = 32; // entries of a group's frontier
@@ -250,13 +227,12 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
       __syncwarp();
       limit = numPackets - pk > gridDim.x * (8ull * PACKET_WARPS) ? 32 : 12;
       if (got) {
-        float bd2;
-        int   err = 0;
+        int err = 0;
         if (CELLS) {
           besttri = cellAnchor(a.cells, qx, qy, qz);
         }
         if (besttri < 0) {
-          err = pointNearest32<true>(m, qx, qy, qz, delta, w, bd2, besttri);
+          err = nearTriangle(m, qx, qy, qz, delta, w, besttri);
         }
         if (err && lane == 0) {
           atomicOr(a.status, err);
@@ -353,9 +329,7 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
         const float4   last = pm.last;
         if (!__any_sync(FULL, own >= 0) && fmaxf(fabsf(r.cx - last.x), fmaxf(fabsf(r.cy - last.y), fabsf(r.cz - last.z))) > 4.f * (hm + last.w)) {
           // a step of the ordering to somewhere else: those winners are far from nearest here
-          float bd2;
-          err |= pointNearest32<true>(m, __shfl_sync(FULL, px, b), __shfl_sync(FULL, py, b), __shfl_sync(FULL, pz, b), delta, w,
-                                bd2, cand);
+          err |= nearTriangle(m, __shfl_sync(FULL, px, b), __shfl_sync(FULL, py, b), __shfl_sync(FULL, pz, b), delta, w, cand);
         }
         const unsigned have = __ballot_sync(FULL, cand >= 0);
         const int      alt  = __shfl_sync(FULL, cand, have ? __ffs(int(have)) - 1 : 0);

@@ -32,7 +32,6 @@ __global__ void __launch_bounds__(32 * POINT_WARPS, F64 ? 5 : 8) kMeshPoint(cons
   PointMem&           w    = mem[threadIdx.x >> 5];
   const int           lane = threadIdx.x & 31;
   const int64_t       nW   = int64_t(gridDim.x) * POINT_WARPS;
-  const float         inf  = __int_as_float(0x7f800000);
   for (int64_t id = int64_t(blockIdx.x) * POINT_WARPS + (threadIdx.x >> 5); id < a.n; id += nW) {
     D3    P;
     float px, py, pz;
@@ -73,26 +72,8 @@ __global__ void __launch_bounds__(32 * POINT_WARPS, F64 ? 5 : 8) kMeshPoint(cons
       }
     }
     else {
-      float bound = FLT_MAX, bd2 = inf;
-      err = pointSearch<true>(m, px, py, pz, bound, delta, w, [&](bool active, uint32_t tri) {
-        float dd = inf;
-        if (active) {
-          const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
-          const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-          float         s, t;
-          int           r;
-          dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
-        }
-        // ties go to the lower leaf position, as in the packet traversal
-        const uint32_t mb = __reduce_min_sync(FULL, __float_as_uint(dd));
-        const uint32_t mt = __reduce_min_sync(FULL, __float_as_uint(dd) == mb ? tri : 0x7fffffffu);
-        const float    md = __uint_as_float(mb);
-        if (md < bd2 || (md == bd2 && int(mt) < bt)) {
-          bd2   = md;
-          bt    = int(mt);
-          bound = fminf(bound, bd2);
-        }
-      });
+      float bd2  = FLT_MAX;
+      err        = pointNearest(m, px, py, pz, delta, w, bd2, bt);
       float dist = bt >= 0 ? signedFromWinner(m, uint32_t(bt), px, py, pz) : FLT_MAX;
       int   tri  = bt;
       if (band64 && bt >= 0 && fabsf(dist) <= a.band) {

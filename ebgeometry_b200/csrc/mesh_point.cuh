@@ -193,6 +193,47 @@ __device__ __forceinline__ int pointSearch(const EbgMeshView& m, float px, float
   return 0;
 }
 
+// The nearest triangle (FP32, ties to the lower leaf position, as in the packet traversal) of one point among
+// those nearer than the root of bd2; bt stays as it is if there is none.  FIRST as for pointSearch.
+// The boxes' upper bounds hold for exact distances.  Where every FP32 distance is above them by more than
+// `slack` (squares that underflow, triangles that FP32 cannot tell from a line) the search runs again
+// without them.
+template <bool FIRST = false>
+__device__ __forceinline__ int pointNearest(const EbgMeshView& m, float px, float py, float pz, float slack, PointMem& w,
+                                            float& bd2, int& bt)
+{
+  const float inf   = __int_as_float(0x7f800000);
+  float       bound = bd2;
+  int         err   = 0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    err |= pointSearch<true, FIRST>(m, px, py, pz, bound, slack, w, [&](bool active, uint32_t tri) {
+      float dd = inf;
+      if (active) {
+        const float4* h  = reinterpret_cast<const float4*>(m.hot + tri);
+        const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+        float         s, t;
+        int           r;
+        dd = triDist2<false>(h0, h1, h2, px, py, pz, s, t, r);
+      }
+      const uint32_t mb = __reduce_min_sync(FULL, __float_as_uint(dd));
+      const uint32_t mt = __reduce_min_sync(FULL, __float_as_uint(dd) == mb ? tri : 0x7fffffffu);
+      const float    md = __uint_as_float(mb);
+      if (md < bd2 || (md == bd2 && int(mt) < bt)) {
+        bd2   = md;
+        bt    = int(mt);
+        bound = fminf(bound, bd2);
+      }
+    });
+    if (FIRST || bound >= bd2) {
+      break;
+    }
+    slack = inf; // shrinks nothing
+    bound = bd2;
+  }
+  return err;
+}
+
 // ---- eight lanes per point ---------------------------------------------------------------------------
 //
 // With more points than warps the 32 lanes of pointSearch are too many for one point: most rounds
@@ -321,41 +362,50 @@ __device__ __forceinline__ int groupSearch(const EbgMeshView& m, bool on, float 
   }
 }
 
-// The nearest triangle (FP32, ties to the lower leaf position) of each group's point.
+// The nearest triangle of each group's point, as pointNearest finds it.
 __device__ __forceinline__ int groupNearest(const EbgMeshView& m, bool on, float px, float py, float pz, float slack,
                                             GroupMem& g, float& bd2, int& bt)
 {
   const int   sub   = threadIdx.x & 7;
   const float inf   = __int_as_float(0x7f800000);
-  float       bound = FLT_MAX, b = inf;
-  int         best  = -1;
-  const int   err   = groupSearch<true>(m, on, px, py, pz, bound, slack, g, [&](bool test, uint32_t t0, int cnt, int most) {
-    float dd  = inf;
-    int   tri = 0x7fffffff;
-    for (int t = sub; t < most; t += 8) {
-      if (t < cnt) {
-        const float4* h  = reinterpret_cast<const float4*>(m.hot + t0 + t);
-        const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-        float         s_, t_;
-        int           r_;
-        const float   d = triDist2<false>(h0, h1, h2, px, py, pz, s_, t_, r_);
-        if (d < dd) {
-          dd  = d;
-          tri = int(t0) + t;
+  float       bound = FLT_MAX, b = FLT_MAX;
+  int         best  = -1, err = 0;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; pass++) {
+    err |= groupSearch<true>(m, on, px, py, pz, bound, slack, g, [&](bool test, uint32_t t0, int cnt, int most) {
+      float dd  = inf;
+      int   tri = 0x7fffffff;
+      for (int t = sub; t < most; t += 8) {
+        if (t < cnt) {
+          const float4* h  = reinterpret_cast<const float4*>(m.hot + t0 + t);
+          const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
+          float         s_, t_;
+          int           r_;
+          const float   d = triDist2<false>(h0, h1, h2, px, py, pz, s_, t_, r_);
+          if (d < dd) {
+            dd  = d;
+            tri = int(t0) + t;
+          }
         }
       }
+      const float dm = groupMin(dd);
+      tri            = dd == dm ? tri : 0x7fffffff;
+      tri            = min(tri, __shfl_xor_sync(FULL, tri, 1));
+      tri            = min(tri, __shfl_xor_sync(FULL, tri, 2));
+      tri            = min(tri, __shfl_xor_sync(FULL, tri, 4));
+      if (test && (dm < b || (dm == b && tri < best))) {
+        b     = dm;
+        best  = tri;
+        bound = fminf(bound, b);
+      }
+    });
+    on = on && bound < b;
+    if (!__any_sync(FULL, on)) {
+      break;
     }
-    const float dm = groupMin(dd);
-    tri            = dd == dm ? tri : 0x7fffffff;
-    tri            = min(tri, __shfl_xor_sync(FULL, tri, 1));
-    tri            = min(tri, __shfl_xor_sync(FULL, tri, 2));
-    tri            = min(tri, __shfl_xor_sync(FULL, tri, 4));
-    if (test && (dm < b || (dm == b && tri < best))) {
-      b     = dm;
-      best  = tri;
-      bound = fminf(bound, b);
-    }
-  });
+    slack = inf; // shrinks nothing
+    bound = b;
+  }
   bd2 = b;
   bt  = best;
   return err;

@@ -143,28 +143,9 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
             for (unsigned rest = who; rest != 0u; rest &= rest - 1) {
               const int   l = __ffs(int(rest)) - 1;
               const float x = __shfl_sync(FULL, lx, l), y = __shfl_sync(FULL, ly, l), z = __shfl_sync(FULL, lz, l);
-              float       bd2 = __shfl_sync(FULL, mb, l), bound = bd2;
+              float       bd2 = __shfl_sync(FULL, mb, l);
               int         tb  = -1;
-              err |= pointSearch<true>(mv, x, y, z, bound, a.delta, *reinterpret_cast<PointMem*>(istk),
-                                       [&](bool active, uint32_t tri) {
-                float dd = inf;
-                if (active) {
-                  const float4* h  = reinterpret_cast<const float4*>(mv.hot + tri);
-                  const float4  h0 = __ldg(h), h1 = __ldg(h + 1), h2 = __ldg(h + 2);
-                  float         s_, t_;
-                  int           r_;
-                  dd = triDist2<false>(h0, h1, h2, x, y, z, s_, t_, r_);
-                }
-                // ties go to the lower leaf position, as in the packet traversal
-                const uint32_t m0 = __reduce_min_sync(FULL, __float_as_uint(dd));
-                const uint32_t mt = __reduce_min_sync(FULL, __float_as_uint(dd) == m0 ? tri : 0x7fffffffu);
-                const float    md = __uint_as_float(m0);
-                if (md < bd2 || (md == bd2 && int(mt) < tb)) {
-                  bd2   = md;
-                  tb    = int(mt);
-                  bound = fminf(bound, bd2);
-                }
-              });
+              err |= pointNearest(mv, x, y, z, a.delta, *reinterpret_cast<PointMem*>(istk), bd2, tb);
               bt = lane == l ? tb : bt;
             }
           }

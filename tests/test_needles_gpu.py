@@ -50,3 +50,17 @@ def test_fp64_against_exhaustive(name, n):
     width = float(name[6:10]) if name.startswith("needle") else 1.0
     t = TriMeshSDF(v, f).signed_distance(pd).abs()
     assert ((t - ref).abs() <= (np.abs(v).max() + size) * 1e-14 / width).all()
+
+
+@pytest.mark.parametrize("n", [3000, 70001])
+@pytest.mark.parametrize("scale", [1e-20, 1e-25])
+def test_fp32_of_tiny_meshes_finds_a_triangle(scale, n):
+    """FP32 squares of these distances underflow: every point still gets the distance of some triangle near
+    it, within the distance to the farthest corner of the mesh's box."""
+    v, f = W.displaced_icosphere(5, 5)
+    m = TriMeshSDF(v * scale, f)
+    for reach in (1.5, 1e4):
+        p = torch.from_numpy((W.uniform_points(n, n, -reach, reach) * np.float32(scale)).astype(np.float32)).cuda()
+        d = m.signed_distance(p)
+        m.check_status()
+        assert (d.abs() <= 1.001 * (p.double().norm(dim=1) + 2.0 * scale) + 2e-23).all()
