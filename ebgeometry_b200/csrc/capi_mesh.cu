@@ -500,11 +500,12 @@ struct Workspace
 // line lies where the least favourable measured input still gains: 65,536 points within 1e-3 of a
 // 1,280-triangle surface take 157 us against the packets' 220 us (262,144 of them 580 against 238 us);
 // uniform points gain up to 0.25-1 M (65,536 on 1.3 M triangles: 0.45 against 6.8 ms).  Counters, phase
-// times and the options of the packet traversal keep the packets.
+// times and the options of the packet traversal keep the packets, and so do FP32 calls that ask for the
+// closest triangles (fp32Triangles; see launchMeshFp32).
 constexpr int64_t POINT_CALL = 65536;
-bool pointPath(int64_t n, const ebg_query_opts* opts, const unsigned long long* statsDev, bool triLeafOrder)
+bool pointPath(int64_t n, const ebg_query_opts* opts, const unsigned long long* statsDev, bool fp32Triangles)
 {
-  return n <= POINT_CALL && statsDev == nullptr && !triLeafOrder &&
+  return n <= POINT_CALL && statsDev == nullptr && !fp32Triangles &&
          !(opts && (opts->timings || opts->top_nodes > 0 || opts->node_width > 0));
 }
 
@@ -522,8 +523,9 @@ float ebg::packetSplit(const ebg_mesh* m)
 //  - meshes of fewer than 4,096 triangles, whose walk is short (4 M points on 1,280 triangles: 0.37
 //    against 0.48 ms near the surface, 0.92 against 0.94 ms everywhere; on 5,120 triangles 1.9 against
 //    1.8 ms everywhere);
-//  - FP32 calls that ask for the closest triangles: of triangles at exactly the same distance the walk
-//    names the one that its order and box rounding leave (2 points of 8 M differed).
+//  - FP32 calls that ask for the closest triangles: of triangles at the same distance the walk names the
+//    one that its order and box rounding leave, another search another one (6 of 20,000 points on and far
+//    from the surface, 2 of 8 M uniform ones).
 cudaError_t ebg::launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool fp32Triangles, int wpb, int occ,
                                 float delta, cudaStream_t s)
 {
@@ -553,6 +555,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   const bool sort   = !(opts && opts->no_sort);
   // an FP64 result re-evaluates every query in FP64 (the band covers all distances)
   const bool fp64all = out64 != nullptr;
+  const bool fp32Tri = outTri != nullptr && !fp64all;
   const bool band64  = fp64all || !(opts && opts->no_fp64_band);
   const int  wpb    = (opts && opts->warps_per_block > 0) ? opts->warps_per_block
                                                           : (m->tunedWpb > 0 ? m->tunedWpb : 4);
@@ -576,7 +579,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   }
   const int width = seed ? 4 : (askedWidth ? askedWidth : (m->tunedWidth == 8 && m->hasWide ? 8 : 4));
 
-  if (pts == nullptr || pointPath(n, opts, statsDev, triLeafOrder)) {
+  if (pts == nullptr || pointPath(n, opts, statsDev, fp32Tri)) {
     MeshQueryArgs a{};
     a.mesh     = m->view;
     a.points   = pts;
@@ -713,7 +716,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     a.out_tri  = tri32;
     a.tri_leaf = 1;
   }
-  if (launchMeshFp32(m, a, outTri != nullptr && !fp64all, wpb, occ, delta, s) != cudaSuccess) {
+  if (launchMeshFp32(m, a, fp32Tri, wpb, occ, delta, s) != cudaSuccess) {
     return setError(EBG_ERR_CUDA, std::string("traversal launch failed: ") + cudaGetErrorString(cudaGetLastError()));
   }
   a.out_tri    = outTri;

@@ -18,7 +18,7 @@ namespace {
 constexpr int POINT_WARPS = 4;
 
 // F64: FP64 points and results with evaluator EVAL (0 the Triangle test, 1 the DCEL face).  Else
-// FP32 points and results: the FP32 search, and the FP64 one where |d| is within the band.
+// FP32 points and distances (no triangles): the FP32 search, and the FP64 one where |d| is within the band.
 // Bound by the latency of its dependent loads (two per tree level and two per leaf batch), so the
 // FP32 form keeps 32 queries in flight per SM at the cost of a few spills in its rare FP64 part.
 // B200, 20,480 triangles, uniform points, packet path before -> now: 1 point 166 -> 15 us, 32 points
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(32 * POINT_WARPS, F64 ? 5 : 8) kMeshPoint(cons
         else {
           a.out_d[id] = FLT_MAX;
         }
-        if (a.out_tri) {
+        if (F64 && a.out_tri) {
           a.out_tri[id] = -1;
         }
       }
@@ -75,21 +75,14 @@ __global__ void __launch_bounds__(32 * POINT_WARPS, F64 ? 5 : 8) kMeshPoint(cons
       float bd2  = FLT_MAX;
       err        = pointNearest(m, px, py, pz, delta, w, bd2, bt);
       float dist = bt >= 0 ? signedFromWinner(m, uint32_t(bt), px, py, pz) : FLT_MAX;
-      int   tri  = bt;
       if (band64 && bt >= 0 && fabsf(dist) <= a.band) {
         const float r = (fabsf(dist) * 1.00001f + delta) * 1.000001f;
         int         b64;
         err |= pointSearch64<0, false, true>(m, P, px, py, pz, 0.f, delta, r * r, best, b64, w);
-        if (b64 >= 0) {
-          dist = float(best);
-          tri  = b64;
-        }
+        dist = b64 >= 0 ? float(best) : dist;
       }
       if (lane == 0) {
         a.out_d[id] = dist;
-        if (a.out_tri) {
-          a.out_tri[id] = tri >= 0 ? __ldg(m.tri_id + tri) : -1;
-        }
       }
     }
     if (err && lane == 0) {
