@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
     }
     const int64_t  pos   = int64_t(pk) * a.per + lane;
     const bool     valid = lane < a.per && pos < a.n;
-    const int64_t  src   = pos < a.n ? pos : a.n - 1;
+    const int64_t  src   = valid ? pos : int64_t(pk) * a.per; // (lanes without a query decide nothing)
     const uint32_t id    = a.order ? __ldg(a.order + src) : uint32_t(src);
     float*         outp  = nullptr;
     const float*   pp    = scenePoint(a, id, &outp);
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
       --sp;
       const float4 A = ostk[2 * sp], B = ostk[2 * sp + 1];
       const float  bb = fmaxf(best, 0.f);
-      const float  bound = bb * bb;
+      const float  bound = valid ? bb * bb : -1.f;
       const float  d2 = boxDist2(A.x, A.y, A.z, B.x, B.y, B.z, px, py, pz);
       if (!__any_sync(FULL, d2 <= bound)) {
         continue;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
         for (int k = 0; k < 4; k++) {
           const float dk = boxDist2(nd.lox[k], nd.loy[k], nd.loz[k], nd.hix[k], nd.hiy[k], nd.hiz[k], px, py, pz);
           const bool  nk = __any_sync(FULL, dk <= bound) && (nd.child[k] | nd.count[k]) != 0u;
-          key[k]         = nk ? __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(dk))) : -1.f;
+          key[k]         = nk ? __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(valid ? dk : FLT_MAX))) : -1.f;
         }
         const int np = int(key[0] >= 0.f) + int(key[1] >= 0.f) + int(key[2] >= 0.f) + int(key[3] >= 0.f);
         if (sp + np > OUTER_DEPTH) {

@@ -59,16 +59,16 @@ __global__ void __launch_bounds__(128, 4) kSceneBand64(const SceneQueryArgs a)
   for (uint32_t pk = warpId; pk < numPk; pk += nWarps) {
     const uint32_t j     = pk * per + lane;
     const bool     valid = lane < int(per) && j < count;
-    const uint32_t pos   = a.band_list[valid ? j : count - 1];
+    const uint32_t pos   = a.band_list[valid ? j : pk * per]; // (an entry of this warp's: others are being written)
     const uint32_t id    = a.order ? a.order[pos] : pos;
     float*         outp  = nullptr;
     const float*   pp    = scenePoint(a, id, &outp);
     const float    px = pp[0], py = pp[1], pz = pp[2];
     const D3       P     = {double(px), double(py), double(pz)};
     const float    d32   = *outp; // the FP32 pass's union value
-    // objects whose box is farther than d32 + delta cannot hold the minimum
+    // objects whose box is farther than d32 + delta cannot hold the minimum (lanes without a query: none can)
     const float    ob    = fmaxf(d32 + delta, 0.f) * 1.00001f;
-    const float    obound = ob * ob;
+    const float    obound = valid ? ob * ob : -1.f;
     // a mesh that can hold the minimum has |value| <= |d32| + delta
     const float    mr    = (fabsf(d32) * 1.00001f + delta) * 1.000001f;
     double         best  = CUDART_INF;
