@@ -127,18 +127,24 @@ __global__ void __launch_bounds__(128) kSceneValue(const SceneQueryArgs a)
           if (who == 0u) {
             continue;
           }
-          const float inf = __int_as_float(0x7f800000);
-          const float ex = warpMax(need ? lx : -inf) - warpMin(need ? lx : inf);
-          const float ey = warpMax(need ? ly : -inf) - warpMin(need ? ly : inf);
-          const float ez = warpMax(need ? lz : -inf) - warpMin(need ? lz : inf);
           // The packet opens about as many leaves as lie within the span of its points' nearest points: of
           // all leaves (span / diagonal)^2, the span shrinking from the points' extent with their distance
           // from the mesh.  A leaf costs the packet about what the rounds of one query's own search cost per
           // sixth of it.  1024 spheres and 48 meshes, 2 M points, limits of 1, 2, 4, 6, 8 and 12 leaves per
           // query: 2267, 2205, 2127, 2122, 2604 and 3190 us; the meshes alone: 6878, 6244, 5815, 5642,
-          // 5544 and 5482 (packets only 5950).  Up to two queries never make a packet.
-          const float far = ob.radius + 3.f * sqrtf(warpMin(need ? bd : inf));
-          if (fmaf(ex, ex, fmaf(ey, ey, ez * ez)) * ob.leaves >= (6.f * float(__popc(who)) - 12.f) * far * far) {
+          // 5544 and 5482 (packets only 5950).  Up to two queries never make a packet; a mesh of no
+          // more leaves than the limit always does (2 M points on 2,000 meshes of 320 and 1,280 triangles).
+          const float limit    = 6.f * float(__popc(who)) - 12.f;
+          bool        separate = ob.leaves >= limit;
+          if (separate) {
+            const float inf = __int_as_float(0x7f800000);
+            const float ex = warpMax(need ? lx : -inf) - warpMin(need ? lx : inf);
+            const float ey = warpMax(need ? ly : -inf) - warpMin(need ? ly : inf);
+            const float ez = warpMax(need ? lz : -inf) - warpMin(need ? lz : inf);
+            const float far = ob.radius + 3.f * sqrtf(warpMin(need ? bd : inf));
+            separate        = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) * ob.leaves >= limit * far * far;
+          }
+          if (separate) {
 #pragma unroll 1
             for (unsigned rest = who; rest != 0u; rest &= rest - 1) {
               const int   l = __ffs(int(rest)) - 1;
