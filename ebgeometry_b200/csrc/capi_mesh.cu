@@ -531,7 +531,7 @@ cudaError_t ebg::launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool 
 {
   if (a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && a.node_width != 8 && !fp32Triangles &&
       m->info.num_triangles >= 4096) {
-    return launchMeshPacket32(a, delta, packetSplit(m), m->info.num_leaves, m->numSms, s);
+    return launchMeshPacket32(a, delta, packetSplit(m), float(m->info.diagonal), m->info.num_leaves, m->numSms, s);
   }
   return launchMeshSdf32(a, wpb, m->numSms, s, occ);
 }
@@ -654,8 +654,8 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     later     = ws.get<uint32_t>(n);
   }
   int32_t* tri32 = fp64all ? ws.get<int32_t>(n) : nullptr;
-  unsigned long long* counters = ws.get<unsigned long long>(3); // [0] packets, [1] band and point list
-                                                                             // counts (u32), [2] FP64 leftovers (u32)
+  // [0] packets; u32: [1] band and point lists, [2] FP64 leftovers and packets put aside, [3] how many of what is aside are taken
+  unsigned long long* counters = ws.get<unsigned long long>(4);
   uint32_t*           bandList = band64 ? ws.get<uint32_t>(n) : nullptr;
   uint8_t*            bandFlag = band64 ? ws.get<uint8_t>(n) : nullptr;
   size_t              selBytes = 0;
@@ -668,7 +668,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   if (!ws.ok) {
     return setError(EBG_ERR_NO_MEMORY, "query workspace allocation failed");
   }
-  cudaMemsetAsync(counters, 0, 3 * sizeof(unsigned long long), s);
+  cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), s);
   if (tm) {
     cudaEventRecord(ev[1], s);
   }

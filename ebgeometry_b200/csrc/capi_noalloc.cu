@@ -137,7 +137,7 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
     off += align256(bytes);
     return p;
   };
-  auto* counters = reinterpret_cast<unsigned long long*>(take(3 * sizeof(unsigned long long)));
+  auto* counters = reinterpret_cast<unsigned long long*>(take(4 * sizeof(unsigned long long)));
   auto* keysIn   = reinterpret_cast<uint32_t*>(take(u32n));
   auto* keysOut  = reinterpret_cast<uint32_t*>(take(u32n));
   auto* idsIn    = reinterpret_cast<uint32_t*>(take(u32n));
@@ -162,7 +162,7 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
 
   // the array keeps the previous call's contents: clear what must start at zero (a stale packet
   // counter would make the traversal skip every packet)
-  if (cudaMemsetAsync(counters, 0, 3 * sizeof(unsigned long long), s) != cudaSuccess) {
+  if (cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), s) != cudaSuccess) {
     return cudaFailed("clearing the allocation-free counters");
   }
   if (sort) {

@@ -26,11 +26,14 @@ struct MeshQueryArgs
   float              band;       // |d| <= band -> FP64 re-evaluation list
   uint32_t*          band_list;  // sorted positions needing FP64 (nullable = no band pass)
   uint32_t*          band_count;
-  uint32_t*          point_list; // sorted positions that the packet search leaves to one warp each; their
-                                 // number is counted in band_count[1] (zeroed before the launch)
+  uint32_t*          point_list; // n words for what the packet search puts aside: from the front the sorted
+                                 // positions that take eight lanes each (their number: band_count[1]), from
+                                 // the back the packets that take the walk, two words each (packet, mask of
+                                 // lanes; their number: later_count[1]).  Both counts zeroed before the launch.
   uint32_t*          later;       // entries of band_list that the packets of the FP64 pass leave to groups of
                                   // lanes, counted in later_count (nullable: every entry takes a group)
-  uint32_t*          later_count; // zeroed before the launch
+  uint32_t*          later_count; // zeroed before the launch, as the three words after it: [1] see point_list,
+                                 // [2] and [3] how many of the packets and points on it are taken
   const int32_t*     tri32;       // the FP32 pass's winning triangles, leaf order, caller order (nullable)
   float*             band_d32;   // FP32 distance of each band entry (nullable: read out_d instead)
   uint8_t*           band_flag;  // per sorted position, 1 = needs FP64 (nullable: the traversal
@@ -59,7 +62,8 @@ cudaError_t launchMeshSdf32(const MeshQueryArgs& a, int warpsPerBlock, int numSm
 
 // The FP32 search by packet boxes (plain, or with an attached model's cells; no counters, hints, top nodes
 // or 8-wide copy); delta as for launchMeshBand64; packets with a half-extent above split are divided.
-cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, int64_t numLeaves, int numSms, cudaStream_t s);
+cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, float diagonal, int64_t numLeaves, int numSms,
+                               cudaStream_t s);
 
 // FP64 re-evaluation of the band list (reads band_count on the device); split as for launchMeshPacket32.
 cudaError_t launchMeshBand64(const MeshQueryArgs& a, float delta, float split, int numSms, cudaStream_t s);

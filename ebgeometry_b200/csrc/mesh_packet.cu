@@ -27,7 +27,8 @@
 //
 // A packet too wide for one box is divided at its widest step.  What stays too wide, holds too few
 // points or reaches too many leaves (points few against the tree's leaves, or near the medial axis) is
-// put on a list, and kMeshListed searches those points eight lanes each.
+// put aside for kMeshAside: eight lanes search for each such point, or, where a packet is too wide as a whole
+// but its points share what they reach, the walk for all of them (sharesReach).
 //
 // Bound by the L1's data stage (89 % of its wavefronts) and by instruction issue (69 %): per packet of
 // the 512^3 grid 10 rounds of 32 children, 104 listed leaves, 27 of them with a pair, 7 passes over
@@ -59,6 +60,8 @@ __device__ __noinline__ int nearTriangle(const EbgMeshView& m, float px, float p
 
 constexpr int PACKET_FRONT = 32; // entries of a group's frontier
 
+constexpr float WALK_LEAVES = 0.2f; // leaves per point up to which a wide packet takes the walk
+
 struct PacketMem
 {
   float4             query[32]; // the lanes' points and bounds
@@ -86,16 +89,61 @@ __device__ __forceinline__ void store(const MeshQueryArgs& a, const EbgMeshView&
   }
 }
 
-// The points that kMeshPacket32 put aside, eight lanes each.
-__global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshListed(const __grid_constant__ MeshQueryArgs a, float delta)
+// What kMeshPacket32 put aside: first the packets (each a long chain of reads), then the points, eight lanes
+// each; a warp takes what is next.
+__global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshAside(const __grid_constant__ MeshQueryArgs a, float delta)
 {
-  __shared__ GroupMem mem[4 * PACKET_WARPS];
-  const EbgMeshView&  m   = a.mesh;
-  const uint32_t      n   = a.band_count[1];
-  const uint32_t      nG  = gridDim.x * (4 * PACKET_WARPS);
-  const uint32_t      grp = threadIdx.x >> 3;
-  for (uint32_t i0 = blockIdx.x * (4 * PACKET_WARPS) + (grp & ~3u); i0 < n; i0 += nG) {
-    const uint32_t i   = i0 + (grp & 3u);
+  union Mem
+  {
+    float4   stack[2 * EBG_STACK_DEPTH + 32];
+    GroupMem group[4];
+  };
+  __shared__ Mem     mem[PACKET_WARPS];
+  Mem&               w    = mem[threadIdx.x >> 5];
+  const EbgMeshView& m    = a.mesh;
+  const int          lane = threadIdx.x & 31;
+  const uint32_t     np   = a.later_count[1];
+  while (np != 0u) {
+    uint32_t i = 0;
+    if (lane == 0) {
+      i = atomicAdd(a.later_count + 2, 1u);
+    }
+    i = __shfl_sync(FULL, i, 0);
+    if (i >= np) {
+      break;
+    }
+    const uint32_t* e    = a.point_list + (a.n - 2 * (int64_t(i) + 1));
+    const int64_t   pos  = int64_t(__ldg(e)) * 32 + lane;
+    const bool      mine = (__ldg(e + 1) >> lane) & 1u;
+    const int64_t   src  = pos < a.n ? pos : a.n - 1;
+    const uint32_t  id   = a.order ? __ldg(a.order + src) : uint32_t(src);
+    const float     px = __ldg(a.points + 3 * size_t(id)), py = __ldg(a.points + 3 * size_t(id) + 1),
+                pz = __ldg(a.points + 3 * size_t(id) + 2);
+    float             best = mine ? FLT_MAX : -1.f; // a lane that was not left needs nothing
+    int               bt = -1, err = 0;
+    uint32_t          iters = 0;
+    TraversalCounters tc;
+    traverseMesh<false, EBG_STACK_DEPTH>(m, px, py, pz, best, bt, w.stack, w.stack + 2 * EBG_STACK_DEPTH, iters, err, tc);
+    if (err && lane == 0) {
+      atomicOr(a.status, err);
+    }
+    if (mine) {
+      store(a, m, bt, px, py, pz, id, pos);
+    }
+    __syncwarp();
+  }
+  const uint32_t n   = a.band_count[1];
+  const uint32_t grp = uint32_t(lane) >> 3;
+  while (n != 0u) {
+    uint32_t i0 = 0;
+    if (lane == 0) {
+      i0 = atomicAdd(a.later_count + 3, 4u);
+    }
+    i0 = __shfl_sync(FULL, i0, 0);
+    if (i0 >= n) {
+      break;
+    }
+    const uint32_t i   = i0 + grp;
     const bool     on  = i < n;
     const uint32_t pos = __ldg(a.point_list + (on ? i : i0));
     const uint32_t id  = a.order ? __ldg(a.order + pos) : pos;
@@ -103,8 +151,8 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshListed(const __grid
                 pz = __ldg(a.points + 3 * size_t(id) + 2);
     float     bd2;
     int       bt;
-    const int err = groupNearest(m, on, px, py, pz, delta, mem[grp], bd2, bt);
-    if (on && (threadIdx.x & 7) == 0) {
+    const int err = groupNearest(m, on, px, py, pz, delta, w.group[grp], bd2, bt);
+    if (on && (lane & 7) == 0) {
       if (err) {
         atomicOr(a.status, err);
       }
@@ -156,11 +204,30 @@ __device__ __forceinline__ int cellAnchor(const SeedCellsView& cv, float px, flo
   return __ldg(cv.anchor + (int64_t(iz) * cv.g + iy) * cv.g + ix);
 }
 
+// Whether a packet too wide for one box takes the walk as a whole: where its points (lanes `in`) share what they
+// reach.  The walk opens what any of them needs: about as many leaves as lie within the span of their
+// nearest points, (span / diagonal)^2 of all.  Points outside the mesh's box count from where they would
+// enter it (the ordering lines them up one behind the other), and the span shrinks with their distance.
+__device__ __noinline__ bool sharesReach(const EbgMeshView& m, bool in, float px, float py, float pz, float diagonal,
+                                         float leaves)
+{
+  const float inf = __int_as_float(0x7f800000);
+  const int   n   = __popc(__ballot_sync(FULL, in));
+  const float qx = fminf(fmaxf(px, m.root_lo[0]), m.root_hi[0]), qy = fminf(fmaxf(py, m.root_lo[1]), m.root_hi[1]),
+              qz = fminf(fmaxf(pz, m.root_lo[2]), m.root_hi[2]);
+  const float ex = warpMax(in ? qx : -inf) - warpMin(in ? qx : inf);
+  const float ey = warpMax(in ? qy : -inf) - warpMin(in ? qy : inf);
+  const float ez = warpMax(in ? qz : -inf) - warpMin(in ? qz : inf);
+  const float dx = px - qx, dy = py - qy, dz = pz - qz;
+  const float far = diagonal + 3.f * sqrtf(warpMin(in ? fmaf(dx, dx, fmaf(dy, dy, dz * dz)) : inf));
+  return n > 4 && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) * leaves < WALK_LEAVES * float(n) * far * far;
+}
+
 // CELLS: the query passes an attached model, and its cells' anchors give the lanes' first bounds and
 // the mesh points `a`.
 template <bool CELLS>
 __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __grid_constant__ MeshQueryArgs a, float delta,
-                                                                     float split, bool sparse)
+                                                                     float split, float diagonal, float leaves)
 {
   __shared__ PacketMem mem[PACKET_WARPS];
   const EbgMeshView&   m    = a.mesh;
@@ -170,6 +237,7 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
   const unsigned       lt   = (1u << lane) - 1u;
   const float          inf  = __int_as_float(0x7f800000);
   const uint64_t       numPackets = (uint64_t(a.n) + 31) / 32;
+  const bool           sparse     = float(numPackets) < leaves;
   unsigned long long   pk = 0, pkEnd = 0;
   int                  besttri = -1, frontN = 0;
   int                  limit = 0; // leaves per point that a range may reach
@@ -297,7 +365,8 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
     }
     float best  = -1.f; // a lane without a live point needs nothing
     int   prev  = besttri, err = 0;
-    bool  later = false; // the lane's point is on the list for kMeshListed
+    bool  later = false; // the lane's point is put aside,
+    bool  walk  = false; // as part of a packet for the walk
     besttri     = -1;
     // ranges [b, e) of lanes, each compact enough for one box
     int  b = 0, e = 32;
@@ -310,6 +379,11 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
       r.hx = fmaxf(mxx - r.cx, r.cx - mnx), r.hy = fmaxf(mxy - r.cy, r.cy - mny), r.hz = fmaxf(mxz - r.cz, r.cz - mnz);
       const float hm  = fmaxf(r.hx, fmaxf(r.hy, r.hz));
       bool        box = hm <= split && !__any_sync(FULL, in && !(fabsf(px) + fabsf(py) + fabsf(pz) < 1e12f));
+      if (!box && e - b == 32 && sharesReach(m, in, px, py, pz, diagonal, leaves)) {
+        walk  = true;
+        later = in;
+        break;
+      }
       if (!box && e - b > 4 && hm <= 16.f * split) {
         // divide at the widest step from one point to the next
         const float ux = __shfl_up_sync(FULL, px, 1), uy = __shfl_up_sync(FULL, py, 1), uz = __shfl_up_sync(FULL, pz, 1);
@@ -525,25 +599,25 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
         }
       }
       if (!box) {
-        // too wide, far away, very few points, too many leaves in reach, or no live lane at all: one
-        // warp per point, later
-        const unsigned todo = __ballot_sync(FULL, in);
-        if (todo != 0u) {
-          uint32_t base = 0;
-          if (lane == 0) {
-            base = atomicAdd(a.band_count + 1, uint32_t(__popc(todo)));
-          }
-          base = __shfl_sync(FULL, base, 0);
-          if (in) {
-            a.point_list[base + __popc(todo & lt)] = uint32_t(pos);
-            later                                  = true;
-          }
-        }
+        // too wide, far away, very few points or too many leaves in reach
+        later = later || in;
       }
       b = e;
       e = 32;
     }
 
+    const unsigned todo = __ballot_sync(FULL, later);
+    if (todo != 0u) {
+      // packets from the list's end, two words each (for at least five points, so that the two never meet)
+      uint32_t at = 0;
+      if (lane == 0) {
+        at = walk ? a.n - 2 * (atomicAdd(a.later_count + 1, 1u) + 1u) : atomicAdd(a.band_count + 1, uint32_t(__popc(todo)));
+      }
+      at = __shfl_sync(FULL, at, 0) + (walk ? uint32_t(lane) : uint32_t(__popc(todo & lt)));
+      if (walk ? lane < 2 : later) {
+        a.point_list[at] = walk ? (lane == 0 ? uint32_t(pk) : todo) : uint32_t(pos);
+      }
+    }
     if (err && lane == 0) {
       atomicOr(a.status, err);
     }
@@ -579,7 +653,8 @@ void launchNodeChildren(const EbgNode4* nodes, int64_t numNodes, EbgChild* child
   }
 }
 
-cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, int64_t numLeaves, int numSms, cudaStream_t s)
+cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, float diagonal, int64_t numLeaves, int numSms,
+                               cudaStream_t s)
 {
   const int64_t packets = (a.n + 31) / 32;
   const int64_t need    = (packets + PACKET_WARPS - 1) / PACKET_WARPS;
@@ -587,12 +662,12 @@ cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, int64_
   const int64_t grid    = need < most ? need : most;
   a.chunk = a.chunk > 1 ? a.chunk : 8; // packets per group
   if (a.cells.count != nullptr) {
-    kMeshPacket32<true><<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta, split, packets < numLeaves);
+    kMeshPacket32<true><<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta, split, diagonal, float(numLeaves));
   }
   else {
-    kMeshPacket32<false><<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta, split, packets < numLeaves);
+    kMeshPacket32<false><<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta, split, diagonal, float(numLeaves));
   }
-  kMeshListed<<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta);
+  kMeshAside<<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta);
   return cudaGetLastError();
 }
 
