@@ -8,6 +8,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "cells_kernels.h"
 #include "ebg_layout.h"
 #include "ebgeometry_b200.h"
@@ -31,6 +33,9 @@ struct ebg_mesh
   void* dNodeObb = nullptr;
   void* dDcelN   = nullptr;
   int*  dStatus = nullptr;
+  // the leaf boxes' diagonals, in units of the mesh's: sums on the device, mean and mean square
+  unsigned long long* dLeafSums = nullptr;
+  double              leafMean = 0.0, leafSquare = 0.0;
   // kept for refitting moved vertices: the soup's triangles, and each leaf's and each interior
   // node's range of leaf positions
   int32_t*  dF         = nullptr;
@@ -123,6 +128,14 @@ inline uint32_t   topNodesFor(const ebg_mesh* m, const ebg_query_opts* opts, boo
 // asked for closest triangles in FP32.
 cudaError_t launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool fp32Triangles, int warpsPerBlock,
                            int occupancy, float delta, cudaStream_t s);
+
+// Mean and mean square from the sums of launchLeafSizes.
+inline void setLeafSizes(ebg_mesh* m, const unsigned long long* sums)
+{
+  const double per = 1.0 / (4294967296.0 * double(std::max<int64_t>(1, m->info.num_leaves)));
+  m->leafMean   = double(sums[0]) * per;
+  m->leafSquare = double(sums[1]) * per;
+}
 
 // The half-extent up to which a packet of points shares one box.
 float packetSplit(const ebg_mesh* m);

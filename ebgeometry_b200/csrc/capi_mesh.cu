@@ -209,6 +209,7 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
 {
   const size_t slots = 4 * size_t(std::max<int64_t>(m->info.num_nodes, 1));
   if (cudaMalloc(&m->dChildren, slots * sizeof(EbgChild)) != cudaSuccess ||
+      cudaMalloc(reinterpret_cast<void**>(&m->dLeafSums), 2 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&m->dStatus), sizeof(int)) != cudaSuccess ||
       cudaMemset(m->dStatus, 0, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
@@ -235,11 +236,14 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
                              size_t(inf.num_leaves) * (sizeof(EbgObb) + 8) +
                              N * (sizeof(EbgTriHot) + sizeof(EbgTriSign) + 33 * sizeof(double) + 4 + 12));
   launchNodeChildren(v.nodes, inf.num_nodes, static_cast<EbgChild*>(m->dChildren), nullptr);
-  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
+  launchLeafSizes(v.children, inf.num_nodes, inf.diagonal, m->dLeafSums, nullptr);
+  unsigned long long sums[2];
+  if (cudaMemcpy(sums, m->dLeafSums, sizeof(sums), cudaMemcpyDeviceToHost) != cudaSuccess) {
     const std::string e = cudaGetErrorString(cudaGetLastError());
     ebg_mesh_destroy(m);
     return setError(EBG_ERR_CUDA, "mesh set-up: " + e);
   }
+  setLeafSizes(m, sums);
   *out = m;
   return EBG_OK;
 }
@@ -511,6 +515,20 @@ bool pointPath(int64_t n, const ebg_query_opts* opts, const unsigned long long* 
 
 } // namespace
 
+// Whether the mesh is what the packet boxes are sized for: a surface about as large as its extent, in leaves
+// of about one size that together cover it about once.  In units of the squared diagonal, spheres, cubes,
+// ellipsoids of 5:1 and several bodies side by side have a surface of 0.75-2 and leaf boxes of 3.4-6.6.
+// Outside these ranges the walk is as fast or faster, whole calls of 8 M points: 327,680 triangles squeezed to a
+// needle (surface 0.03), near it, 6.5 against 18.5 ms; bunched by a power of 5 (leaf boxes 1.3) 13.0 / 18.7; a
+// fine ball beside a coarse sheet (the leaves' mean^2 0.01 of their mean square) 9.5 / 21.0; strips of a
+// cylinder (leaf boxes 6,000) 16.6 / 29.3; a sheet (2.1) 11.9 / 15.2; loose triangles (30) the same.
+static bool packetMesh(const ebg_mesh* m)
+{
+  const double d2 = m->info.diagonal * m->info.diagonal, boxes = m->leafSquare * double(m->info.num_leaves);
+  return m->info.num_triangles >= 4096 && boxes >= 3.0 && boxes <= 8.0 && m->leafMean * m->leafMean >= 0.5 * m->leafSquare &&
+         !m->areaCdf.empty() && m->areaCdf.back() >= 0.6 * d2;
+}
+
 float ebg::packetSplit(const ebg_mesh* m)
 {
   // packets up to three mean leaf sizes wide share one box (the extent of a leaf on a surface of
@@ -523,14 +541,15 @@ float ebg::packetSplit(const ebg_mesh* m)
 //  - meshes of fewer than 4,096 triangles, whose walk is short (4 M points on 1,280 triangles: 0.37
 //    against 0.48 ms near the surface, 0.92 against 0.94 ms everywhere; on 5,120 triangles 1.9 against
 //    1.8 ms everywhere);
+//  - meshes whose leaves are not about as large as a closed surface of the mesh's extent makes them
+//    (packetMesh): the packet boxes are sized by that;
 //  - FP32 calls that ask for the closest triangles: of triangles at the same distance the walk names the
 //    one that its order and box rounding leave, another search another one (6 of 20,000 points on and far
 //    from the surface, 2 of 8 M uniform ones).
 cudaError_t ebg::launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool fp32Triangles, int wpb, int occ,
                                 float delta, cudaStream_t s)
 {
-  if (a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && a.node_width != 8 && !fp32Triangles &&
-      m->info.num_triangles >= 4096) {
+  if (a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && a.node_width != 8 && !fp32Triangles && packetMesh(m)) {
     return launchMeshPacket32(a, delta, packetSplit(m), float(m->info.diagonal), m->info.num_leaves, m->numSms, s);
   }
   return launchMeshSdf32(a, wpb, m->numSms, s, occ);
@@ -840,6 +859,7 @@ ebg_status ebg_mesh_destroy(ebg_mesh* m)
   cudaFree(m->dNodeObb);
   cudaFree(m->dDcelN);
   cudaFree(m->dStatus);
+  cudaFree(m->dLeafSums);
   cudaFree(m->dF);
   cudaFree(m->dLeafFirst);
   cudaFree(m->dLeafCount);

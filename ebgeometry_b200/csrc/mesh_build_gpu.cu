@@ -1971,6 +1971,13 @@ ebg_status refitMeshOnDevice(ebg_mesh* m, const double* V, bool vOnDevice, int64
                                                                    static_cast<EbgNode4*>(m->dNodes));
     launchNodeChildren(m->view.nodes, numNodes, static_cast<EbgChild*>(m->dChildren), s);
   }
+  double d2 = 0;
+  for (int a = 0; a < 3; a++) {
+    d2 += (outHi[a] - outLo[a]) * (outHi[a] - outLo[a]);
+  }
+  launchLeafSizes(m->view.children, numNodes, std::sqrt(d2), m->dLeafSums, s);
+  unsigned long long sums[2];
+  cudaMemcpyAsync(sums, m->dLeafSums, sizeof(sums), cudaMemcpyDeviceToHost, s);
   std::vector<double> cdf(N);
   cudaMemcpyAsync(cdf.data(), area, 8 * N, cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) {
@@ -1980,6 +1987,7 @@ ebg_status refitMeshOnDevice(ebg_mesh* m, const double* V, bool vOnDevice, int64
     cdf[i] += cdf[i - 1];
   }
   m->areaCdf.swap(cdf);
+  setLeafSizes(m, sums);
   return EBG_OK;
 }
 

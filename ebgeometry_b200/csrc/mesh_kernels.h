@@ -57,6 +57,10 @@ void launchQueryKeys(const float* points, int64_t n, const float* lo, const floa
 // children[4 i + k] = slot k of nodes[i].
 void launchNodeChildren(const EbgNode4* nodes, int64_t numNodes, EbgChild* children, cudaStream_t s);
 
+// sums[0], sums[1] = the sum of the leaf boxes' diagonals and of their squares, in units of `diagonal` as 32.32
+// fixed-point numbers.
+void launchLeafSizes(const EbgChild* children, int64_t numNodes, double diagonal, unsigned long long* sums, cudaStream_t s);
+
 // FP32 packet traversal.  warpsPerBlock in {1,2,4,8}; occupancy 0..3 (see ebg_query_opts).
 cudaError_t launchMeshSdf32(const MeshQueryArgs& a, int warpsPerBlock, int numSms, cudaStream_t s, int occupancy = 0);
 

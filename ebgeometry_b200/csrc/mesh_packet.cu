@@ -35,6 +35,7 @@
 // pairs, about 19,000 warp instructions.  B200, 151 M points on 1.3 M triangles, the walk -> here:
 // traversal 172.6 -> 79.5 ms, with a model 92.3 -> 71.2 ms; 1 M uniform points on 20,480 triangles
 // 1.42 -> 0.75 ms; 262,144 on 81,920 triangles 2.11 -> 0.65 ms.
+#include <algorithm>
 #include <cfloat>
 
 #include "ebg_device.cuh"
@@ -643,7 +644,43 @@ __global__ void kNodeChildren(const EbgNode4* __restrict__ nodes, int64_t slots,
     out[i]            = EbgChild{n.lox[k], n.loy[k], n.loz[k], n.child[k], n.hix[k], n.hiy[k], n.hiz[k], n.count[k]};
   }
 }
+
+// sums[0], sums[1]: the leaf boxes' diagonals and their squares, in units of the mesh's diagonal as 32.32
+// fixed-point numbers (whose sum does not depend on the order).
+__global__ void kLeafSizes(const EbgChild* __restrict__ children, int64_t slots, float invDiagonal,
+                           unsigned long long* __restrict__ sums)
+{
+  unsigned long long s1 = 0, s2 = 0;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < slots; i += int64_t(gridDim.x) * blockDim.x) {
+    const float4 lo = __ldg(reinterpret_cast<const float4*>(children + i)), hi = __ldg(reinterpret_cast<const float4*>(children + i) + 1);
+    if (__float_as_uint(lo.w) & EBG_LEAF_BIT) {
+      const float x = (hi.x - lo.x) * invDiagonal, y = (hi.y - lo.y) * invDiagonal, z = (hi.z - lo.z) * invDiagonal;
+      const float l2 = fmaf(x, x, fmaf(y, y, z * z));
+      s1 += (unsigned long long)(sqrtf(l2) * 4294967296.f);
+      s2 += (unsigned long long)(l2 * 4294967296.f);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    s1 += __shfl_xor_sync(FULL, s1, o);
+    s2 += __shfl_xor_sync(FULL, s2, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(sums, s1);
+    atomicAdd(sums + 1, s2);
+  }
+}
 } // namespace
+
+void launchLeafSizes(const EbgChild* children, int64_t numNodes, double diagonal, unsigned long long* sums, cudaStream_t s)
+{
+  cudaMemsetAsync(sums, 0, 2 * sizeof(unsigned long long), s);
+  const int64_t blocks = (4 * numNodes + 255) / 256;
+  if (blocks > 0) {
+    kLeafSizes<<<unsigned(blocks < 1024 ? blocks : 1024), 256, 0, s>>>(children, 4 * numNodes,
+                                                                        float(1.0 / std::max(diagonal, 1e-300)), sums);
+  }
+}
 
 void launchNodeChildren(const EbgNode4* nodes, int64_t numNodes, EbgChild* children, cudaStream_t s)
 {

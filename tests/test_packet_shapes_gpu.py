@@ -46,3 +46,50 @@ def test_distances_and_time_of_the_walk(name, n):
     assert torch.equal(d, walk)
     if n == 8000000:
         assert _ms(lambda: m.signed_distance(p)) <= 1.5 * _ms(lambda: m.signed_distance(p, top_nodes=64))
+
+
+def _uneven(name):
+    v, f = W.displaced_icosphere(7, 5)
+    if name == "needle":
+        return v * [1.0, 0.01, 0.01], f
+    if name == "bunched":
+        return np.sign(v) * np.abs(v) ** 5, f
+    if name == "strips":
+        k = 25000
+        t = np.arange(k) * 2 * np.pi / k
+        ring = np.stack([0.5 * np.cos(t), 0.5 * np.sin(t), np.full(k, -1.0)], 1)
+        i = np.arange(k)
+        j = (i + 1) % k
+        cap = np.full(k, 2 * k)
+        return (np.concatenate([ring, ring * [1, 1, -1], [[0, 0, -1], [0, 0, 1]]]),
+                np.concatenate([np.stack([i, j, j + k], 1), np.stack([i, j + k, i + k], 1), np.stack([j, i, cap], 1),
+                                np.stack([i + k, j + k, cap + 1], 1)]).astype(np.int32))
+    # a fine ball beside a coarse sheet
+    x, y = np.meshgrid(np.linspace(-1, 1, 33), np.linspace(-1, 1, 33))
+    s = np.stack([x.ravel(), y.ravel(), 0.0 * x.ravel()], 1)
+    i = (np.arange(32)[:, None] * 33 + np.arange(32)[None]).ravel()
+    g = np.concatenate([np.stack([i, i + 1, i + 34], 1), np.stack([i, i + 34, i + 33], 1)])
+    return np.concatenate([0.02 * v + [0, 0, 0.5], s]), np.concatenate([f, g + len(v)]).astype(np.int32)
+
+
+@pytest.mark.parametrize("name", ["needle", "bunched", "strips", "ball and sheet"])
+def test_uneven_meshes_take_the_walk(name):
+    """The packet boxes are sized for a surface about as large as the mesh's extent in leaves of one size; on
+    others they took up to 4.5 times the walk's time."""
+    v, f = _uneven(name)
+    m = TriMeshSDF(v, f, build="Morton", on_device=True)
+    lo, hi = v.min(0), v.max(0)
+    near = W.band_points(v, f, 4000000, 3, width=1e-3)
+    wide = (lo + hi) / 2 + np.random.default_rng(1).uniform(-0.6, 0.6, (4000000, 3)) * (hi - lo).max()
+    for p in (near, wide):
+        p = torch.from_numpy(p.astype(np.float32)).cuda()
+        d = m.signed_distance(p)
+        walk = m.signed_distance(p, top_nodes=64)
+        m.check_status()
+        assert torch.equal(d, walk)
+        assert _ms(lambda: m.signed_distance(p)) <= 1.3 * _ms(lambda: m.signed_distance(p, top_nodes=64))
+    # refitted to the round body, the same handle takes the packets again (the same distances either way)
+    if name == "bunched":
+        m.refit(W.displaced_icosphere(7, 5)[0])
+        p = torch.from_numpy(W.uniform_points(200000, 4)).cuda()
+        assert torch.equal(m.signed_distance(p), m.signed_distance(p, top_nodes=64))
