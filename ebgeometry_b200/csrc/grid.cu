@@ -7,7 +7,7 @@
 // for a flat box), coarsened until the grid holds at most 64 + 8 n cells, as the reference sizes
 // it; cell coordinates floor((p - lo) / h) in FP64, clamped; a radix sort of (cell, index) makes
 // every cell a contiguous range of points (float4: xyz and the index bits).
-// Query: one thread per query (more than 1 M queries in Morton order), k best in registers; shells of cells
+// Query: one thread per query (many queries in Morton order), k best in registers; shells of cells
 // at Chebyshev distance r = 0, 1, ... around the query's cell.  After shell r, every point not yet seen
 // lies outside the box of cells [c - r, c + r]; its distance is at least the distance from the query
 // to the nearest open side of that box (FP64, minus a relative 1e-9 of h).  The search stops once
@@ -96,6 +96,23 @@ __global__ void kGridCells(const float* __restrict__ pts, int64_t n, const GridV
     cell[i]          = c;
     ids[i]           = uint32_t(i);
     atomicAdd(counts + c, 1u);
+  }
+}
+
+// The sum over the cells of their squared number of points.
+__global__ void kGridSquares(const uint32_t* __restrict__ counts, int64_t cells, unsigned long long* __restrict__ sum)
+{
+  unsigned long long q = 0;
+  for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < cells; i += int64_t(gridDim.x) * blockDim.x) {
+    const unsigned long long c = counts[i];
+    q += c * c;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    q += __shfl_xor_sync(FULL, q, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(sum, q);
   }
 }
 
@@ -524,6 +541,7 @@ struct ebg_grid
   uint32_t*      dInv    = nullptr;
   int*           dStatus = nullptr;
   double         target  = 1.0;
+  bool           uneven  = false; // see gridQuery's rules
 };
 
 using namespace ebg;
@@ -651,6 +669,14 @@ ebg_status ebg_grid_create(const float* points_host, int64_t n, double target_pe
   cudaMemsetAsync(counts, 0, 4 * size_t(nc + 1), s);
   cudaMemsetAsync(G->dStatus, 0, sizeof(int), s);
   kGridCells<<<gridBlocks(n), 256, 0, s>>>(dPts, n, g, cell, ids, counts);
+  unsigned long long* squares = nullptr;
+  if (!alloc((void**)&squares, 8)) {
+    return fail(EBG_ERR_NO_MEMORY, "grid build workspace");
+  }
+  cudaMemsetAsync(squares, 0, 8, s);
+  kGridSquares<<<std::min(gridBlocks(nc), 1024u), 256, 0, s>>>(counts, nc, squares);
+  unsigned long long hsq = 0;
+  cudaMemcpyAsync(&hsq, squares, 8, cudaMemcpyDeviceToHost, s);
   size_t sortBytes = 0, scanBytes = 0;
   int cellBits = 1;
   while (cellBits < 32 && (int64_t(1) << cellBits) < nc) {
@@ -673,6 +699,8 @@ ebg_status ebg_grid_create(const float* points_host, int64_t n, double target_pe
     return fail(EBG_ERR_CUDA, std::string("grid build: ") + cudaGetErrorString(cudaGetLastError()));
   }
   cudaStreamDestroy(s);
+  // a point of a uniform cloud shares its cell with `target` others
+  G->uneven   = double(hsq) > 2.0 * (G->target + 1.0) * double(n);
   g.points    = G->dPoints;
   g.cellStart = G->dStart;
   *out        = G;
@@ -710,13 +738,18 @@ ebg_status ebg_grid_info(const ebg_grid* G, int32_t* cells_xyz, double* cell_siz
   return EBG_OK;
 }
 
-// External queries are put in Morton order from this count on.  Below it the order costs more than the
-// nearer reads give: 4 M points, 262,144 queries with and without it 208 and 131 us, 1 M queries (k = 4)
-// 395 and 333, (k = 1) 258 and 195; 16 M points, 4 M queries 942 and 1494.
-static constexpr int64_t GRID_ORDERED = (1 << 20) + 1;
-// Calls of this many queries (any number for k > 8, none for k = 1) put those that go beyond shell 1 into a
-// second launch.  4 M points, k = 4, without and with it: 131,072 queries 73 and 92 us, 262,144 132 and 128,
-// 1 M 419 and 328; k = 16, 3000 and 262,144 queries 152 and 147 us, 1002 and 711; k = 1, 1 M: 205 and 310.
+// External queries are put in Morton order from this count on.  In a cloud that fills its box evenly the order
+// costs more than the nearer reads give up to about 1 M: 4 M points, 262,144 queries with and without it 208
+// and 131 us, 1 M queries (k = 4) 395 and 333, (k = 1) 258 and 195; 16 M points, 1 M queries 492 and 495, 4 M
+// 1375 and 1811.  In an uneven one (its points share their cells with more than twice as many others)
+// neighbouring threads that are not neighbours in space wait for the one in the densest cell: half of 1 M
+// points in 64 clusters, queries at cloud points, k = 16: 100,000 queries 3.4 and 4.1 ms, 262,144 5.1 and 7.9,
+// 1 M 8.0 and 25.1; queries anywhere, k = 1: 100,000 286 and 215 us, 1 M 469 and 553.
+static constexpr int64_t GRID_ORDERED = (1 << 20) + 1, GRID_ORDERED_UNEVEN = 1 << 16;
+// Calls of this many queries (any number for k > 8 or in an uneven cloud, none for k = 1) put those that go
+// beyond shell 1 into a second launch.  4 M points, k = 4, without and with it: 131,072 queries 73 and 92 us,
+// 262,144 132 and 128, 1 M 419 and 328; k = 16, 3000 and 262,144 queries 152 and 147 us, 1002 and 711; k = 1,
+// 1 M: 205 and 310.  Uneven, 1 M points, k = 4: 10,000 queries 2.66 and 1.06 ms, 100,000 2.30 and 1.81.
 static constexpr int64_t GRID_SPLIT = 1 << 18;
 
 // The three query forms: external points (queries), self queries of listed cloud indices (ids) and
@@ -740,7 +773,7 @@ static ebg_status gridQuery(const ebg_grid* G, const float* queries_dev, const i
     }
   };
   uint32_t* order = nullptr;
-  if (queries_dev && nq >= GRID_ORDERED) {
+  if (queries_dev && nq >= (G->uneven ? GRID_ORDERED_UNEVEN : GRID_ORDERED)) {
     // Morton order of the queries over the grid's box, so that a warp's queries visit nearby cells
     auto* kin  = static_cast<uint32_t*>(get(4 * size_t(nq)));
     auto* kout = static_cast<uint32_t*>(get(4 * size_t(nq)));
@@ -773,7 +806,7 @@ static ebg_status gridQuery(const ebg_grid* G, const float* queries_dev, const i
   a.outIdx   = idx_dev;
   a.outD2    = d2_dev;
   a.status   = G->dStatus;
-  if (k > 1 && (k > 8 || nq >= GRID_SPLIT)) {
+  if (k > 1 && (k > 8 || G->uneven || nq >= GRID_SPLIT)) {
     a.later      = static_cast<uint32_t*>(get(4 * size_t(nq)));
     a.laterCount = static_cast<uint32_t*>(get(4));
     if (a.later && a.laterCount) {
