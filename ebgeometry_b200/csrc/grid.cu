@@ -19,6 +19,7 @@
 #include <string>
 #include <vector>
 
+#include <cooperative_groups.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cuda_runtime.h>
@@ -29,6 +30,8 @@
 #include "mesh_kernels.h"
 
 namespace ebg {
+
+namespace cg = cooperative_groups;
 namespace {
 
 struct GridView
@@ -386,7 +389,7 @@ __global__ void __launch_bounds__(128, gridOccupancy(K, MODE)) kGridKnn(const __
       if (!stop) {
         // Row by row where cells are dense: lanes of the same cell then read the same points together,
         // and rows beyond the k-th best are left out.  (A uniform cloud has about 27 points here.)
-        if (__any_sync(__activemask(), total > 64)) {
+        if (cg::coalesced_threads().any(total > 64)) {
           const float gy0 = gap(Qy, cy, -1, g.lo[1]), gy2 = gap(Qy, cy, 1, g.lo[1]);
           const float gz0 = gap(Qz, cz, -1, g.lo[2]), gz2 = gap(Qz, cz, 1, g.lo[2]);
 #pragma unroll 1
@@ -429,14 +432,12 @@ __global__ void __launch_bounds__(128, gridOccupancy(K, MODE)) kGridKnn(const __
         stop = done(1);
       }
       if (!stop && rMax >= 2) {
-        const unsigned m    = __activemask();
-        const int      lead = __ffs(m) - 1;
-        uint32_t       at   = 0;
-        if ((tid & 31) == lead) {
-          at = atomicAdd(a.laterCount, uint32_t(__popc(m)));
+        const auto rest = cg::coalesced_threads(); // any part of the warp may take its places together
+        uint32_t   at   = 0;
+        if (rest.thread_rank() == 0) {
+          at = atomicAdd(a.laterCount, uint32_t(rest.size()));
         }
-        at = __shfl_sync(m, at, lead);
-        a.later[at + __popc(m & ((1u << (tid & 31)) - 1u))] = uint32_t(t);
+        a.later[rest.shfl(at, 0) + uint32_t(rest.thread_rank())] = uint32_t(t);
       }
     }
     else {
