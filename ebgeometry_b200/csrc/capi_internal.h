@@ -126,8 +126,9 @@ inline uint32_t   topNodesFor(const ebg_mesh* m, const ebg_query_opts* opts, boo
 
 // The FP32 pass of a query (see the definition for which search it takes); fp32Triangles: the caller
 // asked for closest triangles in FP32.
-cudaError_t launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool fp32Triangles, int warpsPerBlock,
-                           int occupancy, float delta, cudaStream_t s);
+// a.chunk: packets taken from the work counter at a time, 0 = the default.
+cudaError_t launchMeshFp32(const ebg_mesh* m, MeshQueryArgs a, bool fp32Triangles, int warpsPerBlock, int occupancy,
+                           float delta, cudaStream_t s);
 
 // Mean and mean square from the sums of launchLeafSizes.
 inline void setLeafSizes(ebg_mesh* m, const unsigned long long* sums)

@@ -546,10 +546,14 @@ float ebg::packetSplit(const ebg_mesh* m)
 //  - FP32 calls that ask for the closest triangles: of triangles at the same distance the walk names the
 //    one that its order and box rounding leave, another search another one (6 of 20,000 points on and far
 //    from the surface, 2 of 8 M uniform ones).
-cudaError_t ebg::launchMeshFp32(const ebg_mesh* m, const MeshQueryArgs& a, bool fp32Triangles, int wpb, int occ,
-                                float delta, cudaStream_t s)
+cudaError_t ebg::launchMeshFp32(const ebg_mesh* m, MeshQueryArgs a, bool fp32Triangles, int wpb, int occ, float delta,
+                                cudaStream_t s)
 {
+  // (packets taken at a time: the caller's number, else the tuned one, else groups of 8 or single ones)
+  const int chunk = a.chunk;
+  a.chunk         = chunk > 0 ? chunk : std::max(1, m->tunedChunk);
   if (a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && a.node_width != 8 && !fp32Triangles && packetMesh(m)) {
+    a.chunk = chunk > 0 ? chunk : (m->tunedChunk > 1 ? m->tunedChunk : 8);
     return launchMeshPacket32(a, delta, packetSplit(m), float(m->info.diagonal), m->info.num_leaves, m->numSms, s);
   }
   return launchMeshSdf32(a, wpb, m->numSms, s, occ);
@@ -715,7 +719,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   a.work       = counters;
   a.status     = m->dStatus;
   a.stats      = statsDev;
-  a.chunk      = (opts && opts->queue_chunk > 0) ? opts->queue_chunk : (m->tunedChunk > 0 ? m->tunedChunk : 1);
+  a.chunk      = (opts && opts->queue_chunk > 0) ? opts->queue_chunk : 0;
   if (seed) {
     a.cells = m->cellsView;
   }

@@ -191,7 +191,7 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
   a.work       = counters;
   a.status     = m->dStatus;
   a.stats      = nullptr;
-  a.chunk      = (opts && opts->queue_chunk > 0) ? opts->queue_chunk : (m->tunedChunk > 0 ? m->tunedChunk : 1);
+  a.chunk      = (opts && opts->queue_chunk > 0) ? opts->queue_chunk : 0;
   if (seed) {
     a.cells = m->cellsView; // the attached model's entry cuts live with the mesh
   }

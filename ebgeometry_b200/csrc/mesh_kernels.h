@@ -65,8 +65,8 @@ void launchLeafSizes(const EbgChild* children, int64_t numNodes, double diagonal
 cudaError_t launchMeshSdf32(const MeshQueryArgs& a, int warpsPerBlock, int numSms, cudaStream_t s, int occupancy = 0);
 
 // The FP32 search by packet boxes (plain, or with an attached model's cells; no counters, hints, top nodes
-// or 8-wide copy); delta as for launchMeshBand64; packets with a half-extent above split are divided.
-cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, float diagonal, int64_t numLeaves, int numSms,
+// or 8-wide copy; a.chunk: packets per group, at least 1); delta as for launchMeshBand64; packets with a half-extent above split are divided.
+cudaError_t launchMeshPacket32(const MeshQueryArgs& a, float delta, float split, float diagonal, int64_t numLeaves, int numSms,
                                cudaStream_t s);
 
 // FP64 re-evaluation of the band list (reads band_count on the device); split as for launchMeshPacket32.

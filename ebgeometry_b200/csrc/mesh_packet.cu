@@ -690,14 +690,13 @@ void launchNodeChildren(const EbgNode4* nodes, int64_t numNodes, EbgChild* child
   }
 }
 
-cudaError_t launchMeshPacket32(MeshQueryArgs a, float delta, float split, float diagonal, int64_t numLeaves, int numSms,
+cudaError_t launchMeshPacket32(const MeshQueryArgs& a, float delta, float split, float diagonal, int64_t numLeaves, int numSms,
                                cudaStream_t s)
 {
   const int64_t packets = (a.n + 31) / 32;
   const int64_t need    = (packets + PACKET_WARPS - 1) / PACKET_WARPS;
   const int64_t most    = int64_t(numSms) * 8;
   const int64_t grid    = need < most ? need : most;
-  a.chunk = a.chunk > 1 ? a.chunk : 8; // packets per group
   if (a.cells.count != nullptr) {
     kMeshPacket32<true><<<unsigned(grid), 32 * PACKET_WARPS, 0, s>>>(a, delta, split, diagonal, float(numLeaves));
   }

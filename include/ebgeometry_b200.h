@@ -106,7 +106,9 @@ typedef struct ebg_query_opts
                                          seed is set. */
   int32_t            queue_chunk;     /* packets of 32 queries a warp takes from the device work
                                          queue at a time (mesh and union queries); 0 = tuned
-                                         default (1) */
+                                         default (1 for the packet walk and unions, 8 for the search
+                                         by packet boxes, whose packets then start from a common part
+                                         of the tree) */
   int32_t            top_nodes;       /* plain mesh queries: each block of the traversal copies the
                                          tree's first top_nodes nodes (the device build numbers them
                                          level by level: 21 = the root and two levels) with their
