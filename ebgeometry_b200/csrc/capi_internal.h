@@ -51,6 +51,7 @@ struct ebg_mesh
   int tunedOccupancy = 0;
   int tunedWpb       = 0;
   int tunedChunk     = 0;
+  int tunedGroup     = 0; // packets per group of the search by packet boxes
   int tunedWidth     = 0; // 8: plain queries take the 8-wide copy
   // the optional 8-wide copy of the tree (ebg_mesh_widen; plain FP32 queries): its nodes and their
   // oriented boxes, and the view the traversal reads them through (the 4-wide view with nodes,

@@ -553,7 +553,7 @@ cudaError_t ebg::launchMeshFp32(const ebg_mesh* m, MeshQueryArgs a, bool fp32Tri
   const int chunk = a.chunk;
   a.chunk         = chunk > 0 ? chunk : std::max(1, m->tunedChunk);
   if (a.stats == nullptr && a.hint == nullptr && a.top_nodes == 0 && a.node_width != 8 && !fp32Triangles && packetMesh(m)) {
-    a.chunk = chunk > 0 ? chunk : (m->tunedChunk > 1 ? m->tunedChunk : 8);
+    a.chunk = chunk > 0 ? chunk : (m->tunedGroup > 0 ? m->tunedGroup : 8);
     return launchMeshPacket32(a, delta, packetSplit(m), float(m->info.diagonal), m->info.num_leaves, m->numSms, s);
   }
   return launchMeshSdf32(a, wpb, m->numSms, s, occ);
@@ -1370,14 +1370,18 @@ ebg_status ebg_mesh_autotune(ebg_mesh*       m,
   }
   DeviceGuard guard;
   cudaSetDevice(m->device);
-  float*       out = nullptr;
-  cudaStream_t s   = static_cast<cudaStream_t>(stream);
-  if (cudaMallocAsync(reinterpret_cast<void**>(&out), size_t(n) * sizeof(float), s) != cudaSuccess) {
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  Workspace    ws(s);
+  float*       out = ws.get<float>(n);
+  int32_t*     tri = ws.get<int32_t>(n);
+  if (!ws.ok) {
     cudaGetLastError();
-    return setError(EBG_ERR_NO_MEMORY, "autotune output buffer");
+    return setError(EBG_ERR_NO_MEMORY, "autotune output buffers");
   }
-  // the traversal time of one candidate: the best of two timed runs after a warm-up run
-  auto timeOne = [&](int o, int w, int c, float& ms, int width = 4) -> ebg_status {
+  // The traversal time of one candidate: the best of two timed runs after a warm-up run.  The launch shape
+  // is the packet walk's, so it is timed on the walk, which calls for the closest triangles always take.
+  ebg_status rc      = EBG_OK;
+  auto       timeOne = [&](int o, int w, int c, bool walk, int width = 4) -> float {
     ebg_query_opts    q{};
     ebg_phase_timings t{};
     q.occupancy       = o;
@@ -1386,81 +1390,66 @@ ebg_status ebg_mesh_autotune(ebg_mesh*       m,
     q.node_width      = width;
     q.no_fp64_band    = 1;
     q.seed            = seed;
-    ms                = INFINITY;
-    for (int rep = 0; rep < 3; rep++) {
-      q.timings           = &t;
-      const ebg_status rc = meshQuery(m, sample_points_dev, n, out, nullptr, &q, nullptr, s);
-      if (rc != EBG_OK) {
-        return rc;
-      }
-      if (rep > 0) {
-        ms = std::min(ms, t.traverse_ms);
-      }
+    q.timings         = &t;
+    float ms          = INFINITY;
+    for (int rep = 0; rep < 3 && rc == EBG_OK; rep++) {
+      rc = meshQuery(m, sample_points_dev, n, out, walk ? tri : nullptr, &q, nullptr, s);
+      ms = rc == EBG_OK && rep > 0 ? std::min(ms, t.traverse_ms) : ms;
     }
-    return EBG_OK;
+    return ms;
   };
-  float     bestMs = INFINITY;
-  int       bestO = 1, bestW = 4, bestC = 1;
   const int occs[] = {1, 4, 2};
   const int wpbs[] = {2, 4, 8};
-  for (int o : occs) {
-    for (int w : wpbs) {
-      if (o != 4 && w > 4) {
-        continue;
-      }
-      float            ms = INFINITY;
-      const ebg_status rc = timeOne(o, w, 1, ms);
-      if (rc != EBG_OK) {
-        cudaFreeAsync(out, s);
-        return rc;
-      }
-      if (ms < bestMs) {
-        bestMs = ms;
-        bestO  = o;
-        bestW  = w;
-      }
-    }
-  }
-  for (int c : {2, 4}) {
-    float            ms = INFINITY;
-    const ebg_status rc = timeOne(bestO, bestW, c, ms);
-    if (rc != EBG_OK) {
-      cudaFreeAsync(out, s);
-      return rc;
-    }
-    if (ms < bestMs) {
-      bestMs = ms;
-      bestC  = c;
-    }
-  }
-  // node width: the 8-wide copy at the launch shapes again (its node visits differ), kept when faster
-  int bestWidth = 4;
-  if (seed == nullptr && m->hasWide && !(m->view.root_ref & EBG_LEAF_BIT)) {
+  float     bestMs = INFINITY;
+  int       bestO = 1, bestW = 4, bestC = 1, bestWidth = 4, bestGroup = 0;
+  auto      shapes = [&](int c, int width) {
     for (int o : occs) {
       for (int w : wpbs) {
         if (o != 4 && w > 4) {
           continue;
         }
-        float            ms = INFINITY;
-        const ebg_status rc = timeOne(o, w, bestC, ms, 8);
-        if (rc != EBG_OK) {
-          cudaFreeAsync(out, s);
-          return rc;
-        }
+        const float ms = timeOne(o, w, c, true, width);
         if (ms < bestMs) {
           bestMs    = ms;
           bestO     = o;
           bestW     = w;
-          bestWidth = 8;
+          bestWidth = width;
         }
       }
     }
+  };
+  shapes(1, 4);
+  for (int c : {2, 4}) {
+    const float ms = timeOne(bestO, bestW, c, true);
+    if (ms < bestMs) {
+      bestMs = ms;
+      bestC  = c;
+    }
   }
-  cudaFreeAsync(out, s);
+  // what calls for distances alone take on this mesh, and its packets per group
+  if (packetMesh(m)) {
+    float packetMs = INFINITY;
+    for (int c : {8, 4, 16}) {
+      const float ms = timeOne(0, 0, c, false);
+      if (ms < packetMs) {
+        packetMs  = ms;
+        bestGroup = c;
+      }
+    }
+    bestMs = packetMs;
+  }
+  // node width: the 8-wide copy at the launch shapes again (its node visits differ), kept when faster
+  if (seed == nullptr && m->hasWide && !(m->view.root_ref & EBG_LEAF_BIT)) {
+    shapes(bestC, 8);
+  }
   cudaStreamSynchronize(s);
+  if (rc != EBG_OK) {
+    return rc;
+  }
   m->tunedOccupancy = bestO;
   m->tunedWpb       = bestW;
   m->tunedChunk     = bestC;
+  m->tunedGroup     = bestGroup;
   m->tunedWidth     = bestWidth;
   if (best_occupancy) {
     *best_occupancy = bestO;

@@ -409,14 +409,16 @@ ebg_status ebg_mesh_signed_distance_stats(const ebg_mesh*       mesh,
 
 /* Autotuner (no reference counterpart; the reference fixes its branching ratio and SoA width at
  * compile time, DefaultBranchingRatio, BVH.hpp:89-111, and TriangleSoA::DefaultWidth,
- * TriangleSoA.hpp:55-77): times the traversal's launch shapes -- register budget
- * (ebg_query_opts.occupancy 1..4) x warps per block (2, 4, 8), then the work-queue chunk (1, 2, 4
- * packets per grab) at the fastest shape, then (plain traversal of a mesh with an 8-wide copy,
- * ebg_mesh_widen) the node width 8 against 4 at that shape, with the launch shape re-tuned for
- * width 8 -- on the caller's sample points (device), keeps the fastest as this mesh's default for
- * queries that leave those options at 0, and returns it (best_occupancy / best_warps_per_block /
- * best_queue_chunk / best_node_width, any of them nullable; best_ms = the sample's traversal time).
- * `seed` (nullable) times the seeded traversal of a model attached to the mesh (node width 4).
+ * TriangleSoA.hpp:55-77): on the caller's sample points (device) it times the packet walk's launch
+ * shapes -- register budget (ebg_query_opts.occupancy 1, 2, 4) x warps per block (2, 4, 8) -- then its
+ * work-queue chunk (1, 2, 4 packets per grab) at the fastest shape; then, where calls for distances
+ * alone take the search by packet boxes, that search with groups of 4, 8 and 16 packets; then (no
+ * `seed`, a mesh with an 8-wide copy, ebg_mesh_widen) the walk of the 8-wide copy, with its launch
+ * shape re-tuned, kept where it is faster than all of these.  It keeps the fastest as this mesh's
+ * defaults for queries that leave those options at 0, and returns the walk's shape and chunk and the
+ * node width (best_occupancy / best_warps_per_block / best_queue_chunk / best_node_width, any of them
+ * nullable; best_ms = the sample's traversal time in a call for distances).
+ * `seed` (nullable) times the queries that pass a model attached to the mesh (node width 4).
  * Synchronous. */
 ebg_status ebg_mesh_autotune(ebg_mesh*       mesh,
                              const float*    sample_points_dev,
