@@ -191,18 +191,29 @@ __device__ __forceinline__ void testPairs(const EbgMeshView& m, PacketMem& pm, i
   }
 }
 
-// The anchor of the cell that holds a point (nearest cell outside the grid): the triangle nearest to
-// the cell's centre, or -1.
-__device__ __forceinline__ int cellAnchor(const SeedCellsView& cv, float px, float py, float pz)
+// The cell of an attached model that holds a point (nearest cell outside the grid).
+__device__ __forceinline__ int64_t cellOf(const SeedCellsView& cv, float px, float py, float pz)
 {
-  if (cv.anchor == nullptr) {
-    return -1;
-  }
   const float gm = float(cv.g - 1);
   const int   ix = int(fminf(fmaxf((px - cv.lo[0]) * cv.inv[0], 0.f), gm));
   const int   iy = int(fminf(fmaxf((py - cv.lo[1]) * cv.inv[1], 0.f), gm));
   const int   iz = int(fminf(fmaxf((pz - cv.lo[2]) * cv.inv[2], 0.f), gm));
-  return __ldg(cv.anchor + (int64_t(iz) * cv.g + iy) * cv.g + ix);
+  return (int64_t(iz) * cv.g + iy) * cv.g + ix;
+}
+
+// A cell's anchor, the triangle nearest to its centre, or -1.
+__device__ __forceinline__ int cellAnchor(const SeedCellsView& cv, int64_t cell)
+{
+  return cv.anchor ? __ldg(cv.anchor + cell) : -1;
+}
+
+// The model's bound of |d| in the cell that holds a point: FLT_MAX outside the grid, where it says nothing.
+__device__ __forceinline__ float cellRadius(const SeedCellsView& cv, int64_t cell, float px, float py, float pz)
+{
+  const float fx = (px - cv.lo[0]) * cv.inv[0], fy = (py - cv.lo[1]) * cv.inv[1], fz = (pz - cv.lo[2]) * cv.inv[2];
+  const float g  = float(cv.g);
+  const float R  = __ldg(cv.radius + cell);
+  return fx >= 0.f && fx < g && fy >= 0.f && fy < g && fz >= 0.f && fz < g ? fminf(R, FLT_MAX) : FLT_MAX;
 }
 
 // Whether a packet too wide for one box takes the walk as a whole: where its points (lanes `in`) share what they
@@ -224,8 +235,8 @@ __device__ __noinline__ bool sharesReach(const EbgMeshView& m, bool in, float px
   return n > 4 && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) * leaves < WALK_LEAVES * float(n) * far * far;
 }
 
-// CELLS: the query passes an attached model, and its cells' anchors give the lanes' first bounds and
-// the mesh points `a`.
+// CELLS: the query passes an attached model, and its cells give the lanes' first bounds (the smaller of the
+// model's radius and the distance to the anchor) and, by their anchors, the mesh points `a`.
 template <bool CELLS>
 __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __grid_constant__ MeshQueryArgs a, float delta,
                                                                      float split, float diagonal, float leaves)
@@ -298,7 +309,7 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
       if (got) {
         int err = 0;
         if (CELLS) {
-          besttri = cellAnchor(a.cells, qx, qy, qz);
+          besttri = cellAnchor(a.cells, cellOf(a.cells, qx, qy, qz));
         }
         if (besttri < 0) {
           err = nearTriangle(m, qx, qy, qz, delta, w, besttri);
@@ -399,7 +410,8 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
         // the mesh point `a` nearest to c among the winners of the packet before and of the ranges
         // before; the lane's own one is its first bound
         int            cand = besttri >= 0 ? besttri : prev;
-        const int      own  = CELLS ? cellAnchor(a.cells, px, py, pz) : -1;
+        const int64_t  cell = CELLS ? cellOf(a.cells, px, py, pz) : 0;
+        const int      own  = CELLS ? cellAnchor(a.cells, cell) : -1;
         cand                = CELLS && own >= 0 ? own : cand;
         const float4   last = pm.last;
         if (!__any_sync(FULL, own >= 0) && fmaxf(fabsf(r.cx - last.x), fmaxf(fabsf(r.cy - last.y), fabsf(r.cz - last.z))) > 4.f * (hm + last.w)) {
@@ -431,6 +443,25 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
           az             = __shfl_sync(FULL, az, from);
         }
         setCorners(pm.corner, r, ax, ay, az, delta);
+        if (CELLS) {
+          // The model's radius, where it is the smaller bound: of a lane (a lane that then finds nothing is
+          // put aside), and without anchors of the packet.
+          const float R = cellRadius(a.cells, cell, px, py, pz), R2 = __fmul_rd(__fmul_rd(R, R), 0.99998f);
+          if (in && R2 < best) {
+            best    = R2;
+            besttri = -1;
+          }
+          if (a.cells.anchor == nullptr) {
+            const float  most = warpMax(in ? R : 0.f) * 1.00001f + delta;
+            const float4 A0 = pm.corner[0], A1 = pm.corner[1];
+            const bool   nearer = most < fmaxf(fmaxf(fmaxf(A0.x, A0.y), fmaxf(A0.z, A0.w)), fmaxf(fmaxf(A1.x, A1.y), fmaxf(A1.z, A1.w)));
+            __syncwarp();
+            if (nearer && lane < 2) {
+              pm.corner[lane] = make_float4(most, most, most, most);
+            }
+            __syncwarp();
+          }
+        }
         pm.key[lane] = (unsigned long long)__float_as_uint(best) << 32 | uint32_t(besttri);
         if (lane == 0) {
           pm.last = make_float4(r.cx, r.cy, r.cz, hm);
@@ -598,6 +629,7 @@ __global__ void __launch_bounds__(32 * PACKET_WARPS, 8) kMeshPacket32(const __gr
           best    = __uint_as_float(uint32_t(kb >> 32));
           besttri = int(uint32_t(kb));
         }
+        later = later || (CELLS && box && in && besttri < 0);
       }
       if (!box) {
         // too wide, far away, very few points or too many leaves in reach
