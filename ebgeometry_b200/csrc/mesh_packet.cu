@@ -84,6 +84,9 @@ __device__ __forceinline__ void store(const MeshQueryArgs& a, const EbgMeshView&
   if (a.out_tri) {
     a.out_tri[id] = tri >= 0 ? (a.tri_leaf ? tri : __ldg(m.tri_id + tri)) : -1;
   }
+  if (a.out_d64 && tri < 0) {
+    a.out_d64[id] = double(FLT_MAX); // not among the FP64 pass's queries
+  }
   if (a.band_flag) {
     // one flag per sorted position; the list is compacted from them in position order
     a.band_flag[pos] = uint8_t(tri >= 0 && fabsf(dist) <= a.band);

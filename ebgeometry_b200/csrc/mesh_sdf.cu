@@ -332,6 +332,9 @@ __global__ void __launch_bounds__(Bounds<OCC>::threads, Bounds<OCC>::blocks) kMe
       if (a.out_tri) {
         a.out_tri[id] = besttri >= 0 ? (a.tri_leaf ? besttri : __ldg(m.tri_id + besttri)) : -1;
       }
+      if (a.out_d64 && besttri < 0) {
+        a.out_d64[id] = double(FLT_MAX); // not among the FP64 pass's queries
+      }
     }
     if (a.band_flag) {
       // one flag per sorted position; the list is compacted from them in position order
