@@ -239,29 +239,30 @@ def l2_read_bandwidth():
     return out.value if rc == 0 else None
 
 
-def traffic_from_csv(path, kernel="kMeshPacket32"):
-    """DRAM bytes (read + write) per launch of `kernel`, averaged over the launches an ncu CSV
-    (--metrics dram__bytes_read.sum,dram__bytes_write.sum --csv) recorded."""
+def traffic_from_csv(path, kernels=("kMeshPacket32", "kMeshAside")):
+    """DRAM bytes (read + write) of one FP32 search: the sum over `kernels` of each one's average per launch
+    in an ncu CSV (--metrics dram__bytes_read.sum,dram__bytes_write.sum --csv); None without a file or
+    where one of them is missing from it."""
     import csv
     if not path or not os.path.exists(path):
         return None
-    per = {}
+    per = {k: {} for k in kernels}
     with open(path) as fh:
         rows = [ln for ln in fh if ln.startswith('"')]
     for r in csv.DictReader(rows):
-        if kernel not in r.get("Kernel Name", ""):
-            continue
         name, unit, val = r.get("Metric Name"), r.get("Metric Unit", ""), r.get("Metric Value", "0")
         if name not in ("dram__bytes_read.sum", "dram__bytes_write.sum"):
             continue
-        scale = {"byte": 1, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "KB": 1e3, "MB": 1e6, "GB": 1e9}.get(unit, 1)
-        per.setdefault(r.get("ID"), 0.0)
-        per[r.get("ID")] += float(val.replace(",", "")) * scale
-    return (sum(per.values()) / len(per)) if per else None
+        for k in kernels:
+            if k in r.get("Kernel Name", ""):
+                scale = {"byte": 1, "Kbyte": 1e3, "Mbyte": 1e6, "Gbyte": 1e9, "KB": 1e3, "MB": 1e6, "GB": 1e9}.get(unit, 1)
+                per[k][r.get("ID")] = per[k].get(r.get("ID"), 0.0) + float(val.replace(",", "")) * scale
+    return sum(sum(v.values()) / len(v) for v in per.values()) if all(per.values()) else None
 
 
 def packet_bytes(st, n):
-    """Bytes the traversal's warps load per call, counted per packet (each distinct line once per
+    """Bytes that a packet walk of the queries loads (the statistics call's counters; calls for distances search
+    by packet boxes and load other structures), counted per packet (each distinct line once per
     packet: the packet is what a warp executes): 128 B per interior node opened, 64 B per oriented
     box tested, 48 B per triangle record of an opened leaf, 32 B per entry of a cell's cut plus the
     cell's count and radius and one anchor index and record (the lanes read those of their own
@@ -529,15 +530,14 @@ def run_ours(args, rank, world, local_rank):
     if rank != 0:
         return 0
 
-    # roofline of the FP32 search (the launches timed as the "traverse" phase): the bytes that a walk of
-    # the tree by packets loads per call, counted by the statistics entry point on the same queries (the
-    # timed kernel searches by packet boxes and loads less), over the phase's event-timed duration,
-    # against the measured HBM copy roof and the measured L2 read roof
+    # roofline of the FP32 search (the launches timed as the "traverse" phase): the bytes that it cannot do
+    # without -- the mesh's device arrays, the points and the distances once each -- over the phase's
+    # event-timed duration, against the measured HBM copy roof
     hbm_peak, peak_kind = measured_peaks()
     l2_gbs = l2_read_bandwidth()
     st_run = st_seed if seed is not None else st
     nq = float(n)
-    bytes_call = float(packet_bytes(st_run, n))
+    bytes_call = float(mesh.info["device_bytes"]) + 16.0 * n
     trav_ms = float(tms[:, 1].mean())
     achieved = bytes_call / (trav_ms * 1e-3) / 1e9
     traffic = traffic_from_csv(args.traffic_csv)
@@ -597,7 +597,8 @@ def run_ours(args, rank, world, local_rank):
                                f"+ {n_band} points within 1e-3 of the surface = {n} queries/step; FP32 traversal, "
                                f"FP64 band |d| <= 1e-4 diag",
                    "seed": ("learned pruning radius (16-level hash grid + 3x64 BF16 MLP, trained on the GPU) "
-                            "attached as per-cell entry cuts of the tree with anchor triangles"
+                            "attached by cells: a lane's first bound is the smaller of its cell's radius and its "
+                            "distance to the cell's anchor triangle (found by an exact query at attach)"
                             if seed is not None else "none (plain traversal)"),
                    "build_on_device": bool(on_device),
                    "queries_per_step": n, "l2": "inputs larger than L2 "
@@ -616,22 +617,22 @@ def run_ours(args, rank, world, local_rank):
                      "frac": achieved / hbm_peak, "traffic": traffic, "peak_kind": peak_kind,
                      "traffic_source": (f"ncu capture {os.path.basename(args.traffic_csv)}" if traffic is not None
                                         else "none in this run (pass --traffic-csv from an ncu capture of it)"),
-                     "kernel": "kMeshPacket32 (FP32 search by packet boxes" + (", seeded)" if seed is not None else ")"),
+                     "kernel": "kMeshPacket32 + kMeshAside (FP32 search by packet boxes" + (", seeded)" if seed is not None else ")"),
                      "bytes_per_query": bytes_call / nq,
-                     "bytes_basis": "of the packet walk of the same queries, per packet: 128 B per interior node opened + 64 B per oriented box + 48 B per "
-                                    "triangle record of an opened leaf + 32 B per cut entry (+60 B per cut); per "
-                                    "query: 12 B point + 4 B order + 4 B result + 96 B sign record",
-                     "l2_read_gbs_measured": l2_gbs, "frac_of_l2": (achieved / l2_gbs) if l2_gbs else None,
+                     "bytes_basis": "what the search cannot do without: the mesh's device arrays once, 12 B point and "
+                                    "4 B result per query",
+                     "l2_read_gbs_measured": l2_gbs,
+                     # not of the timed kernels: what the packet walk of the statistics call loads
+                     "walk_bytes_per_query": float(packet_bytes(st_run, n)) / nq,
                      "limiter": "the L1's data stage and instruction issue on the SMs (ncu: LSU wavefronts 79 % of peak, "
                                 "issue-active 69 %), not DRAM or L2 bandwidth",
-                     # the floor: every byte the step must touch once (the mesh's device arrays, the
-                     # points in, the distances out) at the measured HBM rate
+                     # the floor: the same bytes at the measured HBM rate
                      "unique_bytes_per_step": int(mesh.info["device_bytes"]) + 16 * n,
                      "unique_floor_ms": (int(mesh.info["device_bytes"]) + 16 * n) / (hbm_peak * 1e6)},
         "e2e": {"value": n * world / (e2e_ms * 1e-3), "unit": UNIT, "h2d_bytes_per_step": int(pts.nbytes),
                 "d2h_bytes_per_step": int(n * 4), "ms_per_step": e2e_ms, "matches_device_path": same},
         "gpu_launches": 5 * args.steps,
-        "gpu_launches_note": "per step: Morton-key kernel, FP32 search by packets and of the points it lists, FP64 band "
+        "gpu_launches_note": "per step: Morton-key kernel, FP32 search by packets and of what it puts aside, FP64 band "
                              "pass by packets and of the queries it lists (plus the CUB radix-sort and "
                              "band-list compaction passes)",
         "clocks": ck,
