@@ -190,10 +190,11 @@ __device__ double dcelFaceUd2(const double* __restrict__ tri, const double* __re
 // (Not "low <= ...": a point on the triangle has no direction and a NaN bound.)
 __device__ __forceinline__ bool mayReach(float low, float dd, float reach) { return !(dd >= 1e-30f) || !(low > reach); }
 
-// The radius about the FP32 point, `shift` from the FP64 one, that holds an FP64 winner of value d.
+// The radius about the FP32 point, `shift` from the FP64 one, that holds an FP64 winner of value d (never so
+// small that its square loses precision).
 __device__ __forceinline__ float winnerRadius(double d, float shift)
 {
-  return (float(fabs(d)) + shift) * 1.000001f + 1e-30f;
+  return (float(fabs(d)) + shift) * 1.000001f + 1e-18f;
 }
 
 // The triangle of smallest |d| in FP64 within `limit` (squared) of the FP32 point (px, py, pz), which lies

@@ -111,6 +111,10 @@ inline double fp32ErrorScale(const ebg_mesh* m)
   return s;
 }
 
+// What covers the FP32 error of a triangle distance near the surface: about 17 FP32 roundings of that length,
+// and never so little that its square loses precision.
+inline float fp32Slack(const ebg_mesh* m) { return float(2e-6 * fp32ErrorScale(m)) + 1e-18f; }
+
 // Nodes of the tree's top levels that each block of the FP32 traversal copies into shared memory
 // (ebg_query_opts.top_nodes, at most MAX_TOP_NODES and the tree's node count): plain queries
 // descend through them from the root; a seeded query starts below them and copies none.

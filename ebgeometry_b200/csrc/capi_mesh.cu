@@ -614,7 +614,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     a.out_tri  = outTri;
     a.band     = float(band);
     a.status   = m->dStatus;
-    if (launchMeshPoint(a, float(2e-6 * fp32ErrorScale(m)) + 1e-30f, band64, m->numSms, s) != cudaSuccess) {
+    if (launchMeshPoint(a, fp32Slack(m), band64, m->numSms, s) != cudaSuccess) {
       return setError(EBG_ERR_CUDA, std::string("point query launch failed: ") + cudaGetErrorString(cudaGetLastError()));
     }
     return EBG_OK;
@@ -730,7 +730,7 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
     a.node_width = 8;
     a.top_nodes  = 0;
   }
-  const float delta = float(2e-6 * fp32ErrorScale(m)) + 1e-30f;
+  const float delta = fp32Slack(m);
   if (tri32) {
     if (outTri) {
       cudaMemsetAsync(outTri, 0xff, size_t(n) * sizeof(int32_t), s); // -1: what is not finite keeps it
@@ -755,8 +755,6 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
                                    a.band_count, int(n), s) != cudaSuccess) {
       return setError(EBG_ERR_CUDA, "band list compaction failed");
     }
-    // delta bounds the FP32 distance error: 2e-6 of the mesh's diagonal, or of its coordinates'
-    // magnitude for a mesh far from the origin (about 17 FP32 roundings of either)
     if (launchMeshBand64(a, delta, packetSplit(m), m->numSms, s) != cudaSuccess) {
       return setError(EBG_ERR_CUDA, "band launch failed");
     }

@@ -199,7 +199,7 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
   a.point_list  = idsIn; // free after the sort
   a.later       = keysIn;
   a.later_count = reinterpret_cast<uint32_t*>(counters + 2);
-  const float delta = float(2e-6 * fp32ErrorScale(m)) + 1e-30f;
+  const float delta = fp32Slack(m);
   if (launchMeshFp32(m, a, closest_tri_dev != nullptr, wpb, occ, delta, s) != cudaSuccess) {
     return cudaFailed("traversal launch");
   }

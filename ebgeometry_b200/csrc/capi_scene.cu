@@ -185,7 +185,7 @@ ebg_status sceneQuery(const ebg_scene*      s,
   a.band_list  = bandList;
   a.band_count = bandCnt;
   // delta bounds the FP32 error of the union's value: the instance transform and the mesh distance
-  a.delta       = float(4e-6 * s->errScale) + 1e-30f;
+  a.delta       = float(4e-6 * s->errScale) + 1e-18f;
   cudaError_t e = launchSceneValue(a, s->numSms, st);
   if (e == cudaSuccess && band64) {
     if (cub::DeviceSelect::Flagged(selTemp, selBytes, thrust::counting_iterator<uint32_t>(0u), flags, bandList,

@@ -64,3 +64,17 @@ def test_fp32_of_tiny_meshes_finds_a_triangle(scale, n):
         d = m.signed_distance(p)
         m.check_status()
         assert (d.abs() <= 1.001 * (p.double().norm(dim=1) + 2.0 * scale) + 2e-23).all()
+
+
+@pytest.mark.parametrize("n", [3000, 70001])
+def test_fp64_of_a_tiny_mesh_from_afar(n):
+    """Squared distances of 1e-44 have one digit in FP32: the FP64 result must not depend on them."""
+    v, f = W.displaced_icosphere(4, 5)
+    v = v * 1e-25
+    rng = np.random.default_rng(n)
+    u = rng.normal(size=(n, 3))
+    p = torch.from_numpy(u / np.linalg.norm(u, axis=1, keepdims=True) * 10.0 ** rng.uniform(-25, -19, (n, 1))).cuda()
+    ref = FlatMeshSDF(v, f).signed_distance(p).abs()
+    for cls in (MeshSDF, TriMeshSDF):
+        d = cls(v, f).signed_distance(p).abs()
+        assert ((d - ref).abs() <= 1e-14 * (1e-25 + ref)).all()
