@@ -33,9 +33,8 @@ struct ebg_mesh
   void* dNodeObb = nullptr;
   void* dDcelN   = nullptr;
   int*  dStatus = nullptr;
-  // the leaf boxes' diagonals, in units of the mesh's: sums on the device, mean and mean square
-  unsigned long long* dLeafSums = nullptr;
-  double              leafMean = 0.0, leafSquare = 0.0;
+  // the leaf boxes' diagonals, in units of the mesh's: mean and mean square (from PACKET_TRIANGLES on)
+  double leafMean = 0.0, leafSquare = 0.0;
   // kept for refitting moved vertices: the soup's triangles, and each leaf's and each interior
   // node's range of leaf positions
   int32_t*  dF         = nullptr;
@@ -134,6 +133,9 @@ inline uint32_t   topNodesFor(const ebg_mesh* m, const ebg_query_opts* opts, boo
 // a.chunk: packets taken from the work counter at a time, 0 = the default.
 cudaError_t launchMeshFp32(const ebg_mesh* m, MeshQueryArgs a, bool fp32Triangles, int warpsPerBlock, int occupancy,
                            float delta, cudaStream_t s);
+
+// Meshes of fewer triangles never take the search by packet boxes (see launchMeshFp32).
+constexpr int64_t PACKET_TRIANGLES = 4096;
 
 // Mean and mean square from the sums of launchLeafSizes.
 inline void setLeafSizes(ebg_mesh* m, const unsigned long long* sums)

@@ -209,7 +209,6 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
 {
   const size_t slots = 4 * size_t(std::max<int64_t>(m->info.num_nodes, 1));
   if (cudaMalloc(&m->dChildren, slots * sizeof(EbgChild)) != cudaSuccess ||
-      cudaMalloc(reinterpret_cast<void**>(&m->dLeafSums), 2 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&m->dStatus), sizeof(int)) != cudaSuccess ||
       cudaMemset(m->dStatus, 0, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
@@ -236,14 +235,24 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
                              size_t(inf.num_leaves) * (sizeof(EbgObb) + 8) +
                              N * (sizeof(EbgTriHot) + sizeof(EbgTriSign) + 33 * sizeof(double) + 4 + 12));
   launchNodeChildren(v.nodes, inf.num_nodes, static_cast<EbgChild*>(m->dChildren), nullptr);
-  launchLeafSizes(v.children, inf.num_nodes, inf.diagonal, m->dLeafSums, nullptr);
-  unsigned long long sums[2];
-  if (cudaMemcpy(sums, m->dLeafSums, sizeof(sums), cudaMemcpyDeviceToHost) != cudaSuccess) {
+  unsigned long long* sums = nullptr;
+  if (nt >= PACKET_TRIANGLES) {
+    if (cudaMalloc(reinterpret_cast<void**>(&sums), 2 * sizeof(unsigned long long)) == cudaSuccess) {
+      unsigned long long back[2] = {0, 0};
+      launchLeafSizes(v.children, inf.num_nodes, inf.diagonal, sums, nullptr);
+      cudaMemcpy(back, sums, sizeof(back), cudaMemcpyDeviceToHost);
+      cudaFree(sums);
+      setLeafSizes(m, back);
+    }
+    else {
+      cudaGetLastError(); // unmeasured: the mesh takes the walk
+    }
+  }
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
     const std::string e = cudaGetErrorString(cudaGetLastError());
     ebg_mesh_destroy(m);
     return setError(EBG_ERR_CUDA, "mesh set-up: " + e);
   }
-  setLeafSizes(m, sums);
   *out = m;
   return EBG_OK;
 }
@@ -525,7 +534,7 @@ bool pointPath(int64_t n, const ebg_query_opts* opts, const unsigned long long* 
 static bool packetMesh(const ebg_mesh* m)
 {
   const double d2 = m->info.diagonal * m->info.diagonal, boxes = m->leafSquare * double(m->info.num_leaves);
-  return m->info.num_triangles >= 4096 && boxes >= 3.0 && boxes <= 8.0 && m->leafMean * m->leafMean >= 0.5 * m->leafSquare &&
+  return m->info.num_triangles >= PACKET_TRIANGLES && boxes >= 3.0 && boxes <= 8.0 && m->leafMean * m->leafMean >= 0.5 * m->leafSquare &&
          !m->areaCdf.empty() && m->areaCdf.back() >= 0.6 * d2;
 }
 
@@ -861,7 +870,6 @@ ebg_status ebg_mesh_destroy(ebg_mesh* m)
   cudaFree(m->dNodeObb);
   cudaFree(m->dDcelN);
   cudaFree(m->dStatus);
-  cudaFree(m->dLeafSums);
   cudaFree(m->dF);
   cudaFree(m->dLeafFirst);
   cudaFree(m->dLeafCount);

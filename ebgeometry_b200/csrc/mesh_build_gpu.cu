@@ -1902,7 +1902,7 @@ ebg_status refitMeshOnDevice(ebg_mesh* m, const double* V, bool vOnDevice, int64
   double *            leafAabb = nullptr, *nodeAabb = nullptr;
   bool ok = alloc((void**)&dTriN, 24 * N) && alloc((void**)&dVN, 72 * N) && alloc((void**)&dEN, 72 * N) &&
             alloc((void**)&triLo, 24 * N) && alloc((void**)&triHi, 24 * N) && alloc((void**)&cen, 24 * N) &&
-            alloc((void**)&area, 8 * N) && alloc((void**)&bounds, 12 * 8) &&
+            alloc((void**)&area, 8 * (N + 2)) && alloc((void**)&bounds, 12 * 8) &&
             alloc((void**)&useful, std::max<size_t>(numNodes, 1)) && alloc((void**)&bad, 4) &&
             alloc((void**)&leafAabb, 48 * size_t(numLeaves)) && alloc((void**)&nodeAabb, 48 * size_t(numNodes));
   if (ok && !vOnDevice) {
@@ -1971,23 +1971,31 @@ ebg_status refitMeshOnDevice(ebg_mesh* m, const double* V, bool vOnDevice, int64
                                                                    static_cast<EbgNode4*>(m->dNodes));
     launchNodeChildren(m->view.nodes, numNodes, static_cast<EbgChild*>(m->dChildren), s);
   }
+  // the leaves' sizes (packetMesh asks for them) come back behind the areas
   double d2 = 0;
   for (int a = 0; a < 3; a++) {
     d2 += (outHi[a] - outLo[a]) * (outHi[a] - outLo[a]);
   }
-  launchLeafSizes(m->view.children, numNodes, std::sqrt(d2), m->dLeafSums, s);
-  unsigned long long sums[2];
-  cudaMemcpyAsync(sums, m->dLeafSums, sizeof(sums), cudaMemcpyDeviceToHost, s);
-  std::vector<double> cdf(N);
-  cudaMemcpyAsync(cdf.data(), area, 8 * N, cudaMemcpyDeviceToHost, s);
+  const bool   measure = n >= PACKET_TRIANGLES;
+  const size_t back    = N + (measure ? 2 : 0);
+  if (measure) {
+    launchLeafSizes(m->view.children, numNodes, std::sqrt(d2), reinterpret_cast<unsigned long long*>(area + N), s);
+  }
+  std::vector<double> cdf(back);
+  cudaMemcpyAsync(cdf.data(), area, 8 * back, cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) {
     return setError(EBG_ERR_CUDA, std::string("refit: ") + cudaGetErrorString(cudaGetLastError()));
+  }
+  if (measure) {
+    unsigned long long sums[2];
+    std::memcpy(sums, cdf.data() + N, sizeof(sums));
+    setLeafSizes(m, sums);
+    cdf.resize(N);
   }
   for (size_t i = 1; i < N; i++) {
     cdf[i] += cdf[i - 1];
   }
   m->areaCdf.swap(cdf);
-  setLeafSizes(m, sums);
   return EBG_OK;
 }
 
