@@ -720,7 +720,6 @@ ebg_status ebg::meshQuery(const ebg_mesh*       m,
   a.band       = float(band);
   a.band_list  = bandList;
   a.band_count = reinterpret_cast<uint32_t*>(counters + 1);
-  a.band_d32   = nullptr;
   a.point_list = pointList;
   a.later       = later;
   a.later_count = reinterpret_cast<uint32_t*>(counters + 2);

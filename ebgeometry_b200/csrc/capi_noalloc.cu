@@ -186,7 +186,6 @@ ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       m,
   a.band       = float(band);
   a.band_list  = b64 ? bandList : nullptr;
   a.band_count = bandCnt;
-  a.band_d32   = nullptr;
   a.band_flag  = b64 ? bandFlag : nullptr;
   a.work       = counters;
   a.status     = m->dStatus;

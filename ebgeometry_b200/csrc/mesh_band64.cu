@@ -100,14 +100,13 @@ __device__ __forceinline__ bool bandCandidate(const EbgMeshView& m, uint32_t tt,
   return mayReach(triLower(h0, h1, h2, px, py, pz, s, t, dd), dd, sqrtf(bound) * 1.00001f + delta);
 }
 
-// Eight lanes per band query (groupSearch), from the root with the query's own bound: the queries of the
-// whole list, or those that kMeshBand64 put aside.
+// Eight lanes per band query that kMeshBand64 put aside (groupSearch), from the root with the query's own bound.
 template <int EVAL>
 __global__ void __launch_bounds__(32 * BAND_WARPS, 6) kMeshBandGroups(const __grid_constant__ MeshQueryArgs a, float delta)
 {
   __shared__ BandMem mem[4 * BAND_WARPS];
   const EbgMeshView& m     = a.mesh;
-  const uint32_t     count = a.later ? *a.later_count : *a.band_count;
+  const uint32_t     count = *a.later_count;
   const uint32_t     nG    = gridDim.x * (4 * BAND_WARPS);
   const int          sub   = threadIdx.x & 7;
   const unsigned     base  = threadIdx.x & 24;
@@ -116,12 +115,11 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 6) kMeshBandGroups(const __gr
   for (uint32_t j0 = blockIdx.x * (4 * BAND_WARPS) + (threadIdx.x >> 5) * 4; j0 < count; j0 += nG) {
     const uint32_t j   = j0 + (base >> 3);
     const bool     on  = j < count;
-    const uint32_t jj  = a.later ? a.later[on ? j : j0] : (on ? j : j0);
-    const uint32_t pos = a.band_list[jj];
+    const uint32_t pos = a.band_list[a.later[on ? j : j0]];
     const uint32_t id  = a.order ? a.order[pos] : pos;
     const float    px = a.points[3 * size_t(id)], py = a.points[3 * size_t(id) + 1], pz = a.points[3 * size_t(id) + 2];
     const D3       P   = bandPoint(a, id, px, py, pz);
-    const float    d32 = a.band_d32 ? a.band_d32[jj] : a.out_d[id]; // the FP32 pass's distance
+    const float    d32 = a.out_d[id]; // the FP32 pass's distance
     float        shift;
     const float  r     = bandRadius(P, px, py, pz, d32, delta, shift);
     float        bound = r * r;
@@ -242,7 +240,7 @@ __global__ void __launch_bounds__(32 * BAND_WARPS, 6) kMeshBand64(const __grid_c
     const uint32_t id  = a.order ? a.order[pos] : pos;
     const float    px = a.points[3 * size_t(id)], py = a.points[3 * size_t(id) + 1], pz = a.points[3 * size_t(id) + 2];
     const D3       P   = bandPoint(a, id, px, py, pz);
-    const float    d32 = a.band_d32 ? a.band_d32[jj] : a.out_d[id]; // the FP32 pass's distance
+    const float    d32 = a.out_d[id]; // the FP32 pass's distance
     float          shift;
     const float    r = bandRadius(P, px, py, pz, d32, delta, shift);
     float          bound = r * r;
@@ -537,18 +535,12 @@ void launchDoubleToFloat(const double* in, float* out, int64_t count, cudaStream
 cudaError_t launchMeshBand64(const MeshQueryArgs& a, float delta, float split, int numSms, cudaStream_t s)
 {
   const unsigned blocks = unsigned(numSms * 6);
-  if (a.later != nullptr) {
-    if (a.eval == 1) {
-      kMeshBand64<1><<<blocks, 32 * BAND_WARPS, 0, s>>>(a, delta, split);
-    }
-    else {
-      kMeshBand64<0><<<blocks, 32 * BAND_WARPS, 0, s>>>(a, delta, split);
-    }
-  }
   if (a.eval == 1) {
+    kMeshBand64<1><<<blocks, 32 * BAND_WARPS, 0, s>>>(a, delta, split);
     kMeshBandGroups<1><<<blocks, 32 * BAND_WARPS, 0, s>>>(a, delta);
   }
   else {
+    kMeshBand64<0><<<blocks, 32 * BAND_WARPS, 0, s>>>(a, delta, split);
     kMeshBandGroups<0><<<blocks, 32 * BAND_WARPS, 0, s>>>(a, delta);
   }
   return cudaGetLastError();

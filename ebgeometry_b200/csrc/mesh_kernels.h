@@ -31,13 +31,12 @@ struct MeshQueryArgs
                                  // the back the packets that take the walk, two words each (packet, mask of
                                  // lanes; their number: later_count[1]).  Both counts zeroed before the launch.
   uint32_t*          later;       // entries of band_list that the packets of the FP64 pass leave to groups of
-                                  // lanes, counted in later_count (nullable: every entry takes a group)
+                                  // lanes, counted in later_count
   uint32_t*          later_count; // zeroed before the launch, as the three words after it: [1] see point_list,
                                  // [2] and [3] how many of the packets and points on it are taken
   const int32_t*     tri32;       // the FP32 pass's winning triangles, leaf order, caller order (nullable)
-  float*             band_d32;   // FP32 distance of each band entry (nullable: read out_d instead)
-  uint8_t*           band_flag;  // per sorted position, 1 = needs FP64 (nullable: the traversal
-                                 // appends to band_list itself, in completion order)
+  uint8_t*           band_flag;  // per sorted position, 1 = needs FP64 (nullable = no band pass); band_list is
+                                 // compacted from it
   unsigned long long* work;      // packet counter (zeroed before the launch)
   int                chunk;      // packets taken from the counter at a time (0, 1: one)
   int*               status;     // device status word (ST_* bits)

@@ -12,13 +12,13 @@
 //   - |p - a| - u . (p - e) is convex in p, so over the packet's box it is largest at a corner: where it
 //     is negative at all eight corners, no query of the packet needs the entry.
 // Unlike a bound from two radii, this keeps what lies beside the packet's own patch only as far as
-// the directions to it and to `a` differ.  What is left is a list of leaves, which all lanes test
-// with their own bounds as the walk does (packetLeaf).
+// the directions to it and to `a` differ.  What is left is a list of leaves for the lanes to test with
+// their own bounds.
 //
 // Packets come off the work counter in groups of up to eight neighbours.  A group's box is taken
 // down the tree once, as far as at most 32 entries reach; its packets start there.  The winners of one
 // packet give the next its `a` and its lanes' first bounds (a query that passes an attached model takes
-// both from the anchors of its cells instead).
+// both from its cells instead: the anchors, and the model's radius where that is smaller).
 //
 // The list is tested in three steps.  The two leaves nearest to c go through all lanes, which brings
 // the bounds near their final values; then a lane per leaf tests its oriented box against the 32
@@ -33,8 +33,8 @@
 // Bound by the L1's data stage (89 % of its wavefronts) and by instruction issue (69 %): per packet of
 // the 512^3 grid 10 rounds of 32 children, 104 listed leaves, 27 of them with a pair, 7 passes over
 // pairs, about 19,000 warp instructions.  B200, 151 M points on 1.3 M triangles, the walk -> here:
-// traversal 172.6 -> 79.5 ms, with a model 92.3 -> 71.2 ms; 1 M uniform points on 20,480 triangles
-// 1.42 -> 0.75 ms; 262,144 on 81,920 triangles 2.11 -> 0.65 ms.
+// traversal 172.6 -> 79.0 ms, with a model 92.3 -> 70.6 ms; 1 M uniform points on 20,480 triangles
+// 1.42 -> 0.73 ms, 8 M on 327,680 11.6 -> 7.4 ms; 8 M about two spheres 12.5 -> 13.1 ms.
 #include <algorithm>
 #include <cfloat>
 
@@ -61,7 +61,10 @@ __device__ __noinline__ int nearTriangle(const EbgMeshView& m, float px, float p
 
 constexpr int PACKET_FRONT = 32; // entries of a group's frontier
 
-constexpr float WALK_LEAVES = 0.2f; // leaves per point up to which a wide packet takes the walk
+// Leaves per point up to which a wide packet takes the walk.  8 M uniform points, 0.05, 0.1, 0.2 and 0.5: about
+// two spheres of 81,920 triangles each 15.7, 13.8, 13.4 and 13.1 ms, about a 5:1 ellipsoid of 327,680 19.9, 17.9,
+// 16.7 and 16.5, about a round body of 327,680 7.9, 7.8, 8.1 and 8.3.
+constexpr float WALK_LEAVES = 0.2f;
 
 struct PacketMem
 {

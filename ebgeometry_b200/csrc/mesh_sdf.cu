@@ -342,22 +342,6 @@ __global__ void __launch_bounds__(Bounds<OCC>::threads, Bounds<OCC>::blocks) kMe
         a.band_flag[pos] = uint8_t(besttri >= 0 && fabsf(dist) <= a.band);
       }
     }
-    else if (a.band_list) {
-      const bool     inb  = valid && besttri >= 0 && fabsf(dist) <= a.band;
-      const unsigned mask = __ballot_sync(FULL, inb);
-      if (mask) {
-        uint32_t base = 0;
-        if (lane == 0) {
-          base = atomicAdd(a.band_count, uint32_t(__popc(mask)));
-        }
-        base = __shfl_sync(FULL, base, 0);
-        if (inb) {
-          const uint32_t r = base + __popc(mask & ((1u << lane) - 1u));
-          a.band_list[r]   = uint32_t(pos);
-          a.band_d32[r]    = dist;
-        }
-      }
-    }
     if (STATS) {
       if (!valid) {
         cNode = cLeaf = cTri = cFall = cBox = 0;

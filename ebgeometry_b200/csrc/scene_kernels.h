@@ -97,8 +97,7 @@ __device__ __forceinline__ const float* scenePoint(const SceneQueryArgs& a, uint
 
 int         sceneOuterDepth();
 cudaError_t launchSceneValue(const SceneQueryArgs& a, int numSms, cudaStream_t s);
-// FP64 re-evaluation of the band list (reads band_count on the device); delta bounds the FP32
-// error of the union's value.
+// FP64 re-evaluation of the band list (reads band_count on the device).
 cudaError_t launchSceneBand64(const SceneQueryArgs& a, int numSms, cudaStream_t s);
 // Sort keys of a batched call: the 30-bit Morton code of every point of every batch, and the
 // identity.
