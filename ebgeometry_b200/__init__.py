@@ -204,8 +204,8 @@ class TriMeshSDF:
         point (synchronous).  Float64 points (numpy or CUDA) take the FP64 entry points: every
         query is re-evaluated in FP64 and the distances come back as float64.  ``timings``: an ``_capi.PhaseTimings`` to fill with per-phase device
         times (the call then synchronises).  ``seed``: a trained :class:`SeedModel` whose predicted
-        radius seeds the traversal's pruning bound (results stay exact).  ``radius_hint``: a CUDA
-        float32 tensor of per-point upper bounds on |d| that seed the bound the same way.
+        radius seeds the pruning bound of calls of more than 65,536 points (results stay exact).  ``radius_hint``: a CUDA
+        float32 tensor of per-point upper bounds on |d| for the packet walk (ebg_query_opts.radius_hint).
         ``top_nodes``: plain queries read the tree's first ``top_nodes`` nodes from a copy in each
         block's shared memory (ebg_query_opts.top_nodes; same results).  ``node_width``: 8 traverses
         the 8-wide copy of the tree made by :meth:`widen` (plain queries; same results), 4 the 4-wide
@@ -267,8 +267,8 @@ class TriMeshSDF:
 
     def attach_seed(self, seed, cells_per_axis=0, max_entries=0, margin_cells=0.0, radius_mode=0, anchors=True,
                     stream=None):
-        """Builds this mesh's per-cell entry cuts from a :class:`SeedModel` (ebg_seed_attach);
-        queries passing ``seed=`` that model then start their packets from the cuts.  Returns the
+        """Builds this mesh's per-cell radii, anchors and entry cuts from a :class:`SeedModel`
+        (ebg_seed_attach); queries passing ``seed=`` that model then start from them.  Returns the
         attach report as a dict.  ``radius_mode``: 0 the model's radius, 1 none, 2 exact."""
         o = _capi.AttachOpts(int(cells_per_axis), int(max_entries), float(margin_cells), int(radius_mode),
                              0 if anchors else 1)
@@ -287,9 +287,10 @@ class TriMeshSDF:
         return {"num_nodes8": n8.value, "depth8": d8.value}
 
     def autotune(self, sample_points, seed=None, stream=None):
-        """Times the traversal launch shapes, the work-queue chunk and (plain queries of a mesh
-        with an 8-wide copy, :meth:`widen`) the node width on a CUDA tensor of sample points (seeded
-        with an attached :class:`SeedModel` if given) and keeps the fastest as this mesh's default;
+        """Times the packet walk's launch shapes and work-queue chunk, the packets per group of the search
+        by packet boxes and (plain queries of a mesh with an 8-wide copy, :meth:`widen`) the node width on
+        a CUDA tensor of sample points (seeded with an attached :class:`SeedModel` if given) and keeps the
+        fastest as this mesh's defaults (ebg_mesh_autotune);
         returns {"occupancy", "warps_per_block", "queue_chunk", "node_width", "ms"}."""
         o, w, c, nw, ms = C.c_int32(), C.c_int32(), C.c_int32(), C.c_int32(), C.c_float()
         check(lib.ebg_mesh_autotune(self._h, C.c_void_p(sample_points.data_ptr()), sample_points.numel() // 3,

@@ -90,8 +90,9 @@ typedef struct ebg_query_opts
   const ebg_seed*    seed;            /* learned pruning-radius model (NULL = plain traversal) */
   int32_t            warps_per_block; /* 0 = tuned default.  This and occupancy shape the packet walk
                                          (statistics, radius hints, top_nodes, the 8-wide tree, meshes
-                                         of fewer than 4,096 triangles, FP32 calls that ask for the
-                                         closest triangles); other calls fix their own */
+                                         of fewer than 4,096 triangles or of uneven resolution, FP32
+                                         calls that ask for the closest triangles); other calls fix
+                                         their own */
   int32_t            occupancy;       /* walk's register budget: 0 = default (= 1); 1, 2, 3 = at
                                          most 64, 51, 42 registers per thread (8, 10, 12 blocks of
                                          128 threads per SM; warps_per_block <= 4); 4 = the
@@ -103,7 +104,9 @@ typedef struct ebg_query_opts
                                          diagonal) that seeds the pruning radius; <= 0 or non-finite
                                          = no hint for that point.  A hint below the true |d| only
                                          costs a second traversal of that point.  Ignored when
-                                         seed is set. */
+                                         seed is set and in calls of at most 65,536 points; larger
+                                         ones take the packet walk with it, where a call without a
+                                         hint may search by packet boxes and be faster. */
   int32_t            queue_chunk;     /* packets of 32 queries a warp takes from the device work
                                          queue at a time (mesh and union queries); 0 = tuned
                                          default (1 for the packet walk and unions, 8 for the search
@@ -113,8 +116,8 @@ typedef struct ebg_query_opts
                                          tree's first top_nodes nodes (the device build numbers them
                                          level by level: 21 = the root and two levels) with their
                                          oriented boxes into shared memory and reads them there;
-                                         at most 512; 0 = none (the default, and the faster on the
-                                         level-8 workload).  Seeded queries start below the top
+                                         at most 512; 0 = none (the default, and the faster: with it
+                                         a call takes the packet walk).  Seeded queries start below the top
                                          levels and ignore it. */
   int32_t            node_width;      /* plain (and radius-hinted) FP32 traversals: 4 = the 4-wide
                                          tree, 8 = the mesh's 8-wide copy (ebg_mesh_widen; without
@@ -389,7 +392,8 @@ ebg_status ebg_mesh_signed_distance_flat_f64_host(const ebg_mesh* mesh,
  * before capturing a CUDA graph.  cudaDeviceReset on the device invalidates the array; do not call
  * this entry point on a device after resetting it.  All calls on a device share the array, so calls
  * whose work overlaps on the GPU (different streams) race and must be serialised.  Results are those
- * of ebg_mesh_signed_distance (the same launch shape, seed and band handling). */
+ * of ebg_mesh_signed_distance.  Calls of every size search in packets here (ebg_mesh_signed_distance
+ * searches calls of at most 65,536 points point by point). */
 ebg_status ebg_mesh_signed_distance_noalloc(const ebg_mesh*       mesh,
                                             const float*          points_dev,
                                             int64_t               n,
@@ -633,9 +637,9 @@ ebg_status ebg_scene_autotune(ebg_scene*   scene,
  * level) feeding a 3-hidden-layer, 64-wide ReLU MLP (BF16 weights, FP32 accumulation on the tensor
  * cores) that predicts the signed distance; its calibrated radius (1 + alpha) |prediction| + beta
  * bounds |d|.  Attached to a mesh (ebg_seed_attach below), it bounds |d| over the cells of a grid,
- * and each cell keeps the part of the mesh's tree within that bound; passed as ebg_query_opts.seed,
- * it starts the traversal of every packet of 32 sorted queries there.  Distances stay exact: the
- * radius only prunes, and a query whose radius holds no triangle is traversed again without it. */
+ * and each cell keeps an anchor triangle and the part of the mesh's tree within that bound; queries that
+ * pass it as ebg_query_opts.seed start there.  Distances stay exact: the radius only prunes, and a
+ * query whose radius holds no triangle is searched again without it. */
 typedef struct ebg_seed_opts
 {
   int64_t  num_samples;     /* exact training samples: half uniform in the domain, half within
@@ -699,10 +703,11 @@ ebg_status ebg_seed_gradients(ebg_seed* seed, const float* points_dev, const flo
  * cells on every side, bounds |d| over that grown cell (R_C); the mesh keeps a CUT of its BVH per
  * cell: at most max_entries subtrees, refined nearest-first from the root, that hold every triangle
  * within R_C of the grown cell, and the cell's ANCHOR, the triangle nearest to the cell centre
- * (found by the mesh path itself).  A query call that passes this model (ebg_query_opts.seed)
- * starts every packet of 32 sorted queries whose box fits a grown cell from that cell's cut, each
- * lane's bound being the smaller of R_C and its distance to the anchor; a query that finds nothing
- * within R_C is traversed again from the root.  Distances are exact whatever the model predicts.
+ * (found by the mesh path itself).  In a query call that passes this model (ebg_query_opts.seed) each
+ * query's first bound is the smaller of R_C and its distance to the anchor of its cell; a query that
+ * finds nothing within R_C is searched again without it.  Calls that take the packet walk (see
+ * warps_per_block) also start every packet of 32 sorted queries whose box fits a grown cell from that
+ * cell's cut.  Calls of at most 65,536 points search point by point and do not use the model.  Distances are exact whatever the model predicts.
  * Queries passing a model that is not attached to the mesh are rejected (EBG_ERR_INVALID). */
 typedef struct ebg_attach_opts
 {
