@@ -208,7 +208,7 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
                       ebg_mesh** out)
 {
   const size_t slots = 4 * size_t(std::max<int64_t>(m->info.num_nodes, 1));
-  if (cudaMalloc(&m->dChildren, slots * sizeof(EbgChild)) != cudaSuccess ||
+  if (cudaMalloc(&m->dChildren, slots * sizeof(EbgChild) + 2 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(reinterpret_cast<void**>(&m->dStatus), sizeof(int)) != cudaSuccess ||
       cudaMemset(m->dStatus, 0, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
@@ -235,18 +235,13 @@ ebg_status finishMesh(ebg_mesh* m, int64_t nv, int64_t nt, int leafSize, const d
                              size_t(inf.num_leaves) * (sizeof(EbgObb) + 8) +
                              N * (sizeof(EbgTriHot) + sizeof(EbgTriSign) + 33 * sizeof(double) + 4 + 12));
   launchNodeChildren(v.nodes, inf.num_nodes, static_cast<EbgChild*>(m->dChildren), nullptr);
-  unsigned long long* sums = nullptr;
   if (nt >= PACKET_TRIANGLES) {
-    if (cudaMalloc(reinterpret_cast<void**>(&sums), 2 * sizeof(unsigned long long)) == cudaSuccess) {
-      unsigned long long back[2] = {0, 0};
-      launchLeafSizes(v.children, inf.num_nodes, inf.diagonal, sums, nullptr);
-      cudaMemcpy(back, sums, sizeof(back), cudaMemcpyDeviceToHost);
-      cudaFree(sums);
-      setLeafSizes(m, back);
-    }
-    else {
-      cudaGetLastError(); // unmeasured: the mesh takes the walk
-    }
+    // (the sums lie behind the slots)
+    auto*              sums    = reinterpret_cast<unsigned long long*>(static_cast<EbgChild*>(m->dChildren) + slots);
+    unsigned long long back[2] = {0, 0};
+    launchLeafSizes(v.children, inf.num_nodes, inf.diagonal, sums, nullptr);
+    cudaMemcpy(back, sums, sizeof(back), cudaMemcpyDeviceToHost);
+    setLeafSizes(m, back);
   }
   if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
     const std::string e = cudaGetErrorString(cudaGetLastError());
