@@ -507,7 +507,9 @@ struct Workspace
 // Calls of at most POINT_CALL points take one warp per point (kMeshPoint) instead of packets.  The
 // line lies where the least favourable measured input still gains: 65,536 points within 1e-3 of a
 // 1,280-triangle surface take 157 us against the packets' 220 us (262,144 of them 580 against 238 us);
-// uniform points gain up to 0.25-1 M (65,536 on 1.3 M triangles: 0.45 against 6.8 ms).  Counters, phase
+// uniform points gain up to 0.25-1 M (65,536 on 1.3 M triangles: 0.45 against 6.8 ms).  (Points packed into 3 % of
+// a mesh's extent share nearly all that a packet reads: 65,536 of them 190 against 162 us on a 327,680-triangle
+// ellipsoid, 40,000 450 against 250 us on the strips of a cylinder.)  Counters, phase
 // times and the options of the packet traversal keep the packets, and so do FP32 calls that ask for the
 // closest triangles (fp32Triangles; see launchMeshFp32).
 constexpr int64_t POINT_CALL = 65536;
